@@ -68,7 +68,7 @@ def build(force=False, verbose=False):
             print(r.stdout + r.stderr)
         return obj
 
-    with cf.ThreadPoolExecutor(max_workers=min(8, os.cpu_count() or 4)) as ex:
+    with cf.ThreadPoolExecutor(max_workers=min(16, os.cpu_count() or 4)) as ex:
         objs = list(ex.map(compile_one, sources()))
     tmp = LIB + ".tmp%d" % os.getpid()
     cmd = [cc, "-shared", "-o", tmp] + objs + ARCH + ["-lcudart"]

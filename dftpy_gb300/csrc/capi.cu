@@ -111,10 +111,12 @@ int gbofdft_plan_create(const int nr[3], const double lattice[9], int precision,
   memset(p, 0, sizeof(*p));
   for (int a = 0; a < 3; ++a) p->n[a] = nr[a];
   p->n2h = nr[2] / 2 + 1;
-  // internal spectrum rows padded to whole 128-byte lines
+  // internal spectrum rows padded to whole 32-byte sectors: the column passes
+  // tile the columns of all rows back to back, so a tile of 128 bytes then
+  // covers whole sectors wherever it starts
   {
-    const int per_line = precision == GBOFDFT_F64 ? 8 : 16;
-    p->ld2 = (p->n2h + per_line - 1) / per_line * per_line;
+    const int per = precision == GBOFDFT_F64 ? 2 : 4;
+    p->ld2 = (p->n2h + per - 1) / per * per;
   }
   p->full = full ? 1 : 0;
   p->prec = precision;
@@ -194,7 +196,7 @@ int gbofdft_plan_create(const int nr[3], const double lattice[9], int precision,
   }
   cudaError_t e = cudaMalloc(&p->spec, cs * (size_t)GB_MAX_FIELDS * p->NGld);
   const int64_t nrows = (int64_t)nr[0] * nr[1];
-  p->max_partials = (nrows + 2 * p->pairs - 1) / (2 * p->pairs) + 1;
+  p->max_partials = (nrows + 1) / 2 + 1;   // a CTA of a row pass takes at least one pair of rows
   if (e == cudaSuccess) e = cudaMalloc(&p->partials, sizeof(double) * GB_NE * p->max_partials);
   if (e == cudaSuccess) e = cudaMalloc(&p->scratch, sizeof(double) * 4096);
   // the counter slot starts at 0
@@ -206,20 +208,22 @@ int gbofdft_plan_create(const int nr[3], const double lattice[9], int precision,
     gbofdft_plan_destroy(p);
     return gb_set_error(GBOFDFT_ERR_CUDA, "plan_create: initial copies: %s", cudaGetErrorString(e));
   }
+  gb_rb_plan(p);
   memcpy(p->gi.bg, p->bg, sizeof(p->bg));
   p->gi.n0 = nr[0]; p->gi.n1 = nr[1]; p->gi.n2 = nr[2]; p->gi.n2h = p->n2h; p->gi.ld2 = p->ld2;
   p->gi.full = p->full;
-  // FP32 grids whose (n0, n1) plane fits in shared memory evaluate through
-  // the plane pipeline (GBOFDFT_PLANE=0 selects the column passes instead)
+  // FP32 grids whose (n0, n1) plane fits in shared memory can evaluate through
+  // the plane pipeline (GBOFDFT_PLANE=1, or chosen as a schedule); the
+  // register-blocked column passes are faster (128^3, WT: 74 against 98 us)
   const char* pe = getenv("GBOFDFT_PLANE");
   p->plane_ok = precision == GBOFDFT_F32 && gb_plane_supported_f32(nr[0], nr[1], nr[2]);
-  p->plane = p->plane_ok && !(pe && pe[0] == '0');
+  p->plane = p->plane_ok && pe && pe[0] == '1';
   p->plane_variant = 0;
   // GBOFDFT_PLANE_PRECOND=1: the TN preconditioner's convolutions through the
   // plane pipeline too (one field: fills fewer SMs than the column passes, so
   // it pays only when other streams run beside it)
   const char* pp = getenv("GBOFDFT_PLANE_PRECOND");
-  p->plane_precond = p->plane && pp && pp[0] == '1';
+  p->plane_precond = p->plane_ok && !(pe && pe[0] == '0') && pp && pp[0] == '1';
   *out = p;
   return GBOFDFT_OK;
 }
@@ -260,9 +264,11 @@ int gbofdft_fft_r2c(gbofdft_plan* p, const void* in, void* out, void* stream) {
   GB_REQUIRE(p && in && out, "fft_r2c: null argument");
   cudaStream_t st = (cudaStream_t)stream;
   const int op = OP_RHO;
-  int rc = gb_rows_fwd(p, in, out, 0, p->n2h, 1, &op, 1.0, p->dV, st);
+  // the row pass writes twice the spectra (scale 2: separating a row pair then
+  // needs no multiplication); the factor is undone in the last pass
+  int rc = gb_rows_fwd(p, in, out, 0, p->n2h, 1, &op, 1.0, 2.0, st);
   if (!rc) rc = gb_cols(p, out, 0, p->n2h, 1, 1, -1, 1.0, st);
-  if (!rc) rc = gb_cols(p, out, 0, p->n2h, 1, 0, -1, 1.0, st);
+  if (!rc) rc = gb_cols(p, out, 0, p->n2h, 1, 0, -1, 0.5 * p->dV, st);
   return rc;
 }
 
@@ -299,9 +305,9 @@ int gbofdft_convolve(gbofdft_plan* p, const void* in, void* out, int kernel, con
     if (!rc) rc = gb_ct_rows_inv_store_pm_f32(p, p->spec, fs, 1, out, 0, st);
     if (rc != 1) return rc;
   }
-  int rc = gb_rows_fwd(p, in, p->spec, 0, p->ld2, 1, &op, 1.0, 1.0, st);
+  int rc = gb_rows_fwd(p, in, p->spec, 0, p->ld2, 1, &op, 1.0, 2.0, st);
   if (!rc) rc = gb_cols(p, p->spec, 0, p->ld2, 1, 1, -1, 1.0, st);
-  if (!rc) rc = gb_cols_conv(p, p->spec, 0, p->ld2, 1, kd, 1.0 / (double)p->N, st);
+  if (!rc) rc = gb_cols_conv(p, p->spec, 0, p->ld2, 1, kd, 0.5 / (double)p->N, st);
   if (!rc) rc = gb_cols(p, p->spec, 0, p->ld2, 1, 1, 1, 1.0, st);
   if (!rc) rc = gb_rows_inv_store(p, p->spec, 0, p->ld2, 1, out, 0, 1.0, st);
   return rc;
@@ -373,9 +379,9 @@ static int eval_impl(gbofdft_plan* p, const void* rho, const gbofdft_functional*
   }
   rc = 0;
   if (nf > 0) {
-    rc = gb_rows_fwd(p, rho, p->spec, fs, p->ld2, nf, ops, f->wt_beta, 1.0, st);
+    rc = gb_rows_fwd(p, rho, p->spec, fs, p->ld2, nf, ops, f->wt_beta, 2.0, st);
     if (!rc) rc = gb_cols(p, p->spec, fs, p->ld2, nf, 1, -1, 1.0, st);
-    if (!rc) rc = gb_cols_conv(p, p->spec, fs, p->ld2, nf, kd, 1.0 / (double)p->N, st);
+    if (!rc) rc = gb_cols_conv(p, p->spec, fs, p->ld2, nf, kd, 0.5 / (double)p->N, st);
     if (!rc) rc = gb_cols(p, p->spec, fs, p->ld2, nf, 1, 1, 1.0, st);
   }
   if (!rc)

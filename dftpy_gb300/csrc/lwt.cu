@@ -421,9 +421,11 @@ BG<T> bg_of(const gbofdft_plan* p) {
   return b;
 }
 
-// forward 3D transform of a real field (scale 1) into spectrum layout ld2
+// forward 3D transform of a real field into spectrum layout ld2, times 2 (the
+// row pass separates a row pair without the factor 1/2; the kernels that read
+// these spectra undo it)
 int fwd3d(gbofdft_plan* p, const void* in, void* spec, int op, double beta, cudaStream_t st) {
-  int rc = gb_rows_fwd(p, in, spec, 0, p->ld2, 1, &op, beta, 1.0, st);
+  int rc = gb_rows_fwd(p, in, spec, 0, p->ld2, 1, &op, beta, 2.0, st);
   if (!rc) rc = gb_cols(p, spec, 0, p->ld2, 1, 1, -1, 1.0, st);
   if (!rc) rc = gb_cols(p, spec, 0, p->ld2, 1, 0, -1, 1.0, st);
   return rc;
@@ -501,7 +503,7 @@ int lwt_run(gbofdft_plan* p, const void* rho, gbofdft_lwt* d, void* pot, double*
   const BG<T> bg = bg_of<T>(p);
   k_lwt_pre<T><<<nb, 256, 0, st>>>(N, rhoT, kfmax, d->alpha, reinterpret_cast<T*>(L.kf), reinterpret_cast<T*>(L.ra));
   GB_CHECK_LAUNCH();
-  const double invN = 1.0 / (double)N;
+  const double invN = 0.5 / (double)N;   // 1 / N of the inverse transforms, 1/2 of fwd3d
   const RowLaunch rl = row_launch(p);
   const size_t fb = lwt_field_bytes(p), sb = lwt_spec_bytes(p);
   const int64_t sfs = (int64_t)(sb / (2 * gb_elem(p)));  // complex elements per spectrum slot

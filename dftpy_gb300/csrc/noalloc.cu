@@ -133,6 +133,7 @@ extern "C" int gbofdft_convolve_noalloc(const int nr[3], const double lattice[9]
   }
   p.pairs = 2;
   memcpy(p.gi.bg, p.bg, sizeof(p.bg));
+  gb_rb_plan(&p);
   p.gi.n0 = nr[0]; p.gi.n1 = nr[1]; p.gi.n2 = nr[2]; p.gi.n2h = p.n2h; p.gi.ld2 = p.ld2; p.gi.full = p.full;
   // scratch layout: three twiddle tables, then one spectrum
   size_t off[4];

@@ -498,11 +498,48 @@ int gb_use_ct() {
   return v;
 }
 
+// The register-blocked pass of the plan's precision and length, whichever
+// translation unit holds it; 1: no such kernel (a prime factor above 7, or a
+// line too long for shared memory)
+#define GB_RB_CALL(name, ...)                                                     \
+  do {                                                                            \
+    if (p->prec == GBOFDFT_F64) return name##_f64_g0(p, __VA_ARGS__);             \
+    int rc_ = name##_f32_g1(p, __VA_ARGS__);                                      \
+    if (rc_ == 1) rc_ = name##_f32_g2(p, __VA_ARGS__);                            \
+    if (rc_ == 1) rc_ = name##_f32_g3(p, __VA_ARGS__);                            \
+    if (rc_ == 1) rc_ = name##_f32_g4(p, __VA_ARGS__);                            \
+    if (rc_ == 1) rc_ = name##_f32_g0(p, __VA_ARGS__);                            \
+    return rc_;                                                                   \
+  } while (0)
+
+static int rb_rows_fwd(gbofdft_plan* p, const void* in, void* spec, int64_t fstride, int ld2, int nf, const int* ops,
+                       double beta, double scale, double rho0, cudaStream_t st) {
+  GB_RB_CALL(gb_rb_rows_fwd, in, spec, fstride, ld2, nf, ops, beta, scale, rho0, st);
+}
+
+static int rb_rows_inv(gbofdft_plan* p, const void* spec, int64_t fstride, int ld2, int nf, void* out,
+                       int64_t ostride, double scale, const EvalDesc* ev, const void* rho, const void* vloc,
+                       void* pot, int calc_e, double* partials, int64_t* nblk, cudaStream_t st) {
+  GB_RB_CALL(gb_rb_rows_inv, spec, fstride, ld2, nf, out, ostride, scale, ev, rho, vloc, pot, calc_e, partials, nblk,
+             st);
+}
+
+static int rb_cols(gbofdft_plan* p, void* spec, int64_t fstride, int ld2, int nf, int axis, int dir, double scale,
+                   const KerDesc* kd, cudaStream_t st) {
+  GB_RB_CALL(gb_rb_cols, spec, fstride, ld2, nf, axis, dir, scale, kd, st);
+}
+
+void gb_rb_plan(gbofdft_plan* p) {
+  for (int a = 0; a < 3; ++a) {
+    p->rb[a] = gbrb::rb_axis(p->n[a], p->prec == GBOFDFT_F64, false);
+    p->rbi[a] = gbrb::rb_axis(p->n[a], p->prec == GBOFDFT_F64, true);
+  }
+}
+
 int gb_rows_fwd(gbofdft_plan* p, const void* in, void* spec, int64_t fstride, int ld2, int nf, const int* ops,
                 double beta, double scale, cudaStream_t st) {
   if (gb_use_ct()) {
-    const int rc = p->prec == GBOFDFT_F64 ? gb_ct_rows_fwd_f64(p, in, spec, fstride, ld2, nf, ops, beta, scale, st)
-                                          : gb_ct_rows_fwd_f32(p, in, spec, fstride, ld2, nf, ops, beta, scale, st);
+    const int rc = rb_rows_fwd(p, in, spec, fstride, ld2, nf, ops, beta, scale, 0.0, st);
     if (rc != 1) return rc;
   }
   return p->prec == GBOFDFT_F64 ? rows_fwd_t<double>(p, in, spec, fstride, ld2, nf, ops, beta, scale, st)
@@ -535,11 +572,8 @@ static int rows_inv_store_t(gbofdft_plan* p, const void* spec, int64_t fstride, 
 int gb_rows_inv_store(gbofdft_plan* p, const void* spec, int64_t fstride, int ld2, int nf, void* out,
                       int64_t ostride, double scale, cudaStream_t st) {
   if (gb_use_ct()) {
-    const int rc = p->prec == GBOFDFT_F64
-                       ? gb_ct_rows_inv_f64(p, spec, fstride, ld2, nf, out, ostride, scale, nullptr, nullptr, nullptr,
-                                            nullptr, 0, nullptr, nullptr, st)
-                       : gb_ct_rows_inv_f32(p, spec, fstride, ld2, nf, out, ostride, scale, nullptr, nullptr, nullptr,
-                                            nullptr, 0, nullptr, nullptr, st);
+    const int rc = rb_rows_inv(p, spec, fstride, ld2, nf, out, ostride, scale, nullptr, nullptr, nullptr, nullptr, 0,
+                               nullptr, nullptr, st);
     if (rc != 1) return rc;
   }
   return p->prec == GBOFDFT_F64 ? rows_inv_store_t<double>(p, spec, fstride, ld2, nf, out, ostride, scale, st)
@@ -571,11 +605,8 @@ int gb_rows_inv_eval(gbofdft_plan* p, const void* spec, int64_t fstride, int nf,
                      const void* rho, const void* vloc, void* pot, int calc_e, double* energies, cudaStream_t st) {
   if (gb_use_ct()) {
     int64_t nblk = 0;
-    const int rc = p->prec == GBOFDFT_F64
-                       ? gb_ct_rows_inv_f64(p, spec, fstride, p->ld2, nf, nullptr, 0, 1.0, &ev, rho, vloc, pot, calc_e,
-                                            p->partials, &nblk, st)
-                       : gb_ct_rows_inv_f32(p, spec, fstride, p->ld2, nf, nullptr, 0, 1.0, &ev, rho, vloc, pot, calc_e,
-                                            p->partials, &nblk, st);
+    const int rc = rb_rows_inv(p, spec, fstride, p->ld2, nf, nullptr, 0, 1.0, &ev, rho, vloc, pot, calc_e,
+                               p->partials, &nblk, st);
     if (rc == 0 && calc_e) {
       if (nblk > p->max_partials) return gb_set_error(GBOFDFT_ERR_STATE, "partials buffer too small");
       k_energy_final<<<6, 256, 0, st>>>(p->partials, nblk, p->dV, ev.e_ion, energies, gb_plan_counter(p));
@@ -623,8 +654,7 @@ static int cols_t(gbofdft_plan* p, void* spec, int64_t fstride, int ld2, int nf,
 int gb_cols(gbofdft_plan* p, void* spec, int64_t fstride, int ld2, int nf, int axis, int dir, double scale,
             cudaStream_t st) {
   if (gb_use_ct()) {
-    const int rc = p->prec == GBOFDFT_F64 ? gb_ct_cols_f64(p, spec, fstride, ld2, nf, axis, dir, scale, nullptr, st)
-                                          : gb_ct_cols_f32(p, spec, fstride, ld2, nf, axis, dir, scale, nullptr, st);
+    const int rc = rb_cols(p, spec, fstride, ld2, nf, axis, dir, scale, nullptr, st);
     if (rc != 1) return rc;
   }
   return p->prec == GBOFDFT_F64 ? cols_t<double>(p, spec, fstride, ld2, nf, axis, dir, scale, st)
@@ -650,8 +680,7 @@ int gb_cols_conv(gbofdft_plan* p, void* spec, int64_t fstride, int ld2, int nf, 
   if (gb_use_ct()) {
     KerDesc k2 = kd;
     for (int f = 0; f < nf; ++f) k2.coef[f] = kd.coef[f] * scale;
-    const int rc = p->prec == GBOFDFT_F64 ? gb_ct_cols_f64(p, spec, fstride, ld2, nf, 0, -1, 1.0, &k2, st)
-                                          : gb_ct_cols_f32(p, spec, fstride, ld2, nf, 0, -1, 1.0, &k2, st);
+    const int rc = rb_cols(p, spec, fstride, ld2, nf, 0, -1, 1.0, &k2, st);
     if (rc != 1) return rc;
   }
   return p->prec == GBOFDFT_F64 ? cols_conv_t<double>(p, spec, fstride, ld2, nf, kd, scale, st)

@@ -9,11 +9,10 @@
 
 #include "fft_ct.cuh"
 #include "gkernels.cuh"
+#include "pass_common.cuh"
 #include "plan.h"
 
 namespace gbct {
-
-constexpr double kZero = 1e-30;
 
 template <typename F>
 __host__ inline bool ct_dispatch(int n, F&& f) {
@@ -64,18 +63,6 @@ template <typename T, int N> struct ColsCfg {     // columns per tile
 template <typename T, int N, bool CONV> constexpr int cols_minb() {
   if constexpr (CONV) return (sizeof(T) == 4 && N <= 128) ? GB_CT_CONV_MINB : 1;
   else return GB_CT_COLS_MINB;
-}
-
-// A scalar kernel parameter in both precisions, converted on the host: the
-// FP32 kernels then run without double->float conversions, which execute on
-// the FP64 pipe (a slow one on this part).
-struct Sc {
-  double d;
-  float f;
-  void set(double v) { d = v; f = (float)v; }
-};
-template <typename T> __device__ __forceinline__ T sc(const Sc& s) {
-  if constexpr (sizeof(T) == 8) return s.d; else return s.f;
 }
 
 // ---- pointwise functions -----------------------------------------------------
@@ -665,20 +652,6 @@ k_ct_cols(CtCols a) {
 }
 
 // ---- launchers -------------------------------------------------------------------
-// Raise a kernel's dynamic shared-memory limit once to the largest size it
-// has been launched with (keyed by kernel address and device).
-template <typename K> inline int ct_smem(K kern, size_t bytes) {
-  if (bytes <= 48 * 1024) return 0;
-  int dev = 0;
-  cudaGetDevice(&dev);
-  const void* key = reinterpret_cast<const void*>(kern);
-  if (gb_smem_granted(key, dev) >= (int)bytes) return 0;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-  if (e != cudaSuccess) return gb_set_error(GBOFDFT_ERR_CUDA, "smem attribute: %s", cudaGetErrorString(e));
-  gb_smem_grant(key, dev, (int)bytes);
-  return 0;
-}
-
 template <typename T, bool PM = false>
 int ct_rows_fwd(gbofdft_plan* p, const void* in, void* spec, int64_t fstride, int ld2, int nf, const int* ops,
                 double beta, double scale, cudaStream_t st, double rho0 = 0.0) {

@@ -1,0 +1,1160 @@
+// The FFT passes of a 3D grid on the register-blocked lines of fft_rb.cuh
+// (any axis length with prime factors up to 7; other lengths run in passes.cu).
+//
+// Layouts and semantics are those of passes.cu.  Per pass:
+//   k_rb_cols      one CTA transforms a tile of 16 (FP32) or 8 (FP64) columns =
+//                  128 contiguous bytes per line element.  The first stage
+//                  reads global memory into registers and the last one
+//                  writes it from registers, so a column crosses shared
+//                  memory once per pair of stages.  Tiles run over the columns
+//                  of all outer indices back to back, so a half spectrum of
+//                  n2/2 + 1 columns leaves no nearly empty last tile.
+//                  CONV: axis-0 forward, kernel multiply and the inverse's
+//                  first stage in the same registers.
+//   k_rb_rows_fwd  prologues, R2C of row pairs.
+//   k_rb_rows_inv  C2R of row pairs: the first stage reads the half spectrum
+//                  straight from global memory, the last one leaves every
+//                  field of a point with one thread, which runs the epilogue.
+#pragma once
+#include <math.h>
+#include <string.h>
+
+#include "fft_rb.cuh"
+#include "gkernels.cuh"
+#include "pass_common.cuh"
+#include "plan.h"
+
+// FP32 lengths with kernels of their own: the even 2, 3, 5, 7-smooth lengths
+// from 24 to 400 whose radices split into two stages of at most 25, and some
+// that need three
+#define GB_RB_LENGTHS_1(X) \
+  X(24, GB_RB_G(8), GB_RB_G(3)) X(28, GB_RB_G(4), GB_RB_G(7)) X(30, GB_RB_G(2, 3), GB_RB_G(5)) \
+  X(32, GB_RB_G(8), GB_RB_G(4)) X(36, GB_RB_G(4), GB_RB_G(3, 3)) X(40, GB_RB_G(8), GB_RB_G(5)) \
+  X(42, GB_RB_G(2, 3), GB_RB_G(7)) X(48, GB_RB_G(8), GB_RB_G(2, 3)) X(50, GB_RB_G(2, 5), GB_RB_G(5)) \
+  X(54, GB_RB_G(2, 3), GB_RB_G(3, 3)) X(56, GB_RB_G(8), GB_RB_G(7)) X(60, GB_RB_G(4, 3), GB_RB_G(5)) \
+  X(64, GB_RB_G(8), GB_RB_G(8)) X(70, GB_RB_G(2, 5), GB_RB_G(7)) X(72, GB_RB_G(8), GB_RB_G(3, 3)) \
+  X(80, GB_RB_G(8), GB_RB_G(2, 5)) X(84, GB_RB_G(4, 3), GB_RB_G(7)) X(90, GB_RB_G(2, 3), GB_RB_G(3, 5)) \
+  X(96, GB_RB_G(8), GB_RB_G(4, 3)) X(98, GB_RB_G(2, 7), GB_RB_G(7))
+#define GB_RB_LENGTHS_2(X) \
+  X(100, GB_RB_G(4, 5), GB_RB_G(5)) X(108, GB_RB_G(4, 3), GB_RB_G(3, 3)) X(112, GB_RB_G(8), GB_RB_G(2, 7)) \
+  X(120, GB_RB_G(8), GB_RB_G(3, 5)) X(126, GB_RB_G(2, 3, 3), GB_RB_G(7)) X(128, GB_RB_G(8), GB_RB_G(4, 4)) \
+  X(140, GB_RB_G(4, 5), GB_RB_G(7)) X(144, GB_RB_G(8, 2), GB_RB_G(3, 3)) \
+  X(150, GB_RB_G(2, 3), GB_RB_G(5, 5)) X(160, GB_RB_G(8), GB_RB_G(4, 5)) \
+  X(162, GB_RB_G(2, 3, 3), GB_RB_G(3, 3))
+#define GB_RB_LENGTHS_3(X) \
+  X(168, GB_RB_G(8), GB_RB_G(3, 7)) X(180, GB_RB_G(4, 3), GB_RB_G(3, 5)) X(192, GB_RB_G(8), GB_RB_G(8, 3)) \
+  X(200, GB_RB_G(8), GB_RB_G(5, 5)) X(216, GB_RB_G(8, 3), GB_RB_G(3, 3)) \
+  X(240, GB_RB_G(8, 2), GB_RB_G(3, 5)) X(250, GB_RB_G(2, 5), GB_RB_G(5, 5))
+#define GB_RB_LENGTHS_4(X) \
+  X(252, GB_RB_G(4, 3), GB_RB_G(3, 7)) X(270, GB_RB_G(2, 3, 3), GB_RB_G(3, 5)) \
+  X(300, GB_RB_G(4, 3), GB_RB_G(5, 5)) X(336, GB_RB_G(8, 2), GB_RB_G(3, 7)) \
+  X(378, GB_RB_G(2, 3, 3), GB_RB_G(3, 7)) X(400, GB_RB_G(8, 2), GB_RB_G(5, 5))
+#define GB_RB_LENGTHS3(X) \
+  X(196, GB_RB_G(4), GB_RB_G(7), GB_RB_G(7)) X(210, GB_RB_G(2, 3), GB_RB_G(5), GB_RB_G(7)) \
+  X(224, GB_RB_G(8), GB_RB_G(4), GB_RB_G(7)) X(256, GB_RB_G(8), GB_RB_G(8), GB_RB_G(4)) \
+  X(280, GB_RB_G(8), GB_RB_G(5), GB_RB_G(7)) X(288, GB_RB_G(8), GB_RB_G(4), GB_RB_G(3, 3)) \
+  X(320, GB_RB_G(8), GB_RB_G(8), GB_RB_G(5)) X(360, GB_RB_G(8), GB_RB_G(5), GB_RB_G(3, 3))
+
+#ifndef GB_RB_GROUP
+#define GB_RB_GROUP 0
+#endif
+#define GB_RB_CAT2(a, b) a##b
+#define GB_RB_CAT(a, b) GB_RB_CAT2(a, b)
+
+namespace gbrb {
+
+using gbct::Sc;
+using gbct::kZero;
+using gbct::sc;
+
+constexpr int kFields = 8;
+
+// element j of a line in shared memory: one complex value of padding per 128
+// bytes, so the stride-radix writes of a first stage spread over the banks
+template <typename T> __device__ __forceinline__ int sidx(int j) {
+  constexpr int S = sizeof(T) == 4 ? 4 : 3;
+  return j + (j >> S);
+}
+template <typename T> __host__ __device__ inline int line_pitch(int n) {
+  constexpr int S = sizeof(T) == 4 ? 4 : 3;
+  return n + (n >> S) + 1;
+}
+
+// ---- FP64 elementary functions from single-precision seeds -------------------
+// 1/x by two Newton steps (seed error 1e-7 -> 1e-14 -> below 1 ulp)
+__device__ __forceinline__ double rcp_nr(double x) {
+  double r = (double)(1.0f / (float)x);
+  r = fma(r, fma(-x, r, 1.0), r);
+  return fma(r, fma(-x, r, 1.0), r);
+}
+__device__ __forceinline__ float rcp_nr(float x) { return 1.0f / x; }
+
+// x^(-1/6), x in the float range: one third-order (Halley-type) step on the
+// seed, y (1 + r/6 + 7 r^2/72) with r = 1 - x y^6 (|r| < 1e-5, so the next term
+// is below 1e-16).  x^(-1/3) and x^(-1/2) are its square and cube: 9 FP64
+// operations for all of them, where separate Newton iterations for the two
+// took 25 (the FP64 pipe bounds the FP64 row passes).
+__device__ __forceinline__ double rroot6(double x) {
+  const double y = (double)rsqrtf(cbrtf((float)x));
+  const double y2 = y * y;
+  const double r = fma(-x, y2 * y2 * y2, 1.0);
+  return fma(y * r, fma(r, 7.0 / 72.0, 1.0 / 6.0), y);
+}
+
+// rho^(-1/3), rho^(-1/2) and (FP64) rho^(-1/6) of a positive density
+template <typename T> struct Roots { T z3, z2, y; };
+__device__ __forceinline__ Roots<float> roots(float x) { return Roots<float>{rcbrtf(x), rsqrtf(x), 0.0f}; }
+__device__ __forceinline__ Roots<double> roots(double x) {
+  const double y = rroot6(x), y2 = y * y;
+  return Roots<double>{y2, y2 * y, y};
+}
+__device__ __forceinline__ float sqrt_of(float x, const Roots<float>& r) { return x * r.z2; }
+// one more Newton step: the rounding of sqrt(rho) is what the G^2 kernel amplifies
+__device__ __forceinline__ double sqrt_of(double x, const Roots<double>& r) {
+  const double s = x * r.z2;
+  return fma(0.5 * r.z2, fma(-s, s, x), s);
+}
+// x^(5/6)
+__device__ __forceinline__ float pow56(float x, const Roots<float>& r) { return (x * r.z2) * (x * r.z3 * r.z3); }
+__device__ __forceinline__ double pow56(double x, const Roots<double>& r) { return x * r.y; }
+
+// ---- forward rows ---------------------------------------------------------------
+struct RowsFwd {
+  const void* in;
+  void* out;
+  int64_t fstride;
+  int nrows, n2h, ld2, nf, lp;
+  int op[kFields];
+  int b56, rsq;           // rsq: sqrt(rho) as rho rsqrt(rho) (FP32)
+  Sc beta, half, rho0, inv0;
+  RbAxis ax;
+  FastDiv dn, dnh;
+  const void* tw;
+};
+
+template <typename T>
+__device__ __noinline__ T pow_general(T x, T b) { return pow(x, b); }
+template <typename T>
+__device__ __noinline__ T sqrt_call(T x) { return sqrt(x); }
+
+// Prologues of the forward rows.  A kernel per kind: a plain transform holds
+// none of the root arithmetic (the compiler would compute it ahead of the
+// branch, at 12 FP64 operations a point).
+enum { PK_PLAIN = 0, PK_ROOTS = 1, PK_GENERAL = 2 };
+
+// the values of one density that the derived fields are made of
+template <typename T> struct Derived { T rho, sq, b, u; };
+template <typename T, int KIND>
+__device__ __forceinline__ Derived<T> derived(const RowsFwd& a, T rho) {
+  Derived<T> d;
+  d.rho = d.sq = d.b = d.u = rho;
+  if constexpr (KIND != PK_PLAIN) {
+    const T kz = (T)kZero;
+    const T rc = rho > kz ? rho : kz;
+    const Roots<T> r = roots(rc);
+    d.sq = sqrt_of(rc, r);
+    if (sizeof(T) == 4 && !a.rsq) d.sq = sqrt(rc);
+    if (rho > (T)0 && rho < kz) d.sq = sqrt_call<T>(rho);
+    if constexpr (KIND == PK_ROOTS) {
+      d.b = pow56(rc, r);
+    } else {
+      d.b = pow_general<T>(rc, sc<T>(a.beta));
+      d.u = (rc - sc<T>(a.rho0)) * sc<T>(a.inv0);
+    }
+  }
+  return d;
+}
+template <typename T, int KIND>
+__device__ __forceinline__ T field_of(int op, const Derived<T>& d) {
+  if constexpr (KIND == PK_PLAIN) return d.rho;
+  T v = d.rho;
+  if (op == OP_SQRT) v = d.sq;
+  else if (op == OP_POWB || op == OP_WGC0) v = d.b;
+  if constexpr (KIND == PK_GENERAL) {
+    if (op == OP_WGC1) v = d.u * d.b;
+    else if (op == OP_WGC2) v = d.u * d.u * d.b;
+  }
+  return v;
+}
+// one derived field alone (FP32: the roots of a field cost less than passing
+// every field through shared memory)
+template <typename T>
+__device__ __forceinline__ T field_direct(int op, T rho, bool rsq) {
+  const T kz = (T)kZero;
+  if (op == OP_SQRT) {
+    const T rc = rho > (T)0 ? rho : kz;
+    return rsq && rc >= kz ? rc * rsqrtf(rc) : sqrtf(rc);
+  }
+  if (op == OP_POWB) {
+    const T rc = rho < kz ? kz : rho;
+    return pow56(rc, roots(rc));
+  }
+  return rho;
+}
+
+// transform of all lines of the CTA between two shared buffers (line pitch
+// ls); returns the buffer with the result.  FIRST = false: the first stage's
+// results are in b already.
+template <int DIR, bool FIRST, typename T, typename AX>
+__device__ __forceinline__ cpx<T>* lines(cpx<T>* a, cpx<T>* b, int ls, int nl, const AX& ax,
+                                         const cpx<T>* __restrict__ tw) {
+  const int tid = threadIdx.x, nthr = blockDim.x, n = ax.n();
+  if constexpr (FIRST) {
+    ax.first([&](auto rc) {
+      constexpr int R = decltype(rc)::R;
+      const int nb = ax.nbf();
+      for (int t0 = tid; t0 < nl * nb; t0 += nthr) {
+        const int l = ax.div_nbf(t0), i = t0 - l * nb;
+        cpx<T> u[R];
+        const cpx<T>* src = a + l * ls;
+#pragma unroll
+        for (int t = 0; t < R; ++t) u[t] = src[sidx<T>(i + t * nb)];
+        stage_first<DIR, T>(rc, u, tw, n);
+        cpx<T>* dst = b + l * ls;
+#pragma unroll
+        for (int t = 0; t < R; ++t) dst[sidx<T>(i * R + t)] = u[t];
+      }
+    });
+  }
+  __syncthreads();
+  cpx<T>* x = a;
+  a = b;
+  b = x;
+  ax.middle([&](auto rc, auto nb, auto p, auto div_nb, auto div_p) {
+    constexpr int R = decltype(rc)::R;
+    for (int t0 = tid; t0 < nl * nb; t0 += nthr) {
+      const int l = div_nb(t0), i = t0 - l * nb;
+      const int k = i - p * div_p(i);
+      cpx<T> u[R];
+      load_stage<DIR, T>(rc, u, a + l * ls, tw, i, k, nb, p, n, sidx<T>);
+      cpx<T>* dst = b + l * ls;
+      const int j0 = (i - k) * R + k;
+#pragma unroll
+      for (int t = 0; t < R; ++t) dst[sidx<T>(j0 + t * p)] = u[t];
+    }
+    __syncthreads();
+    cpx<T>* y = a;
+    a = b;
+    b = y;
+  });
+  if (ax.nst() < 2) return a;
+  ax.last([&](auto rc) {
+    constexpr int R = decltype(rc)::R;
+    const int nb = ax.nbl();
+    for (int t0 = tid; t0 < nl * nb; t0 += nthr) {
+      const int l = ax.div_nbl(t0), i = t0 - l * nb;
+      cpx<T> u[R];
+      // the last stage writes the elements that it read
+      cpx<T>* x = a + l * ls;
+      load_stage<DIR, T>(rc, u, x, tw, i, i, nb, nb, n, sidx<T>);
+#pragma unroll
+      for (int t = 0; t < R; ++t) x[sidx<T>(i + t * nb)] = u[t];
+    }
+  });
+  __syncthreads();
+  return a;
+}
+
+// forward rows whose first stage reads global memory: FP32, fields of rho,
+// sqrt(rho) and rho^(5/6), a first radix whose inputs fit in registers beside
+// a field's butterfly
+template <typename T, int KIND, typename AX> constexpr bool direct_rows() {
+  if constexpr (sizeof(T) == 4 && AX::kFixed && KIND != PK_GENERAL)
+    return AX::n() / AX::nbf() <= (KIND == PK_PLAIN ? 16 : 12);
+  else return false;
+}
+template <typename T, int KIND, typename AX> constexpr bool kDirect = direct_rows<T, KIND, AX>();
+// ... and that then needs one shared buffer only (two stages)
+template <typename T, int KIND, typename AX> constexpr bool one_buffer() {
+  if constexpr (direct_rows<T, KIND, AX>()) return AX::nst() == 2;
+  else return false;
+}
+
+template <typename T, typename AX = AxRun<T>> struct RowCta {
+  static constexpr int NT = sizeof(T) == 4 ? 128 : 96;      // threads of a row CTA, at most
+  static constexpr int MINB = sizeof(T) == 8 || !AX::kFixed ? 4 : 7;   // resident CTAs per SM to allocate registers for
+};
+
+template <typename T, int KIND, typename AX>
+__global__ void __launch_bounds__(RowCta<T>::NT, (RowCta<T, AX>::MINB)) k_rb_rows_fwd(const __grid_constant__ RowsFwd a) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const AX ax(a.ax);
+  const int n = ax.n(), lp = a.lp, ls = line_pitch<T>(n), nl = a.nf * lp;
+  cpx<T>* A = reinterpret_cast<cpx<T>*>(smem_raw);
+  cpx<T>* B = one_buffer<T, KIND, AX>() ? A : A + nl * ls;
+  const int tid = threadIdx.x, nthr = blockDim.x;
+  const int base = blockIdx.x * 2 * lp;
+  const T* in = reinterpret_cast<const T*>(a.in);
+  const cpx<T>* tw = reinterpret_cast<const cpx<T>*>(a.tw);
+  cpx<T>* res;
+  if constexpr (kDirect<T, KIND, AX>) {
+    // FP32: the first stage reads the rows from global memory and derives its
+    // field in registers
+    const bool rsq = a.rsq != 0;
+    ax.first([&](auto rc) {
+      constexpr int R = decltype(rc)::R;
+      constexpr int nb = AX::nbf();
+      for (int t0 = tid; t0 < lp * nb; t0 += nthr) {
+        const int l = ax.div_nbf(t0), i = t0 - l * nb;
+        const int ra = base + 2 * l;
+        const T* src = in + (int64_t)ra * n + i;
+        T x0[R], x1[R];
+#pragma unroll
+        for (int t = 0; t < R; ++t) {
+          x0[t] = ra < a.nrows ? __ldg(src + t * nb) : (T)0;
+          x1[t] = ra + 1 < a.nrows ? __ldg(src + n + t * nb) : (T)0;
+        }
+        for (int f = 0; f < a.nf; ++f) {
+          const int op = a.op[f];
+          cpx<T> u[R];
+          if (op == OP_RHO || KIND == PK_PLAIN) {
+#pragma unroll
+            for (int t = 0; t < R; ++t) u[t] = cpx<T>{x0[t], x1[t]};
+          } else if (op == OP_SQRT) {
+#pragma unroll
+            for (int t = 0; t < R; ++t) u[t] = cpx<T>{field_direct<T>(OP_SQRT, x0[t], rsq), field_direct<T>(OP_SQRT, x1[t], rsq)};
+          } else {
+#pragma unroll
+            for (int t = 0; t < R; ++t) u[t] = cpx<T>{field_direct<T>(OP_POWB, x0[t], rsq), field_direct<T>(OP_POWB, x1[t], rsq)};
+          }
+          stage_first<-1, T>(rc, u, tw, AX::n());
+          cpx<T>* dst = B + (f * lp + l) * ls;
+#pragma unroll
+          for (int t = 0; t < R; ++t) dst[sidx<T>(i * R + t)] = u[t];
+        }
+      }
+    });
+    res = lines<-1, false, T>(A, B, ls, nl, ax, tw);
+  } else {
+#pragma unroll 2
+    for (int idx = tid; idx < lp * n; idx += nthr) {
+      const int l = AX::kFixed ? idx / n : (int)a.dn.div(idx), j = idx - l * n;
+      const int ra = base + 2 * l;
+      const bool ok0 = ra < a.nrows, ok1 = ra + 1 < a.nrows;
+      const T* src = in + (int64_t)ra * n + j;
+      const Derived<T> d0 = derived<T, KIND>(a, ok0 ? __ldg(src) : (T)0);
+      const Derived<T> d1 = derived<T, KIND>(a, ok1 ? __ldg(src + n) : (T)0);
+      cpx<T>* o = A + l * ls + sidx<T>(j);
+      for (int f = 0; f < a.nf; ++f)
+        o[f * lp * ls] = cpx<T>{field_of<T, KIND>(a.op[f], d0), field_of<T, KIND>(a.op[f], d1)};
+    }
+    __syncthreads();
+    res = lines<-1, true, T>(A, B, ls, nl, ax, tw);
+  }
+  cpx<T>* out = reinterpret_cast<cpx<T>*>(a.out);
+  const T half = sc<T>(a.half);
+  const int nh = AX::kFixed ? n / 2 + 1 : a.n2h;
+  for (int f = 0; f < a.nf; ++f) {
+    cpx<T>* o = out + f * a.fstride;
+    const cpx<T>* src = res + f * lp * ls;
+    for (int idx = tid; idx < lp * nh; idx += nthr) {
+      const int l = AX::kFixed ? idx / nh : (int)a.dnh.div(idx), k = idx - l * nh;
+      const int ra = base + 2 * l;
+      if (ra >= a.nrows) continue;
+      const cpx<T> Z = src[l * ls + sidx<T>(k)];
+      const cpx<T> Zc = src[l * ls + sidx<T>(k == 0 ? 0 : n - k)];
+      cpx<T>* q = o + (int64_t)ra * a.ld2 + k;
+      cpx<T> va = {Z.x + Zc.x, Z.y - Zc.y}, vb = {Z.y + Zc.y, Zc.x - Z.x};
+      if (half != (T)1) {
+        va = c_scale(va, half);
+        vb = c_scale(vb, half);
+      }
+      q[0] = va;
+      if (ra + 1 < a.nrows) q[a.ld2] = vb;
+    }
+  }
+}
+
+// ---- inverse rows ----------------------------------------------------------------
+struct RowsInv {
+  const void* in;
+  int64_t fstride;
+  int nrows, n2h, ld2, nf, lp;
+  RbAxis ax;
+  const void* tw;
+  void* out;
+  int64_t ostride;
+  Sc scale;
+  EvalDesc ev;
+  Sc tf_v, tf_e, vw_y, two_alpha, inv_two_alpha, wt_beta;
+  int b56;
+  const void* rho;
+  const void* vloc;
+  void* pot;
+  double* partials;
+};
+
+// a call, so that the compiler cannot compute the logarithm of the r_s < 1
+// branch for every point (35 FP64 operations)
+static __device__ __noinline__ double log_call(double x) { return log(x); }
+static __device__ __forceinline__ float log_call(float x) { return logf(x); }
+
+// Perdew-Zunger 1981 LDA at rho > 0 given its roots: potential and (want_e)
+// energy per particle
+template <typename T>
+__device__ __forceinline__ void pz_lda(T rho, const Roots<T>& r, T& eps, T& pot, bool want_e) {
+  const T a = (T)0.0311, b = (T)-0.048, c = (T)0.0020, d = (T)-0.0116;
+  const T g = (T)-0.1423, b1 = (T)1.0529, b2 = (T)0.3334;
+  const T cx = (T)0.98474502184269654115;                 // (3/pi)^(1/3)
+  const T rc = rho * r.z3 * r.z3;
+  const T rs = (T)0.62035049089940001667 * r.z3;          // (3/(4 pi))^(1/3) / rho^(1/3)
+  pot = -cx * rc;
+  eps = (T)(-0.75) * cx * rc;
+  if (rs < (T)1) {
+    const T lr = log_call(rs);
+    pot += lr * (a + (T)(2.0 / 3.0) * c * rs) + b - (T)(1.0 / 3.0) * a + (T)(1.0 / 3.0) * ((T)2 * d - c) * rs;
+    if (want_e) eps += a * lr + b + c * rs * lr + d * rs;
+  } else {
+    T sq;
+    if constexpr (sizeof(T) == 8) sq = 0.78762331789974326286 * r.y;   // sqrt(0.62035...) rho^(-1/6)
+    else sq = sqrt(rs);
+    const T inv = rcp_nr((T)1 + b1 * sq + b2 * rs);
+    pot += (g + ((T)(7.0 / 6.0) * g * b1) * sq + ((T)(4.0 / 3.0) * g * b2 * rs)) * (inv * inv);
+    if (want_e) eps += g * inv;
+  }
+}
+
+// the pointwise terms at rho <= 1e-30 (the reference's clamps), out of line
+template <typename T>
+__device__ __noinline__ void point_tiny(const RowsInv& a, T rho, T w, T kc, T vh, T vl, bool want_e, T* pot_out,
+                                        T* es) {
+  const EvalDesc& ev = a.ev;
+  T pot = (T)0;
+  const T kz = (T)kZero;
+  if (ev.tf) {
+    pot += sc<T>(a.tf_v) * cbrt(rho * rho);
+    if (want_e) {
+      T r5 = rho * rho;
+      r5 = r5 * rho; r5 = r5 * rho; r5 = r5 * rho;
+      es[0] += cbrt(r5) * sc<T>(a.tf_e);
+    }
+  }
+  if (ev.vw) {
+    const T v = (T)0.5 * w * (rho > (T)0 ? (T)1 / fmax(sqrt(rho), kz) : (T)1e15);
+    pot += v * sc<T>(a.vw_y);
+    if (want_e && rho > (T)0) es[1] += rho * v * sc<T>(a.vw_y);
+  }
+  if (ev.wt) {
+    const T rb = a.b56 ? sqrt(kz) * cbrt(kz) / kz : pow(kz, sc<T>(a.wt_beta)) / kz;
+    const T v = sc<T>(a.two_alpha) * rb * kc;
+    pot += v;
+    if (want_e) es[2] += v * rho * sc<T>(a.inv_two_alpha);
+  }
+  if (ev.xc) {
+    const T cx = (T)0.98474502184269654115;
+    T rc = cbrt(rho);
+    if (rc < kz) rc = kz;
+    const T inv = (T)1 / rc;
+    T vx, eps;
+    Roots<T> r;
+    r.z3 = inv;
+    r.z2 = (T)0;
+    r.y = sqrt(inv);
+    // pz_lda forms rho^(1/3) as rho z3^2; here it is the clamped rc
+    pz_lda<T>(rc * rc * rc, r, eps, vx, want_e);
+    vx += cx * (rc * rc * rc * inv * inv) - cx * rc;
+    eps += (T)0.75 * cx * (rc * rc * rc * inv * inv) - (T)0.75 * cx * rc;
+    pot += vx;
+    if (want_e) es[3] += eps * rho;
+  }
+  if (ev.hartree) {
+    pot += vh;
+    if (want_e) es[4] += (T)0.5 * vh * rho;
+  }
+  if (ev.pp) {
+    pot += vl;
+    if (want_e) es[5] += vl * rho;
+  }
+  *pot_out = pot;
+}
+
+// potential at one point from its density and convolution results; energy
+// densities added to es
+template <typename T, bool WANT_E>
+__device__ __forceinline__ T point(const RowsInv& a, T rho, T w, T kc, T vh, T vl, T* es) {
+  const EvalDesc& ev = a.ev;
+  if (!(rho > (T)kZero)) {
+    T p;
+    T e6[6] = {0, 0, 0, 0, 0, 0};
+    point_tiny<T>(a, rho, w, kc, vh, vl, WANT_E, &p, e6);
+    if constexpr (WANT_E) {
+#pragma unroll
+      for (int q = 0; q < 6; ++q) es[q] += e6[q];
+    }
+    return p;
+  }
+  const Roots<T> r = roots(rho);
+  T pot = (T)0;
+  if (ev.tf) {
+    const T r23 = rho * r.z3;                           // rho^(2/3)
+    pot += sc<T>(a.tf_v) * r23;
+    if (WANT_E) es[0] += rho * r23 * sc<T>(a.tf_e);
+  }
+  if (ev.vw) {
+    const T v = (T)0.5 * w * r.z2 * sc<T>(a.vw_y);
+    pot += v;
+    if (WANT_E) es[1] += rho * v;
+  }
+  if (ev.wt) {
+    // rho^(beta - 1)
+    const T rb = a.b56 ? (sizeof(T) == 8 ? r.y : rho * r.z3 * r.z3 * r.z2) : pow_general<T>(rho, sc<T>(a.wt_beta)) / rho;
+    const T v = sc<T>(a.two_alpha) * rb * kc;
+    pot += v;
+    if (WANT_E) es[2] += v * rho * sc<T>(a.inv_two_alpha);
+  }
+  if (ev.xc) {
+    T eps, vx;
+    pz_lda<T>(rho, r, eps, vx, WANT_E);
+    pot += vx;
+    if (WANT_E) es[3] += eps * rho;
+  }
+  if (ev.hartree) {
+    pot += vh;
+    if (WANT_E) es[4] += (T)0.5 * vh * rho;
+  }
+  if (ev.pp) {
+    pot += vl;
+    if (WANT_E) es[5] += vl * rho;
+  }
+  return pot;
+}
+
+enum { RI_STORE = 0, RI_EVAL = 1, RI_EVAL_E = 2 };
+
+template <typename T, int MODE, typename AX>
+__global__ void __launch_bounds__(RowCta<T>::NT, (RowCta<T, AX>::MINB)) k_rb_rows_inv(const __grid_constant__ RowsInv a) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const AX ax(a.ax);
+  const int n = ax.n(), lp = a.lp, ls = line_pitch<T>(n), nl = a.nf * lp;
+  cpx<T>* A = reinterpret_cast<cpx<T>*>(smem_raw);
+  cpx<T>* B = A + nl * ls;                               // used by three or more stages
+  const int tid = threadIdx.x, nthr = blockDim.x;
+  const int base = blockIdx.x * 2 * lp;
+  const cpx<T>* in = reinterpret_cast<const cpx<T>*>(a.in);
+  const cpx<T>* tw = reinterpret_cast<const cpx<T>*>(a.tw);
+  // first stage: line element j of a row pair is X_a[j] + i X_b[j] for
+  // j <= n/2 and the conjugates' combination above
+  ax.first([&](auto rc) {
+    constexpr int R = decltype(rc)::R;
+    const int nb = ax.nbf();
+    for (int t0 = tid; t0 < nl * nb; t0 += nthr) {
+      const int line = ax.div_nbf(t0), i = t0 - line * nb;
+      const int f = line / lp, l = line - f * lp;
+      const int ra = base + 2 * l;
+      cpx<T> u[R];
+      const cpx<T>* pa = in + f * a.fstride + (int64_t)ra * a.ld2;
+      const bool ok0 = ra < a.nrows, ok1 = ra + 1 < a.nrows;
+#pragma unroll
+      for (int t = 0; t < R; ++t) {
+        const int j = i + t * nb;
+        // j > n/2, and j in {0, n/2}, whose imaginary parts do not count
+        bool up, edge;
+        if constexpr (R % 2 == 0) {
+          up = t > R / 2 || (t == R / 2 && i > 0);
+          edge = t % (R / 2) == 0 && i == 0;
+        } else {
+          up = 2 * j > n;
+          edge = j == 0 || 2 * j == n;
+        }
+        const int k = up ? n - j : j;
+        cpx<T> va = {(T)0, (T)0}, vb = {(T)0, (T)0};
+        if (ok0) va = pa[k];
+        if (ok1) vb = pa[a.ld2 + k];
+        if (edge) { va.y = (T)0; vb.y = (T)0; }
+        u[t] = up ? cpx<T>{va.x + vb.y, vb.x - va.y} : cpx<T>{va.x - vb.y, va.y + vb.x};
+      }
+      stage_first<1, T>(rc, u, tw, n);
+      cpx<T>* dst = A + line * ls;
+#pragma unroll
+      for (int t = 0; t < R; ++t) dst[sidx<T>(i * R + t)] = u[t];
+    }
+  });
+  __syncthreads();
+  cpx<T>* cur = A;
+  cpx<T>* oth = B;
+  ax.middle([&](auto rc, auto nb, auto p, auto div_nb, auto div_p) {
+    constexpr int R = decltype(rc)::R;
+    for (int t0 = tid; t0 < nl * nb; t0 += nthr) {
+      const int line = div_nb(t0), i = t0 - line * nb;
+      const int k = i - p * div_p(i);
+      cpx<T> u[R];
+      load_stage<1, T>(rc, u, cur + line * ls, tw, i, k, nb, p, n, sidx<T>);
+      cpx<T>* dst = oth + line * ls;
+      const int j0 = (i - k) * R + k;
+#pragma unroll
+      for (int t = 0; t < R; ++t) dst[sidx<T>(j0 + t * p)] = u[t];
+    }
+    __syncthreads();
+    cpx<T>* x = cur;
+    cur = oth;
+    oth = x;
+  });
+  // last stage: a thread transforms butterfly i of every field of a row pair
+  // in place (its own elements), so the points i + t nb are complete in it
+  const int nb = ax.nbl(), rl = ax.rl();
+  T es[6] = {0, 0, 0, 0, 0, 0};
+  for (int t0 = tid; t0 < lp * nb; t0 += nthr) {
+    const int l = ax.div_nbl(t0), i = t0 - l * nb;
+    const int ra = base + 2 * l;
+    if (ra >= a.nrows) continue;
+    const bool ok1 = ra + 1 < a.nrows;
+    if (ax.nst() > 1) {
+      ax.last([&](auto rc) {
+        constexpr int R = decltype(rc)::R;
+        for (int f = 0; f < a.nf; ++f) {
+          cpx<T>* src = cur + (f * lp + l) * ls;
+          cpx<T> u[R];
+          load_stage<1, T>(rc, u, src, tw, i, i, nb, nb, n, sidx<T>);
+#pragma unroll
+          for (int t = 0; t < R; ++t) src[sidx<T>(i + t * nb)] = u[t];
+        }
+      });
+    }
+    const cpx<T>* fld = cur + l * ls;
+    if constexpr (MODE == RI_STORE) {
+      T* out = reinterpret_cast<T*>(a.out);
+      const T scl = sc<T>(a.scale);
+      for (int f = 0; f < a.nf; ++f) {
+        T* o = out + f * a.ostride + (int64_t)ra * n + i;
+        for (int t = 0; t < rl; ++t) {
+          const cpx<T> z = fld[f * lp * ls + sidx<T>(i + t * nb)];
+          o[t * nb] = z.x * scl;
+          if (ok1) o[t * nb + n] = z.y * scl;
+        }
+      }
+    } else {
+      const EvalDesc& ev = a.ev;
+      const int64_t g0 = (int64_t)ra * n + i;
+      const T* rp = reinterpret_cast<const T*>(a.rho) + g0;
+      const T* vp = reinterpret_cast<const T*>(a.vloc) + g0;
+      T* pp = reinterpret_cast<T*>(a.pot) + g0;
+      const int fs = lp * ls;
+      // density and v_loc of the next point pair are in flight while this
+      // one's terms are formed
+      T r0 = __ldg(rp), r1 = ok1 ? __ldg(rp + n) : (T)1, v0 = (T)0, v1 = (T)0;
+      if (ev.pp) {
+        v0 = __ldg(vp);
+        if (ok1) v1 = __ldg(vp + n);
+      }
+#pragma unroll 1
+      for (int t = 0; t < rl; ++t) {
+        const int j = t * nb;
+        const int o = sidx<T>(i + j);
+        T nr0 = (T)1, nr1 = (T)1, nv0 = (T)0, nv1 = (T)0;
+        if (t + 1 < rl) {
+          nr0 = __ldg(rp + j + nb);
+          if (ok1) nr1 = __ldg(rp + j + nb + n);
+          if (ev.pp) {
+            nv0 = __ldg(vp + j + nb);
+            if (ok1) nv1 = __ldg(vp + j + nb + n);
+          }
+        }
+        cpx<T> w = {(T)0, (T)0}, kc = {(T)0, (T)0}, vh = {(T)0, (T)0};
+        if (ev.vw) w = fld[ev.slot_vw * fs + o];
+        if (ev.wt) kc = fld[ev.slot_wt * fs + o];
+        if (ev.hartree) vh = fld[ev.slot_h * fs + o];
+        if constexpr (sizeof(T) == 8) {
+          if (ev.cout) {
+            // copy of the convolution results (delta-evaluation reference)
+            T* c = reinterpret_cast<T*>(ev.cout) + g0 + j;
+            if (ev.vw) { c[ev.slot_vw * ev.cstride] = w.x; if (ok1) c[ev.slot_vw * ev.cstride + n] = w.y; }
+            if (ev.wt) { c[ev.slot_wt * ev.cstride] = kc.x; if (ok1) c[ev.slot_wt * ev.cstride + n] = kc.y; }
+            if (ev.hartree) { c[ev.slot_h * ev.cstride] = vh.x; if (ok1) c[ev.slot_h * ev.cstride + n] = vh.y; }
+          }
+        }
+        constexpr bool E = MODE == RI_EVAL_E;
+        pp[j] = point<T, E>(a, r0, w.x, kc.x, vh.x, v0, es);
+        if (ok1) pp[j + n] = point<T, E>(a, r1, w.y, kc.y, vh.y, v1, es);
+        r0 = nr0;
+        r1 = nr1;
+        v0 = nv0;
+        v1 = nv1;
+      }
+    }
+  }
+  if constexpr (MODE != RI_EVAL_E) return;
+  __shared__ double red[8][6];
+  const int lane = tid & 31, warp = tid >> 5;
+#pragma unroll
+  for (int c = 0; c < 6; ++c) {
+    const double v = warp_sum((double)es[c]);
+    if (lane == 0) red[warp][c] = v;
+  }
+  __syncthreads();
+  if (tid < 6) {
+    KSum t;
+    t.init();
+    for (int w = 0; w < (nthr + 31) / 32; ++w) t.add(red[w][tid]);
+    a.partials[(int64_t)blockIdx.x * GB_NE + tid] = t.value();
+  }
+}
+
+// ---- columns -------------------------------------------------------------------
+struct Cols {
+  void* data;
+  int64_t fstride, stride, ostride;
+  unsigned ncol;          // columns over all outer indices (pitch ld2 each)
+  int n2h;
+  FastDiv dld;
+  RbAxis ax, inv;         // the axis; the same radices in reverse order (CONV)
+  const void* tw;
+  Sc scale;
+  Sc coef[GB_MAX_FIELDS];
+  Sc bg[9];
+  int type[GB_MAX_FIELDS];
+  const void* arr[GB_MAX_FIELDS];
+  int n0, n1, n2, full;
+};
+
+template <typename T> struct ColTile { static constexpr int TB = 128 / (2 * (int)sizeof(T)); };
+
+// reciprocal-space kernel along one axis-0 column (i1, k2)
+template <typename T> struct ColKernel {
+  T b0, b1, b2;           // axis-0 reciprocal vector
+  T ux, uy, uz;           // m1 b1 + m2 b2
+  T px, py, pz;           // the same at the conjugate partner (-i1, -k2)
+  int sym;                // 0: no partner average, 1: at i0 = n0/2, 2: at every i0
+  int n0;
+
+  __device__ __forceinline__ void init(const Cols& a, int i1, int k2) {
+    n0 = a.n0;
+    const bool ny1 = (a.n1 & 1) == 0 && 2 * i1 == a.n1, ny2 = (a.n2 & 1) == 0 && 2 * k2 == a.n2;
+    const T m1 = (T)gbk::ffreq(i1, a.n1), m2 = (T)(a.full ? gbk::ffreq(k2, a.n2) : k2);
+    const T q1 = ny1 ? m1 : -m1, q2 = a.full ? (ny2 ? m2 : -m2) : m2;
+    b0 = sc<T>(a.bg[0]); b1 = sc<T>(a.bg[1]); b2 = sc<T>(a.bg[2]);
+    ux = m1 * sc<T>(a.bg[3]) + m2 * sc<T>(a.bg[6]);
+    uy = m1 * sc<T>(a.bg[4]) + m2 * sc<T>(a.bg[7]);
+    uz = m1 * sc<T>(a.bg[5]) + m2 * sc<T>(a.bg[8]);
+    px = q1 * sc<T>(a.bg[3]) + q2 * sc<T>(a.bg[6]);
+    py = q1 * sc<T>(a.bg[4]) + q2 * sc<T>(a.bg[7]);
+    pz = q1 * sc<T>(a.bg[5]) + q2 * sc<T>(a.bg[8]);
+    const bool plane = a.full || k2 == 0 || ny2;
+    sym = plane ? ((ny1 || (a.full && ny2)) ? 2 : 1) : 0;
+  }
+  static __device__ __forceinline__ T gg(T x, T y, T z) { return x * x + y * y + z * z; }
+  static __device__ __forceinline__ T val(bool hart, T g) {
+    if (!hart) return g;
+    return g > (T)0 ? (T)(4.0 * 3.14159265358979323846) * rcp_nr(g) : (T)0;
+  }
+  // K at axis-0 index j, averaged with the conjugate partner's on Nyquist planes
+  __device__ __forceinline__ T at(bool hart, int j) const {
+    const T m0 = (T)gbk::ffreq(j, n0);
+    T k = val(hart, gg(m0 * b0 + ux, m0 * b1 + uy, m0 * b2 + uz));
+    const bool ny0 = 2 * j == n0;
+    if (sym == 2 || (sym == 1 && ny0)) {
+      const T q0 = ny0 ? m0 : -m0;
+      k = (k + val(hart, gg(q0 * b0 + px, q0 * b1 + py, q0 * b2 + pz))) * (T)0.5;
+    }
+    return k;
+  }
+};
+
+template <typename T, int DIR, bool CONV, typename AX, typename AXI>
+__global__ void __launch_bounds__(sizeof(T) == 4 ? 400 : 256) k_rb_cols(const __grid_constant__ Cols a) {
+  constexpr int TB = ColTile<T>::TB;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const AX ax(a.ax);
+  const AXI axi(a.inv);
+  const int n = ax.n(), nst = ax.nst();
+  cpx<T>* A = reinterpret_cast<cpx<T>*>(smem_raw);
+  cpx<T>* B = A + n * TB;
+  const int c = threadIdx.x % TB, i0 = threadIdx.x / TB, ni = blockDim.x / TB;
+  const unsigned col = blockIdx.x * TB + c;
+  const int outer = a.dld.div(col), k2 = col - outer * a.dld.d;
+  const bool ok = col < a.ncol && k2 < a.n2h;
+  const int f = blockIdx.y;
+  cpx<T>* g = reinterpret_cast<cpx<T>*>(a.data) + f * a.fstride + outer * a.ostride + k2;
+  const cpx<T>* tw = reinterpret_cast<const cpx<T>*>(a.tw);
+  const int64_t st = a.stride;
+  ColKernel<T> ker;
+  int type = KER_NONE;
+  T coef = (T)1;
+  const T* karr = nullptr;
+  if constexpr (CONV) {
+    type = a.type[f];
+    coef = sc<T>(a.coef[f]);
+    if (type == KER_HARTREE || type == KER_G2) ker.init(a, outer, k2);
+    // the API table layout [n0][n1][n2h]
+    if (type == KER_ARRAY) karr = reinterpret_cast<const T*>(a.arr[f]) + (int64_t)outer * a.n2h + k2;
+  }
+  const int64_t kst = (int64_t)a.n1 * a.n2h;
+  auto kmul = [&](int j, cpx<T> v) {
+    T k = (T)1;
+    if (type == KER_ARRAY) k = ok ? __ldg(karr + j * kst) : (T)0;
+    else if (type != KER_NONE) k = ker.at(type == KER_HARTREE, j);
+    return c_scale(v, k * coef);
+  };
+  const T scl = sc<T>(a.scale);
+  constexpr int D0 = CONV ? -1 : DIR;
+  if (nst == 1) {
+    if (i0 > 0) return;
+    ax.first([&](auto rc) {
+      constexpr int R = decltype(rc)::R;
+      cpx<T> u[R];
+#pragma unroll
+      for (int t = 0; t < R; ++t) u[t] = ok ? g[t * st] : cpx<T>{(T)0, (T)0};
+      stage_first<D0, T>(rc, u, tw, n);
+      if constexpr (CONV) {
+#pragma unroll
+        for (int t = 0; t < R; ++t) u[t] = kmul(t, u[t]);
+        stage_first<1, T>(rc, u, tw, n);
+      }
+      if (ok) {
+#pragma unroll
+        for (int t = 0; t < R; ++t) g[t * st] = c_scale(u[t], scl);
+      }
+    });
+    return;
+  }
+  auto sx = [&](int j) { return j * TB + c; };
+  ax.first([&](auto rc) {
+    constexpr int R = decltype(rc)::R;
+    const int nb = ax.nbf();
+    for (int i = i0; i < nb; i += ni) {
+      cpx<T> u[R];
+#pragma unroll
+      for (int t = 0; t < R; ++t) u[t] = ok ? g[(i + t * nb) * st] : cpx<T>{(T)0, (T)0};
+      stage_first<D0, T>(rc, u, tw, n);
+#pragma unroll
+      for (int t = 0; t < R; ++t) A[sx(i * R + t)] = u[t];
+    }
+  });
+  __syncthreads();
+  cpx<T>* cur = A;
+  cpx<T>* oth = B;
+  auto middle = [&](const auto& x, auto dir) {
+    constexpr int D = decltype(dir)::value;
+    x.middle([&](auto rc, auto nb, auto p, auto, auto div_p) {
+      constexpr int R = decltype(rc)::R;
+      for (int i = i0; i < nb; i += ni) {
+        const int k = i - p * div_p(i);
+        cpx<T> u[R];
+        load_stage<D, T>(rc, u, cur, tw, i, k, nb, p, n, sx);
+        const int j0 = (i - k) * R + k;
+#pragma unroll
+        for (int t = 0; t < R; ++t) oth[sx(j0 + t * p)] = u[t];
+      }
+      __syncthreads();
+      cpx<T>* y = cur;
+      cur = oth;
+      oth = y;
+    });
+  };
+  middle(ax, std::integral_constant<int, D0>{});
+  ax.last([&](auto rc) {
+    constexpr int R = decltype(rc)::R;
+    const int nb = ax.nbl();
+    for (int i = i0; i < nb; i += ni) {
+      cpx<T> u[R];
+      load_stage<D0, T>(rc, u, cur, tw, i, i, nb, nb, n, sx);
+      if constexpr (CONV) {
+#pragma unroll
+        for (int t = 0; t < R; ++t) u[t] = kmul(i + t * nb, u[t]);
+        stage_first<1, T>(rc, u, tw, n);
+#pragma unroll
+        for (int t = 0; t < R; ++t) oth[sx(i * R + t)] = u[t];
+      } else if (ok) {
+        if (scl != (T)1) {
+#pragma unroll
+          for (int t = 0; t < R; ++t) u[t] = c_scale(u[t], scl);
+        }
+#pragma unroll
+        for (int t = 0; t < R; ++t) g[(i + t * nb) * st] = u[t];
+      }
+    }
+  });
+  if constexpr (CONV) {
+    __syncthreads();
+    cpx<T>* x = cur;
+    cur = oth;
+    oth = x;
+    middle(axi, std::integral_constant<int, 1>{});
+    axi.last([&](auto rc) {
+      constexpr int R = decltype(rc)::R;
+      const int nb = axi.nbl();
+      for (int i = i0; i < nb; i += ni) {
+        cpx<T> u[R];
+        load_stage<1, T>(rc, u, cur, tw, i, i, nb, nb, n, sx);
+        if (ok) {
+#pragma unroll
+          for (int t = 0; t < R; ++t) g[(i + t * nb) * st] = u[t];
+        }
+      }
+    });
+  }
+}
+
+// ---- host side --------------------------------------------------------------------
+// what the launch shapes need to know of an axis type
+struct AxisInfo { int n, nst, nbf, nbl, nbmax; };
+template <typename AX> inline AxisInfo axis_info(const RbAxis& a) {
+  AxisInfo x;
+  if constexpr (AX::kFixed) {
+    x = AxisInfo{AX::n(), AX::nst(), AX::nbf(), AX::nbl(), AX::nbf() > AX::nbl() ? AX::nbf() : AX::nbl()};
+  } else {
+    x = AxisInfo{a.n, a.nst, a.nb[0], a.nb[a.nst - 1], 0};
+    for (int s = 0; s < a.nst; ++s) x.nbmax = a.nb[s] > x.nbmax ? a.nb[s] : x.nbmax;
+  }
+  return x;
+}
+
+template <typename K> inline int launch_check(const char* what) {
+  gb_count_launch();
+  cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess ? 0 : gb_set_error(GBOFDFT_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e));
+}
+
+// f(axis type, reversed axis type) for a length.  The FP32 lengths listed
+// above have kernels with every index folded at compile time: the FP32 passes
+// are bound by instruction issue and fetch (128^3, three fields: a column pass
+// 12.5 -> 9.4 us, the convolution 34 -> 16 us), the FP64 ones by the FP64 pipe,
+// where the kernels with run-time lengths are as fast.  Each translation unit
+// holds one group of lengths (GB_RB_GROUP); group 0 holds every other length.
+// 1: the length belongs to another group.
+template <typename A, typename B> struct AxPair { using ax = A; using inv = B; };
+// inverse rows: the order whose last radix is the smaller (a thread ends with
+// that many points of a row pair)
+template <typename P, bool FIXED> struct InverseOrder { using type = typename P::ax; };
+template <typename P> struct InverseOrder<P, true> {
+  using type = std::conditional_t<(P::ax::rl() <= P::inv::rl()), typename P::ax, typename P::inv>;
+};
+template <typename P> using inverse_order = typename InverseOrder<P, P::ax::kFixed>::type;
+#define GB_RB_G(...) Rad<__VA_ARGS__>
+template <typename T, typename F> static int by_axis(const RbAxis& ax, F&& f) {
+#define GB_RB_TWO(N, A, B) \
+  case N: return f(AxPair<Ax2<A, B>, Ax2<B, A>>{});
+#define GB_RB_THREE(N, A, B, C) \
+  case N: return f(AxPair<Ax3<A, B, C>, Ax3<C, B, A>>{});
+#define GB_RB_OTHER(N, ...) case N: return 1;
+  if constexpr (sizeof(T) == 4) {
+    switch (ax.n) {
+#if GB_RB_GROUP == 0
+      GB_RB_LENGTHS_1(GB_RB_OTHER) GB_RB_LENGTHS_2(GB_RB_OTHER) GB_RB_LENGTHS_3(GB_RB_OTHER)
+      GB_RB_LENGTHS_4(GB_RB_OTHER) GB_RB_LENGTHS3(GB_RB_OTHER)
+#elif GB_RB_GROUP == 1
+      GB_RB_LENGTHS_1(GB_RB_TWO)
+#elif GB_RB_GROUP == 2
+      GB_RB_LENGTHS_2(GB_RB_TWO)
+#elif GB_RB_GROUP == 3
+      GB_RB_LENGTHS_3(GB_RB_TWO)
+#elif GB_RB_GROUP == 4
+      GB_RB_LENGTHS_4(GB_RB_TWO)
+      GB_RB_LENGTHS3(GB_RB_THREE)
+#endif
+      default: break;
+    }
+  }
+#undef GB_RB_TWO
+#undef GB_RB_THREE
+#undef GB_RB_OTHER
+#if GB_RB_GROUP == 0
+  return f(AxPair<AxRun<T>, AxRun<T>>{});
+#else
+  return 1;
+#endif
+}
+
+constexpr size_t kMaxSmem = 227 * 1024;   // longer lines take the run-time-radix passes (return 1)
+constexpr int kSMs = 152;
+
+// Row pairs and threads of a row CTA.  Every candidate is rated by the lanes
+// that its stages keep busy (a warp instruction costs the same with idle
+// lanes) and by how evenly the CTAs divide over the SMs; shared memory lets
+// four CTAs be resident.
+struct RowShape { int lp, threads; };
+template <typename T> inline RowShape row_shape(const AxisInfo& ax, int nf, int nbuf, int nrows) {
+  const int lines = nf > 0 ? nf : 1;
+  const size_t per = sizeof(cpx<T>) * (size_t)line_pitch<T>(ax.n) * lines * nbuf;
+  const int nbl = ax.nbl, nbf = ax.nbf;
+  RowShape best{1, 32};
+  double rate = -1.0;
+  for (int lp = 1; lp <= RowCta<T>::NT && (lp == 1 || lp * per <= 56 * 1024); ++lp) {
+    int th = (lp * nbl + 31) / 32 * 32;
+    if (th > RowCta<T>::NT) {
+      if (lp > 1) break;
+      th = RowCta<T>::NT;
+    }
+    auto busy = [&](int tasks) { return tasks / (double)((tasks + th - 1) / th * th); };
+    const double lanes = 0.5 * busy(lp * nbl) + 0.5 * busy(lines * lp * nbf);
+    const double ctas = (double)((nrows + 2 * lp - 1) / (2 * lp));
+    const double waves = ctas / kSMs, even = waves / ceil(waves);
+    // fewer than 8 warps on an SM, or CTAs of one warp, leave latencies exposed
+    const double warps = waves * th / 32.0;
+    const double r = lanes * even * (th < 64 ? 0.9 : 1.0) * (warps < 8.0 ? warps / 8.0 : 1.0);
+    if (r > rate + 1e-9) {
+      rate = r;
+      best = RowShape{lp, th};
+    }
+  }
+  return best;
+}
+
+template <typename T>
+static int rows_fwd(gbofdft_plan* p, const void* in, void* spec, int64_t fstride, int ld2, int nf, const int* ops,
+             double beta, double scale, double rho0, cudaStream_t st) {
+  RowsFwd a;
+  a.ax = p->rb[2];
+  if (a.ax.nst == 0) return 1;
+  a.in = in; a.out = spec; a.fstride = fstride;
+  a.nrows = p->n[0] * p->n[1]; a.n2h = p->n2h; a.ld2 = ld2; a.nf = nf;
+  for (int f = 0; f < kFields; ++f) a.op[f] = f < nf ? ops[f] : OP_RHO;
+  a.b56 = fabs(beta - 5.0 / 6.0) < 1e-15;
+  a.rsq = rb_rsqrt_length(p->n[2]);
+  a.beta.set(beta);
+  a.half.set(0.5 * scale);
+  a.rho0.set(rho0);
+  a.inv0.set(rho0 > 0.0 ? 1.0 / rho0 : 0.0);
+  a.tw = p->tw[2];
+  a.dn.set(p->n[2]);
+  a.dnh.set(p->n2h);
+  int kind = PK_PLAIN;
+  for (int f = 0; f < nf; ++f) {
+    if (ops[f] == OP_SQRT || (ops[f] == OP_POWB && a.b56)) kind = kind > PK_ROOTS ? kind : PK_ROOTS;
+    else if (ops[f] != OP_RHO) kind = PK_GENERAL;
+  }
+  auto go = [&](auto kern, const AxisInfo& x, int nbuf) -> int {
+    const RowShape sh = row_shape<T>(x, nf, nbuf, a.nrows);
+    a.lp = sh.lp;
+    const size_t sm = nbuf * sizeof(cpx<T>) * (size_t)nf * a.lp * line_pitch<T>(x.n);
+    if (sm > kMaxSmem) return 1;
+    if (int rc = gbct::ct_smem(kern, sm)) return rc;
+    kern<<<(a.nrows + 2 * a.lp - 1) / (2 * a.lp), sh.threads, sm, st>>>(a);
+    return launch_check<T>("rb_rows_fwd");
+  };
+  return by_axis<T>(a.ax, [&](auto x) {
+    using AX = typename decltype(x)::ax;
+    const AxisInfo xi = axis_info<AX>(a.ax);
+    if (kind == PK_GENERAL) return go(k_rb_rows_fwd<T, PK_GENERAL, AX>, xi, 2);
+    if (kind == PK_ROOTS) return go(k_rb_rows_fwd<T, PK_ROOTS, AX>, xi, one_buffer<T, PK_ROOTS, AX>() ? 1 : 2);
+    return go(k_rb_rows_fwd<T, PK_PLAIN, AX>, xi, one_buffer<T, PK_PLAIN, AX>() ? 1 : 2);
+  });
+}
+
+template <typename T>
+static int rows_inv(gbofdft_plan* p, const void* spec, int64_t fstride, int ld2, int nf, void* out, int64_t ostride,
+             double scale, const EvalDesc* ev, const void* rho, const void* vloc, void* pot, int calc_e,
+             double* partials, int64_t* nblk_out, cudaStream_t st) {
+  RowsInv a;
+  memset(&a, 0, sizeof(a));
+  a.ax = p->rb[2];
+  if (a.ax.nst == 0) return 1;
+  a.in = spec; a.fstride = fstride; a.nrows = p->n[0] * p->n[1]; a.n2h = p->n2h; a.ld2 = ld2; a.nf = nf;
+  a.tw = p->tw[2];
+  a.out = out; a.ostride = ostride; a.scale.set(scale);
+  const int nrows = a.nrows;
+  auto go = [&](auto kern, const AxisInfo& x) -> int {
+    const int nbuf = x.nst > 2 ? 2 : 1;
+    const RowShape sh = row_shape<T>(x, nf, nbuf, nrows);
+    a.lp = sh.lp;
+    const int nblk = (nrows + 2 * sh.lp - 1) / (2 * sh.lp);
+    if (nblk_out) *nblk_out = nblk;
+    const size_t sm = nbuf * sizeof(cpx<T>) * (size_t)nf * a.lp * line_pitch<T>(x.n);
+    if (sm > kMaxSmem) return 1;
+    if (int rc = gbct::ct_smem(kern, sm)) return rc;
+    kern<<<nblk, sh.threads, sm, st>>>(a);
+    return launch_check<T>("rb_rows_inv");
+  };
+  if (!ev)
+    return by_axis<T>(a.ax, [&](auto x) {
+      using AX = inverse_order<decltype(x)>;
+      return go(k_rb_rows_inv<T, RI_STORE, AX>, axis_info<AX>(a.ax));
+    });
+  a.ev = *ev; a.rho = rho; a.vloc = vloc; a.pot = pot; a.partials = partials;
+  const double ctf = 2.87123400018819181594;    // (3/10)(3 pi^2)^(2/3)
+  a.tf_v.set(5.0 / 3.0 * ctf * ev->tf_x);
+  a.tf_e.set(ctf * ev->tf_x);
+  a.vw_y.set(ev->vw_y);
+  a.two_alpha.set(2.0 * ev->wt_alpha);
+  a.inv_two_alpha.set(ev->wt_alpha != 0.0 ? 1.0 / (2.0 * ev->wt_alpha) : 0.0);
+  a.wt_beta.set(ev->wt_beta);
+  a.b56 = fabs(ev->wt_beta - 5.0 / 6.0) < 1e-15;
+  return by_axis<T>(a.ax, [&](auto x) {
+    using AX = inverse_order<decltype(x)>;
+    const AxisInfo xi = axis_info<AX>(a.ax);
+    return calc_e ? go(k_rb_rows_inv<T, RI_EVAL_E, AX>, xi) : go(k_rb_rows_inv<T, RI_EVAL, AX>, xi);
+  });
+}
+
+template <typename T>
+static int cols(gbofdft_plan* p, void* spec, int64_t fstride, int ld2, int nf, int axis, int dir, double scale,
+         const KerDesc* kd, cudaStream_t st) {
+  Cols a;
+  memset(&a, 0, sizeof(a));
+  a.ax = p->rb[axis];
+  if (a.ax.nst == 0) return 1;
+  a.inv = p->rbi[axis];
+  const int outer = p->n[axis == 1 ? 0 : 1];
+  a.data = spec; a.fstride = fstride;
+  a.stride = axis == 1 ? ld2 : (int64_t)p->n[1] * ld2;
+  a.ostride = axis == 1 ? (int64_t)p->n[1] * ld2 : ld2;
+  a.ncol = (unsigned)outer * ld2; a.n2h = p->n2h; a.dld.set(ld2);
+  a.tw = p->tw[axis]; a.scale.set(scale);
+  a.n0 = p->n[0]; a.n1 = p->n[1]; a.n2 = p->n[2]; a.full = p->full;
+  for (int i = 0; i < 9; ++i) a.bg[i].set(p->bg[i]);
+  if (kd)
+    for (int f = 0; f < nf; ++f) {
+      a.type[f] = kd->type[f];
+      a.arr[f] = kd->arr[f];
+      a.coef[f].set(kd->coef[f]);
+    }
+  constexpr int TB = ColTile<T>::TB;
+  const dim3 grid((a.ncol + TB - 1) / TB, nf);
+  auto go = [&](auto kern, const AxisInfo& x) -> int {
+    // butterflies of a column side by side.  FP64: one per thread of the stage
+    // with the most (idle warps cost nothing on the FP64 pipe).  FP32: as many
+    // as keep the threads of every stage busy (the last stage counts twice in
+    // the convolution, which continues with the inverse's first).
+    const int cap = (sizeof(T) == 4 ? 400 : 256) / TB;
+    const int rounds = (x.nbmax + cap - 1) / cap;
+    int ni = (x.nbmax + rounds - 1) / rounds;
+    if (sizeof(T) == 4) {
+      double best = -1.0;
+      for (int c = x.nbl < x.nbf ? x.nbl : x.nbf; c <= x.nbmax && c <= cap; ++c) {
+        auto busy = [&](int nb) { return nb / (double)((nb + c - 1) / c * c); };
+        const double r = busy(x.nbf) + (kd ? 2.0 : 1.0) * busy(x.nbl) + 1e-3 * c;
+        if (r > best) {
+          best = r;
+          ni = c;
+        }
+      }
+    }
+    const int nbuf = x.nst < 2 ? 0 : (kd || x.nst > 2 ? 2 : 1);
+    const size_t sm = nbuf * sizeof(cpx<T>) * (size_t)TB * x.n;
+    if (sm > kMaxSmem) return 1;
+    if (int rc = gbct::ct_smem(kern, sm)) return rc;
+    kern<<<grid, TB * ni, sm, st>>>(a);
+    return launch_check<T>("rb_cols");
+  };
+  return by_axis<T>(a.ax, [&](auto x) {
+    using AX = typename decltype(x)::ax;
+    using AXI = typename decltype(x)::inv;
+    const AxisInfo xi = axis_info<AX>(a.ax);
+    if (kd) return go(k_rb_cols<T, -1, true, AX, AXI>, xi);
+    return dir < 0 ? go(k_rb_cols<T, -1, false, AX, AXI>, xi) : go(k_rb_cols<T, 1, false, AX, AXI>, xi);
+  });
+}
+
+}  // namespace gbrb
+
+// Instantiate the launchers of one precision and group of lengths (row and
+// column passes in translation units of their own: they compile in parallel).
+#define GB_RB_NAME(base, SUF) GB_RB_CAT(GB_RB_CAT(base##_##SUF, _g), GB_RB_GROUP)
+#define GB_RB_DEFINE_FWD(T, SUF)                                                                                \
+  int GB_RB_NAME(gb_rb_rows_fwd, SUF)(gbofdft_plan* p, const void* in, void* spec, int64_t fstride, int ld2,   \
+                                      int nf, const int* ops, double beta, double scale, double rho0,          \
+                                      cudaStream_t st) {                                                       \
+    return gbrb::rows_fwd<T>(p, in, spec, fstride, ld2, nf, ops, beta, scale, rho0, st);                       \
+  }
+#define GB_RB_DEFINE_INV(T, SUF)                                                                                \
+  int GB_RB_NAME(gb_rb_rows_inv, SUF)(gbofdft_plan* p, const void* spec, int64_t fstride, int ld2, int nf,     \
+                                      void* out, int64_t ostride, double scale, const EvalDesc* ev,            \
+                                      const void* rho, const void* vloc, void* pot, int calc_e,                \
+                                      double* partials, int64_t* nblk, cudaStream_t st) {                      \
+    return gbrb::rows_inv<T>(p, spec, fstride, ld2, nf, out, ostride, scale, ev, rho, vloc, pot, calc_e,        \
+                             partials, nblk, st);                                                              \
+  }
+#define GB_RB_DEFINE_COLS(T, SUF)                                                                               \
+  int GB_RB_NAME(gb_rb_cols, SUF)(gbofdft_plan* p, void* spec, int64_t fstride, int ld2, int nf, int axis,     \
+                                  int dir, double scale, const KerDesc* kd, cudaStream_t st) {                 \
+    return gbrb::cols<T>(p, spec, fstride, ld2, nf, axis, dir, scale, kd, st);                                  \
+  }

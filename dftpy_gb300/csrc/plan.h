@@ -1,6 +1,7 @@
 // Host-side plan: grid geometry, FFT schedules, device tables and workspaces.
 #pragma once
 #include "common.cuh"
+#include "rb_axis.h"
 
 struct GInfo {           // reciprocal-space geometry passed to kernels by value
   double bg[9];          // reciprocal lattice vectors, rows (2 pi inv(L)^T)
@@ -22,6 +23,7 @@ struct gbofdft_plan {
   int64_t NG;            // n0 n1 n2h (API spectrum size)
   int64_t NGld;          // n0 n1 ld2 (internal spectrum size)
   AxisPlan ax[3];
+  gbrb::RbAxis rb[3], rbi[3];   // register-blocked passes: radices largest first, smallest first
   void* tw[3];           // device twiddle tables, complex<prec>[n_axis]
   void* spec;            // GB_MAX_FIELDS internal spectra
   double* partials;      // per-CTA energy partial sums
@@ -88,6 +90,25 @@ int gb_cols(gbofdft_plan* p, void* spec, int64_t fstride, int ld2, int nf, int a
             double scale, cudaStream_t st);
 int gb_cols_conv(gbofdft_plan* p, void* spec, int64_t fstride, int ld2, int nf, const KerDesc& kd,
                  double scale, cudaStream_t st);
+// register-blocked passes (passes_rb_*.cu): return 1 when the axis length has a
+// prime factor above 7, 0 on success, an error code otherwise
+#define GB_RB_DECLARE(SUF)                                                                                     \
+  int gb_rb_rows_fwd_##SUF(gbofdft_plan*, const void* in, void* spec, int64_t fstride, int ld2, int nf,        \
+                           const int* ops, double beta, double scale, double rho0, cudaStream_t);              \
+  int gb_rb_rows_inv_##SUF(gbofdft_plan*, const void* spec, int64_t fstride, int ld2, int nf, void* out,       \
+                           int64_t ostride, double scale, const EvalDesc* ev, const void* rho,                 \
+                           const void* vloc, void* pot, int calc_e, double* partials, int64_t* nblk,           \
+                           cudaStream_t);                                                                      \
+  int gb_rb_cols_##SUF(gbofdft_plan*, void* spec, int64_t fstride, int ld2, int nf, int axis, int dir,          \
+                       double scale, const KerDesc* kd, cudaStream_t);
+GB_RB_DECLARE(f64_g0)
+GB_RB_DECLARE(f32_g0)
+GB_RB_DECLARE(f32_g1)
+GB_RB_DECLARE(f32_g2)
+GB_RB_DECLARE(f32_g3)
+GB_RB_DECLARE(f32_g4)
+#undef GB_RB_DECLARE
+void gb_rb_plan(gbofdft_plan* p);   // the plan's rb / rbi from its lengths and precision
 // compile-time-size passes (passes_ct_*.cu): return 1 when the size has no
 // specialisation, 0 on success, an error code otherwise
 int gb_ct_rows_fwd_f32(gbofdft_plan*, const void*, void*, int64_t, int, int, const int*, double, double, cudaStream_t);

@@ -229,7 +229,8 @@ __global__ void __launch_bounds__(kThreads) k_wgc_final(int64_t n, const T* __re
       if (two) {
         const T B = pb ? pb[i] : wpow(rc, b);
         const T Y0 = y0[i], Y1 = y1[i], Y2 = y2[i];
-        v = a * A / rc * sx + A * inv0 * (X1 + (T)2 * u * X2) + b * B / rc * (Y0 + u * Y1 + u * u * Y2) +
+        const T irc = (T)1 / rc;
+        v = a * A * irc * sx + A * inv0 * (X1 + (T)2 * u * X2) + b * B * irc * (Y0 + u * Y1 + u * u * Y2) +
             B * inv0 * (Y1 + (T)2 * u * Y2);
       } else {
         v = (T)2 * (a * A / rc * sx + A * inv0 * (X1 + (T)2 * u * X2));
@@ -357,13 +358,13 @@ int wgc_xfields(gbofdft_plan* p, const WgcBufs& W, int two, const void* kernels,
   const int nfield = two ? 6 : 3;
   const int op = OP_RHO;
   for (int i = 0; i < nfield; ++i) {
-    int rc = gb_rows_fwd(p, W.f[i], W.s[i], 0, p->ld2, 1, &op, 1.0, 1.0, st);
+    int rc = gb_rows_fwd(p, W.f[i], W.s[i], 0, p->ld2, 1, &op, 1.0, 2.0, st);
     if (!rc) rc = gb_cols(p, W.s[i], 0, p->ld2, 1, 1, -1, 1.0, st);
     if (!rc) rc = gb_cols(p, W.s[i], 0, p->ld2, 1, 0, -1, 1.0, st);
     if (rc) return rc;
   }
   const T* K = reinterpret_cast<const T*>(kernels);
-  const T scale = (T)(1.0 / (double)p->N);
+  const T scale = (T)(0.5 / (double)p->N);   // 1 / N, and the row pass's factor 2
   for (int h = 0; h < (two ? 2 : 1); ++h) {
     k_wgc_combine<T><<<kBlocks, kThreads, 0, st>>>(p->gi, p->ld2, K, scale, (cpx<T>*)W.s[3 * h],
                                                     (cpx<T>*)W.s[3 * h + 1], (cpx<T>*)W.s[3 * h + 2]);
