@@ -23,16 +23,17 @@ void gb_count_launch() { g_launches.fetch_add(1, std::memory_order_relaxed); }
 static std::mutex g_smem_mu;
 static std::map<std::pair<const void*, int>, int> g_smem;
 
-int gb_smem_granted(const void* kern, int dev) {
-  std::lock_guard<std::mutex> lk(g_smem_mu);
-  auto it = g_smem.find({kern, dev});
-  return it == g_smem.end() ? 0 : it->second;
-}
-
-void gb_smem_grant(const void* kern, int dev, int bytes) {
+// One lock over look-up and call: a kernel of run-time lengths is granted a
+// different size by each thread, and the last call alone counts.
+int gb_smem_grant(const void* kern, int bytes) {
+  int dev = 0;
+  GB_CUDA(cudaGetDevice(&dev));
   std::lock_guard<std::mutex> lk(g_smem_mu);
   int& v = g_smem[{kern, dev}];
-  if (bytes > v) v = bytes;
+  if (v >= bytes) return 0;
+  GB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+  v = bytes;
+  return 0;
 }
 
 int gb_set_error(int code, const char* fmt, ...) {

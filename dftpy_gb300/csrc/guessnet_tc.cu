@@ -439,13 +439,7 @@ __global__ void k_pack_tc(const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __
 // plans' registry of granted sizes, shared with the other passes)
 template <typename K>
 int tc_smem(K kern, int bytes) {
-  int dev = 0;
-  GB_CUDA(cudaGetDevice(&dev));
-  const void* key = reinterpret_cast<const void*>(kern);
-  if (gb_smem_granted(key, dev) >= bytes) return 0;
-  GB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-  gb_smem_grant(key, dev, bytes);
-  return 0;
+  return gb_smem_grant(reinterpret_cast<const void*>(kern), bytes);
 }
 
 template <int CIN, int COUT>

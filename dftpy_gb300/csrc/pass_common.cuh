@@ -22,14 +22,7 @@ template <typename T> __device__ __forceinline__ T sc(const Sc& s) {
 // has been launched with (keyed by kernel address and device).
 template <typename K> inline int ct_smem(K kern, size_t bytes) {
   if (bytes <= 40 * 1024) return 0;   // 48 KB, less the kernels' static arrays
-  int dev = 0;
-  cudaGetDevice(&dev);
-  const void* key = reinterpret_cast<const void*>(kern);
-  if (gb_smem_granted(key, dev) >= (int)bytes) return 0;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-  if (e != cudaSuccess) return gb_set_error(GBOFDFT_ERR_CUDA, "smem attribute: %s", cudaGetErrorString(e));
-  gb_smem_grant(key, dev, (int)bytes);
-  return 0;
+  return gb_smem_grant(reinterpret_cast<const void*>(kern), (int)bytes);
 }
 
 }  // namespace gbct

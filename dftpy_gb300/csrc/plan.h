@@ -166,8 +166,7 @@ int gb_eval_delta_core(gbofdft_plan* p64, gbofdft_plan* p32, const double* rho, 
 // the reference density of a delta-evaluation state (device, N doubles)
 const double* gb_delta_ref(const gbofdft_delta* d);
 void gb_count_launch();
-int gb_smem_granted(const void* kern, int dev);
-void gb_smem_grant(const void* kern, int dev, int bytes);
+int gb_smem_grant(const void* kern, int bytes);
 int gb_use_ct();  // 0 forces the generic passes (GBOFDFT_GENERIC_FFT=1)
 
 int gb_lwt_eval(gbofdft_plan* p, const void* rho, gbofdft_lwt* d, void* pot, double* energies, int calc_v,
