@@ -96,7 +96,6 @@ int gbofdft_plan_destroy(gbofdft_plan* p) {
   if (p->scratch) cudaFree(p->scratch);
   if (p->wt_pm) cudaFree(p->wt_pm);
   if (p->precond_pm) cudaFree(p->precond_pm);
-  if (p->wgc_pm) cudaFree(p->wgc_pm);
   delete p;
   return GBOFDFT_OK;
 }
@@ -370,6 +369,16 @@ static int eval_impl(gbofdft_plan* p, const void* rho, const gbofdft_functional*
   ev.cout = cout;
   ev.cstride = p->N;
   const int64_t fs = p->NGld;
+  if (!cout && extras && f->wgc && !p->plane && (calc & GBOFDFT_CALC_V)) {
+    rc = gb_wgc_eval_fused(p, rho, nf, ops, f->wt_beta, kd, ev, f->vloc, f->wgc, pot, energies,
+                           (calc & GBOFDFT_CALC_E) ? 1 : 0, st);
+    if (rc == 0 && f->lwt) {
+      gbofdft_functional rest = *f;
+      rest.wgc = nullptr;
+      return eval_extra(p, rho, &rest, pot, energies, calc, st);
+    }
+    if (rc != 1) return rc;
+  }
   if (!cout) {
     rc = gb_eval_plane(p, rho, nf, ops, f->wt_beta, kd, ev, f->vloc, pot, (calc & GBOFDFT_CALC_E) ? 1 : 0, energies,
                        st);

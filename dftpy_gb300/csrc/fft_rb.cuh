@@ -284,7 +284,7 @@ __device__ __forceinline__ void dft7_direct(cpx<T>* u, const cpx<T>* __restrict_
 template <int DIR, typename T, bool ONE, int Q, int... Qs>
 __device__ __forceinline__ void rad_dft(Rad<Q, Qs...>, cpx<T>* u, const cpx<T>* __restrict__ tw, int k, int p, int n) {
   constexpr int M = Rad<Q, Qs...>::R / Q;
-  if constexpr (Q == 7 && M == 1) {
+  if constexpr (Q == 7 && M == 1 && DIR < 0) {   // (inverse inputs carry no mean)
     dft7_direct<DIR, T>(u, tw, ONE ? 0 : k * (n / (p * Q)), n);
     return;
   }

@@ -512,21 +512,69 @@ int gb_use_ct() {
     return rc_;                                                                   \
   } while (0)
 
+int gb_rb_rows_fwd(gbofdft_plan* p, const RbFwd& d, cudaStream_t st) { GB_RB_CALL(gb_rb_rows_fwd, d, st); }
+int gb_rb_rows_inv(gbofdft_plan* p, const RbInv& d, int64_t* nblk, cudaStream_t st) {
+  GB_RB_CALL(gb_rb_rows_inv, d, nblk, st);
+}
+int gb_rb_cols(gbofdft_plan* p, const RbCols& d, cudaStream_t st) { GB_RB_CALL(gb_rb_cols, d, st); }
+int gb_rb_wgc(gbofdft_plan* p, const RbCols& d, cudaStream_t st) { GB_RB_CALL(gb_rb_wgc, d, st); }
+
+bool gb_rb_wgc_ok(const gbofdft_plan* p) {
+  if (!gb_use_ct()) return false;
+  for (int a = 0; a < 3; ++a)
+    if (p->rb[a].nst == 0) return false;
+  // columns of 128 bytes per element, five buffers along axis 0 and two along
+  // axis 1; rows of all fields, one pair, two buffers
+  const size_t row = 2 * gb_elem(p) * (size_t)(p->n[2] + p->n[2] / 8 + 1);
+  return p->rb[0].nst > 1 && 128 * 5 * (size_t)p->n[0] <= 227 * 1024 && 128 * 2 * (size_t)p->n[1] <= 227 * 1024 &&
+         2 * GB_RB_FIELDS * row <= 227 * 1024;
+}
+
+// spectra at base + f * stride complex elements
+static void rb_fields(const gbofdft_plan* p, void** f, const void* base, int64_t stride, int nf) {
+  for (int i = 0; i < nf; ++i)
+    f[i] = const_cast<char*>(reinterpret_cast<const char*>(base)) + 2 * gb_elem(p) * (size_t)(i * stride);
+}
+
 static int rb_rows_fwd(gbofdft_plan* p, const void* in, void* spec, int64_t fstride, int ld2, int nf, const int* ops,
-                       double beta, double scale, double rho0, cudaStream_t st) {
-  GB_RB_CALL(gb_rb_rows_fwd, in, spec, fstride, ld2, nf, ops, beta, scale, rho0, st);
+                       double beta, double scale, cudaStream_t st) {
+  RbFwd d;
+  memset(&d, 0, sizeof(d));
+  rb_fields(p, d.out, spec, fstride, nf);
+  for (int f = 0; f < nf; ++f) {
+    d.in[f] = in;
+    d.op[f] = ops[f];
+  }
+  d.nf = nf; d.ld2 = ld2; d.beta = beta; d.scale = scale;
+  return gb_rb_rows_fwd(p, d, st);
 }
 
 static int rb_rows_inv(gbofdft_plan* p, const void* spec, int64_t fstride, int ld2, int nf, void* out,
                        int64_t ostride, double scale, const EvalDesc* ev, const void* rho, const void* vloc,
                        void* pot, int calc_e, double* partials, int64_t* nblk, cudaStream_t st) {
-  GB_RB_CALL(gb_rb_rows_inv, spec, fstride, ld2, nf, out, ostride, scale, ev, rho, vloc, pot, calc_e, partials, nblk,
-             st);
+  RbInv d;
+  memset(&d, 0, sizeof(d));
+  rb_fields(p, const_cast<void**>(d.in), spec, fstride, nf);
+  d.nf = nf; d.ld2 = ld2; d.out = out; d.ostride = ostride; d.scale = scale;
+  d.ev = ev; d.rho = rho; d.vloc = vloc; d.pot = pot; d.calc_e = calc_e; d.partials = partials;
+  return gb_rb_rows_inv(p, d, nblk, st);
 }
 
 static int rb_cols(gbofdft_plan* p, void* spec, int64_t fstride, int ld2, int nf, int axis, int dir, double scale,
                    const KerDesc* kd, cudaStream_t st) {
-  GB_RB_CALL(gb_rb_cols, spec, fstride, ld2, nf, axis, dir, scale, kd, st);
+  RbCols d;
+  memset(&d, 0, sizeof(d));
+  rb_fields(p, d.data, spec, fstride, nf);
+  d.nf = nf; d.ld2 = ld2; d.axis = axis; d.dir = dir; d.scale = scale; d.kd = kd;
+  return gb_rb_cols(p, d, st);
+}
+
+int gb_energy_final(gbofdft_plan* p, const double* partials, int64_t nblk, double e_ion, double* energies,
+                    cudaStream_t st) {
+  if (nblk > p->max_partials) return gb_set_error(GBOFDFT_ERR_STATE, "partials buffer too small");
+  k_energy_final<<<6, 256, 0, st>>>(partials, nblk, p->dV, e_ion, energies, gb_plan_counter(p));
+  GB_CHECK_LAUNCH();
+  return 0;
 }
 
 void gb_rb_plan(gbofdft_plan* p) {
@@ -539,7 +587,7 @@ void gb_rb_plan(gbofdft_plan* p) {
 int gb_rows_fwd(gbofdft_plan* p, const void* in, void* spec, int64_t fstride, int ld2, int nf, const int* ops,
                 double beta, double scale, cudaStream_t st) {
   if (gb_use_ct()) {
-    const int rc = rb_rows_fwd(p, in, spec, fstride, ld2, nf, ops, beta, scale, 0.0, st);
+    const int rc = rb_rows_fwd(p, in, spec, fstride, ld2, nf, ops, beta, scale, st);
     if (rc != 1) return rc;
   }
   return p->prec == GBOFDFT_F64 ? rows_fwd_t<double>(p, in, spec, fstride, ld2, nf, ops, beta, scale, st)

@@ -67,8 +67,6 @@ using gbct::Sc;
 using gbct::kZero;
 using gbct::sc;
 
-constexpr int kFields = 8;
-
 // element j of a line in shared memory: one complex value of padding per 128
 // bytes, so the stride-radix writes of a first stage spread over the banks
 template <typename T> __device__ __forceinline__ int sidx(int j) {
@@ -120,16 +118,18 @@ __device__ __forceinline__ double pow56(double x, const Roots<double>& r) { retu
 
 // ---- forward rows ---------------------------------------------------------------
 struct RowsFwd {
-  const void* in;
-  void* out;
-  int64_t fstride;
+  const void* in[GB_RB_FIELDS];   // per field (the derived kinds read in[0])
+  void* out[GB_RB_FIELDS];
   int nrows, n2h, ld2, nf, lp;
-  int op[kFields];
+  int op[GB_RB_FIELDS];
   int b56, rsq;           // rsq: sqrt(rho) as rho rsqrt(rho) (FP32)
-  Sc beta, half, rho0, inv0;
+  Sc beta, beta2, half, rho0, inv0;
   RbAxis ax;
   FastDiv dn, dnh;
   const void* tw;
+  // PK_WGC, FP64: keep rho^beta and rho^beta2 / take rho^beta from an earlier launch
+  void *pw_out, *pw2_out;
+  const void* pw_in;
 };
 
 template <typename T>
@@ -137,10 +137,17 @@ __device__ __noinline__ T pow_general(T x, T b) { return pow(x, b); }
 template <typename T>
 __device__ __noinline__ T sqrt_call(T x) { return sqrt(x); }
 
+// x^b.  FP64: exp(b ln x), one logarithm for both exponents where two powers
+// of a density are wanted; its relative error, |b ln x| ulp, is below 1e-14 for
+// x >= 1e-30.
+__device__ __forceinline__ float pow_of(float x, float b) { return powf(x, b); }
+__device__ __forceinline__ double pow_of(double x, double b) { return exp(b * log(x)); }
+
 // Prologues of the forward rows.  A kernel per kind: a plain transform holds
 // none of the root arithmetic (the compiler would compute it ahead of the
 // branch, at 12 FP64 operations a point).
-enum { PK_PLAIN = 0, PK_ROOTS = 1, PK_GENERAL = 2 };
+// PK_WGC: the three fields rho^e, u rho^e, u^2 rho^e of one exponent.
+enum { PK_PLAIN = 0, PK_ROOTS = 1, PK_GENERAL = 2, PK_WGC = 3 };
 
 // the values of one density that the derived fields are made of
 template <typename T> struct Derived { T rho, sq, b, u; };
@@ -148,32 +155,37 @@ template <typename T, int KIND>
 __device__ __forceinline__ Derived<T> derived(const RowsFwd& a, T rho) {
   Derived<T> d;
   d.rho = d.sq = d.b = d.u = rho;
-  if constexpr (KIND != PK_PLAIN) {
+  if constexpr (KIND == PK_WGC) {
+    const T rc = rho > (T)kZero ? rho : (T)kZero;
+    d.u = (rc - sc<T>(a.rho0)) * sc<T>(a.inv0);
+    if constexpr (sizeof(T) == 8) {
+      if (!a.pw_in) {
+        const T l = log(rc);
+        d.b = exp(sc<T>(a.beta) * l);
+        if (a.pw2_out) d.sq = exp(sc<T>(a.beta2) * l);      // kept for the other exponent's fields
+      }
+    } else {
+      d.b = pow_of(rc, sc<T>(a.beta));
+    }
+  } else if constexpr (KIND != PK_PLAIN) {
     const T kz = (T)kZero;
     const T rc = rho > kz ? rho : kz;
     const Roots<T> r = roots(rc);
     d.sq = sqrt_of(rc, r);
     if (sizeof(T) == 4 && !a.rsq) d.sq = sqrt(rc);
     if (rho > (T)0 && rho < kz) d.sq = sqrt_call<T>(rho);
-    if constexpr (KIND == PK_ROOTS) {
-      d.b = pow56(rc, r);
-    } else {
-      d.b = pow_general<T>(rc, sc<T>(a.beta));
-      d.u = (rc - sc<T>(a.rho0)) * sc<T>(a.inv0);
-    }
+    if constexpr (KIND == PK_ROOTS) d.b = pow56(rc, r);
+    else d.b = pow_general<T>(rc, sc<T>(a.beta));
   }
   return d;
 }
 template <typename T, int KIND>
 __device__ __forceinline__ T field_of(int op, const Derived<T>& d) {
   if constexpr (KIND == PK_PLAIN) return d.rho;
+  if constexpr (KIND == PK_WGC) return op == OP_WGC0 ? d.b : (op == OP_WGC1 ? d.u * d.b : d.u * d.u * d.b);
   T v = d.rho;
   if (op == OP_SQRT) v = d.sq;
-  else if (op == OP_POWB || op == OP_WGC0) v = d.b;
-  if constexpr (KIND == PK_GENERAL) {
-    if (op == OP_WGC1) v = d.u * d.b;
-    else if (op == OP_WGC2) v = d.u * d.u * d.b;
-  }
+  else if (op == OP_POWB) v = d.b;
   return v;
 }
 // one derived field alone (FP32: the roots of a field cost less than passing
@@ -260,7 +272,7 @@ __device__ __forceinline__ cpx<T>* lines(cpx<T>* a, cpx<T>* b, int ls, int nl, c
 // a field's butterfly
 template <typename T, int KIND, typename AX> constexpr bool direct_rows() {
   if constexpr (sizeof(T) == 4 && AX::kFixed && KIND != PK_GENERAL)
-    return AX::n() / AX::nbf() <= (KIND == PK_PLAIN ? 16 : 12);
+    return AX::n() / AX::nbf() <= (KIND == PK_PLAIN ? 16 : KIND == PK_ROOTS ? 12 : 8);
   else return false;
 }
 template <typename T, int KIND, typename AX> constexpr bool kDirect = direct_rows<T, KIND, AX>();
@@ -284,7 +296,6 @@ __global__ void __launch_bounds__(RowCta<T>::NT, (RowCta<T, AX>::MINB)) k_rb_row
   cpx<T>* B = one_buffer<T, KIND, AX>() ? A : A + nl * ls;
   const int tid = threadIdx.x, nthr = blockDim.x;
   const int base = blockIdx.x * 2 * lp;
-  const T* in = reinterpret_cast<const T*>(a.in);
   const cpx<T>* tw = reinterpret_cast<const cpx<T>*>(a.tw);
   cpx<T>* res;
   if constexpr (kDirect<T, KIND, AX>) {
@@ -297,17 +308,36 @@ __global__ void __launch_bounds__(RowCta<T>::NT, (RowCta<T, AX>::MINB)) k_rb_row
       for (int t0 = tid; t0 < lp * nb; t0 += nthr) {
         const int l = ax.div_nbf(t0), i = t0 - l * nb;
         const int ra = base + 2 * l;
-        const T* src = in + (int64_t)ra * n + i;
-        T x0[R], x1[R];
+        const int64_t off = (int64_t)ra * n + i;
+        T x0[R], x1[R], b0[KIND == PK_WGC ? R : 1], b1[KIND == PK_WGC ? R : 1];
+        auto load = [&](const void* p) {
+          const T* src = reinterpret_cast<const T*>(p) + off;
 #pragma unroll
-        for (int t = 0; t < R; ++t) {
-          x0[t] = ra < a.nrows ? __ldg(src + t * nb) : (T)0;
-          x1[t] = ra + 1 < a.nrows ? __ldg(src + n + t * nb) : (T)0;
+          for (int t = 0; t < R; ++t) {
+            x0[t] = ra < a.nrows ? __ldg(src + t * nb) : (T)0;
+            x1[t] = ra + 1 < a.nrows ? __ldg(src + n + t * nb) : (T)0;
+          }
+        };
+        load(a.in[0]);
+        if constexpr (KIND == PK_WGC) {
+#pragma unroll
+          for (int t = 0; t < R; ++t) {
+            const Derived<T> d0 = derived<T, KIND>(a, x0[t]), d1 = derived<T, KIND>(a, x1[t]);
+            x0[t] = d0.u; b0[t] = d0.b;
+            x1[t] = d1.u; b1[t] = d1.b;
+          }
         }
         for (int f = 0; f < a.nf; ++f) {
           const int op = a.op[f];
           cpx<T> u[R];
-          if (op == OP_RHO || KIND == PK_PLAIN) {
+          if constexpr (KIND == PK_WGC) {
+#pragma unroll
+            for (int t = 0; t < R; ++t) {
+              const Derived<T> d0{x0[t], x0[t], b0[t], x0[t]}, d1{x1[t], x1[t], b1[t], x1[t]};
+              u[t] = cpx<T>{field_of<T, KIND>(op, d0), field_of<T, KIND>(op, d1)};
+            }
+          } else if (op == OP_RHO || KIND == PK_PLAIN) {
+            if (KIND == PK_PLAIN && f > 0 && a.in[f] != a.in[f - 1]) load(a.in[f]);
 #pragma unroll
             for (int t = 0; t < R; ++t) u[t] = cpx<T>{x0[t], x1[t]};
           } else if (op == OP_SQRT) {
@@ -331,21 +361,45 @@ __global__ void __launch_bounds__(RowCta<T>::NT, (RowCta<T, AX>::MINB)) k_rb_row
       const int l = AX::kFixed ? idx / n : (int)a.dn.div(idx), j = idx - l * n;
       const int ra = base + 2 * l;
       const bool ok0 = ra < a.nrows, ok1 = ra + 1 < a.nrows;
-      const T* src = in + (int64_t)ra * n + j;
-      const Derived<T> d0 = derived<T, KIND>(a, ok0 ? __ldg(src) : (T)0);
-      const Derived<T> d1 = derived<T, KIND>(a, ok1 ? __ldg(src + n) : (T)0);
+      const int64_t off = (int64_t)ra * n + j;
       cpx<T>* o = A + l * ls + sidx<T>(j);
-      for (int f = 0; f < a.nf; ++f)
-        o[f * lp * ls] = cpx<T>{field_of<T, KIND>(a.op[f], d0), field_of<T, KIND>(a.op[f], d1)};
+      if constexpr (KIND == PK_PLAIN) {
+        for (int f = 0; f < a.nf; ++f) {
+          const T* src = reinterpret_cast<const T*>(a.in[f]) + off;
+          o[f * lp * ls] = cpx<T>{ok0 ? __ldg(src) : (T)0, ok1 ? __ldg(src + n) : (T)0};
+        }
+      } else {
+        const T* src = reinterpret_cast<const T*>(a.in[0]) + off;
+        Derived<T> d0 = derived<T, KIND>(a, ok0 ? __ldg(src) : (T)0);
+        Derived<T> d1 = derived<T, KIND>(a, ok1 ? __ldg(src + n) : (T)0);
+        if constexpr (KIND == PK_WGC && sizeof(T) == 8) {
+          if (a.pw_in) {
+            const T* pw = reinterpret_cast<const T*>(a.pw_in) + off;
+            if (ok0) d0.b = pw[0];
+            if (ok1) d1.b = pw[n];
+          }
+          if (a.pw_out) {
+            T* pw = reinterpret_cast<T*>(a.pw_out) + off;
+            if (ok0) pw[0] = d0.b;
+            if (ok1) pw[n] = d1.b;
+          }
+          if (a.pw2_out) {
+            T* pw = reinterpret_cast<T*>(a.pw2_out) + off;
+            if (ok0) pw[0] = d0.sq;
+            if (ok1) pw[n] = d1.sq;
+          }
+        }
+        for (int f = 0; f < a.nf; ++f)
+          o[f * lp * ls] = cpx<T>{field_of<T, KIND>(a.op[f], d0), field_of<T, KIND>(a.op[f], d1)};
+      }
     }
     __syncthreads();
     res = lines<-1, true, T>(A, B, ls, nl, ax, tw);
   }
-  cpx<T>* out = reinterpret_cast<cpx<T>*>(a.out);
   const T half = sc<T>(a.half);
   const int nh = AX::kFixed ? n / 2 + 1 : a.n2h;
   for (int f = 0; f < a.nf; ++f) {
-    cpx<T>* o = out + f * a.fstride;
+    cpx<T>* o = reinterpret_cast<cpx<T>*>(a.out[f]);
     const cpx<T>* src = res + f * lp * ls;
     for (int idx = tid; idx < lp * nh; idx += nthr) {
       const int l = AX::kFixed ? idx / nh : (int)a.dnh.div(idx), k = idx - l * nh;
@@ -367,8 +421,7 @@ __global__ void __launch_bounds__(RowCta<T>::NT, (RowCta<T, AX>::MINB)) k_rb_row
 
 // ---- inverse rows ----------------------------------------------------------------
 struct RowsInv {
-  const void* in;
-  int64_t fstride;
+  const void* in[GB_RB_FIELDS];
   int nrows, n2h, ld2, nf, lp;
   RbAxis ax;
   const void* tw;
@@ -382,6 +435,14 @@ struct RowsInv {
   const void* vloc;
   void* pot;
   double* partials;
+  int base;             // the fused terms are wanted (else the WGC term alone)
+  int add;              // add to pot
+  // WGC term: its fields X0..X2 (Y0..Y2) are the line fields from slot wslot on
+  int wgc, wslot, two;
+  Sc w_rho0, w_inv0, w_a, w_b;
+  const void *pa, *pb;  // FP64: rho^a and rho^b of the forward rows
+  void* wstore[6];      // FP64: copies of the fields and of the potential (delta-evaluation reference)
+  void* vstore;
 };
 
 // a call, so that the compiler cannot compute the logarithm of the r_s < 1
@@ -519,6 +580,27 @@ __device__ __forceinline__ T point(const RowsInv& a, T rho, T w, T kc, T vh, T v
   return pot;
 }
 
+// the WGC term at one point from its six fields (FP64: and the powers A, B of
+// the forward rows): potential; energy density added to es[2]
+template <typename T, bool WANT_E>
+__device__ __forceinline__ T wgc_point(const RowsInv& a, T rho, T A, T B, T X0, T X1, T X2, T Y0, T Y1, T Y2, T* es) {
+  const T rc = rho > (T)kZero ? rho : (T)kZero;
+  const T inv0 = sc<T>(a.w_inv0), u = (rc - sc<T>(a.w_rho0)) * inv0;
+  if constexpr (sizeof(T) == 4) A = pow_of(rc, sc<T>(a.w_a));
+  const T ir = rcp_nr(rc);
+  const T sx = X0 + u * X1 + u * u * X2, tx = X1 + (T)2 * u * X2;
+  if (WANT_E) es[2] += A * sx;
+  T v = A * (sc<T>(a.w_a) * ir * sx + inv0 * tx);
+  if (a.two) {
+    if constexpr (sizeof(T) == 4) B = pow_of(rc, sc<T>(a.w_b));
+    const T sy = Y0 + u * Y1 + u * u * Y2, ty = Y1 + (T)2 * u * Y2;
+    v += B * (sc<T>(a.w_b) * ir * sy + inv0 * ty);
+  } else {
+    v *= (T)2;
+  }
+  return v;
+}
+
 enum { RI_STORE = 0, RI_EVAL = 1, RI_EVAL_E = 2 };
 
 template <typename T, int MODE, typename AX>
@@ -530,7 +612,6 @@ __global__ void __launch_bounds__(RowCta<T>::NT, (RowCta<T, AX>::MINB)) k_rb_row
   cpx<T>* B = A + nl * ls;                               // used by three or more stages
   const int tid = threadIdx.x, nthr = blockDim.x;
   const int base = blockIdx.x * 2 * lp;
-  const cpx<T>* in = reinterpret_cast<const cpx<T>*>(a.in);
   const cpx<T>* tw = reinterpret_cast<const cpx<T>*>(a.tw);
   // first stage: line element j of a row pair is X_a[j] + i X_b[j] for
   // j <= n/2 and the conjugates' combination above
@@ -542,7 +623,7 @@ __global__ void __launch_bounds__(RowCta<T>::NT, (RowCta<T, AX>::MINB)) k_rb_row
       const int f = line / lp, l = line - f * lp;
       const int ra = base + 2 * l;
       cpx<T> u[R];
-      const cpx<T>* pa = in + f * a.fstride + (int64_t)ra * a.ld2;
+      const cpx<T>* pa = reinterpret_cast<const cpx<T>*>(a.in[f]) + (int64_t)ra * a.ld2;
       const bool ok0 = ra < a.nrows, ok1 = ra + 1 < a.nrows;
 #pragma unroll
       for (int t = 0; t < R; ++t) {
@@ -663,8 +744,57 @@ __global__ void __launch_bounds__(RowCta<T>::NT, (RowCta<T, AX>::MINB)) k_rb_row
           }
         }
         constexpr bool E = MODE == RI_EVAL_E;
-        pp[j] = point<T, E>(a, r0, w.x, kc.x, vh.x, v0, es);
-        if (ok1) pp[j + n] = point<T, E>(a, r1, w.y, kc.y, vh.y, v1, es);
+        T p0 = (T)0, p1 = (T)0;
+        if (a.base) {
+          p0 = point<T, E>(a, r0, w.x, kc.x, vh.x, v0, es);
+          if (ok1) p1 = point<T, E>(a, r1, w.y, kc.y, vh.y, v1, es);
+        }
+        if (a.add) {
+          p0 += pp[j];
+          if (ok1) p1 += pp[j + n];
+        }
+        if (a.wgc) {
+          cpx<T> x[3], y[3];
+          const int ys = a.two ? 3 : 0;
+#pragma unroll
+          for (int q = 0; q < 3; ++q) {
+            x[q] = fld[(a.wslot + q) * fs + o];
+            y[q] = fld[(a.wslot + ys + q) * fs + o];
+          }
+          T A0 = (T)0, B0 = (T)0, A1 = (T)0, B1 = (T)0;
+          if constexpr (sizeof(T) == 8) {
+            const T *qa = reinterpret_cast<const T*>(a.pa) + g0 + j, *qb = reinterpret_cast<const T*>(a.pb) + g0 + j;
+            A0 = qa[0]; B0 = qb[0];
+            if (ok1) { A1 = qa[n]; B1 = qb[n]; }
+            if (a.vstore) {
+#pragma unroll
+              for (int q = 0; q < 3; ++q) {
+                T* c = reinterpret_cast<T*>(a.wstore[q]) + g0 + j;
+                c[0] = x[q].x;
+                if (ok1) c[n] = x[q].y;
+                if (a.two) {
+                  c = reinterpret_cast<T*>(a.wstore[3 + q]) + g0 + j;
+                  c[0] = y[q].x;
+                  if (ok1) c[n] = y[q].y;
+                }
+              }
+            }
+          }
+          const T w0 = wgc_point<T, E>(a, r0, A0, B0, x[0].x, x[1].x, x[2].x, y[0].x, y[1].x, y[2].x, es);
+          T w1 = (T)0;
+          if (ok1) w1 = wgc_point<T, E>(a, r1, A1, B1, x[0].y, x[1].y, x[2].y, y[0].y, y[1].y, y[2].y, es);
+          if constexpr (sizeof(T) == 8) {
+            if (a.vstore) {
+              T* c = reinterpret_cast<T*>(a.vstore) + g0 + j;
+              c[0] = w0;
+              if (ok1) c[n] = w1;
+            }
+          }
+          p0 += w0;
+          p1 += w1;
+        }
+        pp[j] = p0;
+        if (ok1) pp[j + n] = p1;
         r0 = nr0;
         r1 = nr1;
         v0 = nv0;
@@ -691,8 +821,8 @@ __global__ void __launch_bounds__(RowCta<T>::NT, (RowCta<T, AX>::MINB)) k_rb_row
 
 // ---- columns -------------------------------------------------------------------
 struct Cols {
-  void* data;
-  int64_t fstride, stride, ostride;
+  void* data[GB_RB_FIELDS];
+  int64_t stride, ostride;
   unsigned ncol;          // columns over all outer indices (pitch ld2 each)
   int n2h;
   FastDiv dld;
@@ -704,6 +834,8 @@ struct Cols {
   int type[GB_MAX_FIELDS];
   const void* arr[GB_MAX_FIELDS];
   int n0, n1, n2, full;
+  const void* K;          // WGC: K0, K1, Kq, Kx (API layout), kstride values each
+  int64_t kstride;
 };
 
 template <typename T> struct ColTile { static constexpr int TB = 128 / (2 * (int)sizeof(T)); };
@@ -763,7 +895,7 @@ __global__ void __launch_bounds__(sizeof(T) == 4 ? 400 : 256) k_rb_cols(const __
   const int outer = a.dld.div(col), k2 = col - outer * a.dld.d;
   const bool ok = col < a.ncol && k2 < a.n2h;
   const int f = blockIdx.y;
-  cpx<T>* g = reinterpret_cast<cpx<T>*>(a.data) + f * a.fstride + outer * a.ostride + k2;
+  cpx<T>* g = reinterpret_cast<cpx<T>*>(a.data[f]) + outer * a.ostride + k2;
   const cpx<T>* tw = reinterpret_cast<const cpx<T>*>(a.tw);
   const int64_t st = a.stride;
   ColKernel<T> ker;
@@ -884,6 +1016,155 @@ __global__ void __launch_bounds__(sizeof(T) == 4 ? 400 : 256) k_rb_cols(const __
   }
 }
 
+// WGC term along axis 0: forward transforms of the three fields F0..F2 of one
+// exponent (blockIdx.y), X0 = K0 F0 + K1/6 F1 + Kq F2, X1 = K1/6 F0 + Kx F1,
+// X2 = Kq F0, and the inverse transforms, in one pass over the spectra.  The
+// forward results stay in shared memory; each output is combined in the
+// registers of its inverse's first stage.  blockDim.y = 3: the fields, then the
+// outputs, side by side; 1: one after the other.  Three column buffers and,
+// per side, one (two for three or more stages).
+// FP32: one field's butterflies (128 to 256 threads) leave the SM waiting on the
+// loads of each stage: 96^3, six fields, 42.7 us; side by side 24.4 us
+// FP64: bound by the FP64 pipe either way.
+template <typename T> constexpr int kWgcThreads = sizeof(T) == 4 ? 768 : 256;
+template <typename T, typename AX, typename AXI>
+__global__ void __launch_bounds__(kWgcThreads<T>) k_rb_wgc(const __grid_constant__ Cols a) {
+  constexpr int TB = ColTile<T>::TB;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const AX ax(a.ax);
+  const AXI axi(a.inv);
+  const int n = ax.n();
+  cpx<T>* S = reinterpret_cast<cpx<T>*>(smem_raw);
+  const int f0 = threadIdx.y, nf = blockDim.y;
+  cpx<T>* D = S + (3 + f0) * n * TB;
+  cpx<T>* E = D + nf * n * TB;                           // three or more stages
+  const int c = threadIdx.x % TB, i0 = threadIdx.x / TB, ni = blockDim.x / TB;
+  const unsigned col = blockIdx.x * TB + c;
+  const int outer = a.dld.div(col), k2 = col - outer * a.dld.d;
+  const bool ok = col < a.ncol && k2 < a.n2h;
+  const int64_t off = outer * a.ostride + k2;
+  const cpx<T>* tw = reinterpret_cast<const cpx<T>*>(a.tw);
+  const int64_t st = a.stride;
+  auto sx = [&](int j) { return j * TB + c; };
+  auto field = [&](int f) { return reinterpret_cast<cpx<T>*>(a.data[3 * blockIdx.y + f]) + off; };
+  // middle stages of one column buffer: cur -> oth -> cur ...; the result's buffer
+  auto middle = [&](const auto& x, auto dir, cpx<T>* cur, cpx<T>* oth) {
+    constexpr int DR = decltype(dir)::value;
+    x.middle([&](auto rc, auto nb, auto p, auto, auto div_p) {
+      constexpr int R = decltype(rc)::R;
+      for (int i = i0; i < nb; i += ni) {
+        const int k = i - p * div_p(i);
+        cpx<T> u[R];
+        load_stage<DR, T>(rc, u, cur, tw, i, k, nb, p, n, sx);
+        const int j0 = (i - k) * R + k;
+#pragma unroll
+        for (int t = 0; t < R; ++t) oth[sx(j0 + t * p)] = u[t];
+      }
+      __syncthreads();
+      cpx<T>* y = cur;
+      cur = oth;
+      oth = y;
+    });
+    return cur;
+  };
+#pragma unroll 1
+  for (int f = f0; f < 3; f += nf) {
+    const cpx<T>* g = field(f);
+    cpx<T>* s = S + f * n * TB;
+    ax.first([&](auto rc) {
+      constexpr int R = decltype(rc)::R;
+      const int nb = ax.nbf();
+      for (int i = i0; i < nb; i += ni) {
+        cpx<T> u[R];
+#pragma unroll
+        for (int t = 0; t < R; ++t) u[t] = ok ? g[(i + t * nb) * st] : cpx<T>{(T)0, (T)0};
+        stage_first<-1, T>(rc, u, tw, n);
+#pragma unroll
+        for (int t = 0; t < R; ++t) s[sx(i * R + t)] = u[t];
+      }
+    });
+  }
+  __syncthreads();
+  const int nbl = ax.nbl();
+#pragma unroll 1
+  for (int f = f0; f < 3; f += nf) {
+    cpx<T>* s = S + f * n * TB;
+    const cpx<T>* cur = s;
+    if (ax.nst() > 2) cur = middle(ax, std::integral_constant<int, -1>{}, s, D);
+    ax.last([&](auto rc) {
+      constexpr int R = decltype(rc)::R;
+      for (int i = i0; i < nbl; i += ni) {
+        cpx<T> u[R];
+        load_stage<-1, T>(rc, u, cur, tw, i, i, nbl, nbl, n, sx);
+#pragma unroll
+        for (int t = 0; t < R; ++t) s[sx(i + t * nbl)] = u[t];
+      }
+    });
+    __syncthreads();      // D is read before the next field's middle stages write it, S written before it is combined
+  }
+  const T* K = reinterpret_cast<const T*>(a.K) + (int64_t)outer * a.n2h + k2;
+  const int64_t kst = (int64_t)a.n1 * a.n2h;
+  const T scl = sc<T>(a.scale), sc6 = scl * (T)(1.0 / 6.0);
+#pragma unroll 1
+  for (int o = f0; o < 3; o += nf) {
+    ax.last([&](auto rc) {
+      constexpr int R = decltype(rc)::R;
+      for (int i = i0; i < nbl; i += ni) {
+        cpx<T> u[R];
+#pragma unroll
+        for (int t = 0; t < R; ++t) {
+          const int j = i + t * nbl;
+          const T* kj = K + j * kst;
+          // coefficients of F0, F1, F2
+          T q0 = (T)0, q1 = (T)0, q2 = (T)0;
+          if (ok) {
+            if (o == 0) {
+              q0 = __ldg(kj) * scl;
+              q1 = __ldg(kj + a.kstride) * sc6;
+              q2 = __ldg(kj + 2 * a.kstride) * scl;
+            } else if (o == 1) {
+              q0 = __ldg(kj + a.kstride) * sc6;
+              q1 = __ldg(kj + 3 * a.kstride) * scl;
+            } else {
+              q0 = __ldg(kj + 2 * a.kstride) * scl;
+            }
+          }
+          const cpx<T> g0 = S[sx(j)];
+          cpx<T> v = {q0 * g0.x, q0 * g0.y};
+          if (o < 2) {
+            const cpx<T> g1 = S[n * TB + sx(j)];
+            v = cpx<T>{v.x + q1 * g1.x, v.y + q1 * g1.y};
+          }
+          if (o == 0) {
+            const cpx<T> g2 = S[2 * n * TB + sx(j)];
+            v = cpx<T>{v.x + q2 * g2.x, v.y + q2 * g2.y};
+          }
+          u[t] = v;
+        }
+        stage_first<1, T>(rc, u, tw, n);
+#pragma unroll
+        for (int t = 0; t < R; ++t) D[sx(i * R + t)] = u[t];
+      }
+    });
+    __syncthreads();
+    const cpx<T>* cur = middle(axi, std::integral_constant<int, 1>{}, D, E);
+    cpx<T>* g = field(o);
+    axi.last([&](auto rc) {
+      constexpr int R = decltype(rc)::R;
+      const int nb = axi.nbl();
+      for (int i = i0; i < nb; i += ni) {
+        cpx<T> u[R];
+        load_stage<1, T>(rc, u, cur, tw, i, i, nb, nb, n, sx);
+        if (ok) {
+#pragma unroll
+          for (int t = 0; t < R; ++t) g[(i + t * nb) * st] = u[t];
+        }
+      }
+    });
+    __syncthreads();
+  }
+}
+
 // ---- host side --------------------------------------------------------------------
 // what the launch shapes need to know of an axis type
 struct AxisInfo { int n, nst, nbf, nbl, nbmax; };
@@ -990,26 +1271,34 @@ template <typename T> inline RowShape row_shape(const AxisInfo& ax, int nf, int 
 }
 
 template <typename T>
-static int rows_fwd(gbofdft_plan* p, const void* in, void* spec, int64_t fstride, int ld2, int nf, const int* ops,
-             double beta, double scale, double rho0, cudaStream_t st) {
+static int rows_fwd(gbofdft_plan* p, const RbFwd& d, cudaStream_t st) {
   RowsFwd a;
+  memset(&a, 0, sizeof(a));
   a.ax = p->rb[2];
   if (a.ax.nst == 0) return 1;
-  a.in = in; a.out = spec; a.fstride = fstride;
-  a.nrows = p->n[0] * p->n[1]; a.n2h = p->n2h; a.ld2 = ld2; a.nf = nf;
-  for (int f = 0; f < kFields; ++f) a.op[f] = f < nf ? ops[f] : OP_RHO;
-  a.b56 = fabs(beta - 5.0 / 6.0) < 1e-15;
+  const int nf = d.nf;
+  const int* ops = d.op;
+  for (int f = 0; f < GB_RB_FIELDS; ++f) {
+    a.in[f] = f < nf ? d.in[f] : nullptr;
+    a.out[f] = f < nf ? d.out[f] : nullptr;
+    a.op[f] = f < nf ? ops[f] : OP_RHO;
+  }
+  a.nrows = p->n[0] * p->n[1]; a.n2h = p->n2h; a.ld2 = d.ld2; a.nf = nf;
+  a.b56 = fabs(d.beta - 5.0 / 6.0) < 1e-15;
   a.rsq = rb_rsqrt_length(p->n[2]);
-  a.beta.set(beta);
-  a.half.set(0.5 * scale);
-  a.rho0.set(rho0);
-  a.inv0.set(rho0 > 0.0 ? 1.0 / rho0 : 0.0);
+  a.beta.set(d.beta);
+  a.beta2.set(d.beta2);
+  a.half.set(0.5 * d.scale);
+  a.rho0.set(d.rho0);
+  a.inv0.set(d.rho0 > 0.0 ? 1.0 / d.rho0 : 0.0);
+  a.pw_out = d.pw_out; a.pw2_out = d.pw2_out; a.pw_in = d.pw_in;
   a.tw = p->tw[2];
   a.dn.set(p->n[2]);
   a.dnh.set(p->n2h);
   int kind = PK_PLAIN;
   for (int f = 0; f < nf; ++f) {
-    if (ops[f] == OP_SQRT || (ops[f] == OP_POWB && a.b56)) kind = kind > PK_ROOTS ? kind : PK_ROOTS;
+    if (ops[f] >= OP_WGC0) kind = PK_WGC;
+    else if (ops[f] == OP_SQRT || (ops[f] == OP_POWB && a.b56)) kind = kind > PK_ROOTS ? kind : PK_ROOTS;
     else if (ops[f] != OP_RHO) kind = PK_GENERAL;
   }
   auto go = [&](auto kern, const AxisInfo& x, int nbuf) -> int {
@@ -1025,22 +1314,24 @@ static int rows_fwd(gbofdft_plan* p, const void* in, void* spec, int64_t fstride
     using AX = typename decltype(x)::ax;
     const AxisInfo xi = axis_info<AX>(a.ax);
     if (kind == PK_GENERAL) return go(k_rb_rows_fwd<T, PK_GENERAL, AX>, xi, 2);
+    if (kind == PK_WGC) return go(k_rb_rows_fwd<T, PK_WGC, AX>, xi, one_buffer<T, PK_WGC, AX>() ? 1 : 2);
     if (kind == PK_ROOTS) return go(k_rb_rows_fwd<T, PK_ROOTS, AX>, xi, one_buffer<T, PK_ROOTS, AX>() ? 1 : 2);
     return go(k_rb_rows_fwd<T, PK_PLAIN, AX>, xi, one_buffer<T, PK_PLAIN, AX>() ? 1 : 2);
   });
 }
 
 template <typename T>
-static int rows_inv(gbofdft_plan* p, const void* spec, int64_t fstride, int ld2, int nf, void* out, int64_t ostride,
-             double scale, const EvalDesc* ev, const void* rho, const void* vloc, void* pot, int calc_e,
-             double* partials, int64_t* nblk_out, cudaStream_t st) {
+static int rows_inv(gbofdft_plan* p, const RbInv& d, int64_t* nblk_out, cudaStream_t st) {
   RowsInv a;
   memset(&a, 0, sizeof(a));
   a.ax = p->rb[2];
   if (a.ax.nst == 0) return 1;
-  a.in = spec; a.fstride = fstride; a.nrows = p->n[0] * p->n[1]; a.n2h = p->n2h; a.ld2 = ld2; a.nf = nf;
+  const int nf = d.nf;
+  const EvalDesc* ev = d.ev;
+  for (int f = 0; f < nf; ++f) a.in[f] = d.in[f];
+  a.nrows = p->n[0] * p->n[1]; a.n2h = p->n2h; a.ld2 = d.ld2; a.nf = nf;
   a.tw = p->tw[2];
-  a.out = out; a.ostride = ostride; a.scale.set(scale);
+  a.out = d.out; a.ostride = d.ostride; a.scale.set(d.scale);
   const int nrows = a.nrows;
   auto go = [&](auto kern, const AxisInfo& x) -> int {
     const int nbuf = x.nst > 2 ? 2 : 1;
@@ -1059,7 +1350,21 @@ static int rows_inv(gbofdft_plan* p, const void* spec, int64_t fstride, int ld2,
       using AX = inverse_order<decltype(x)>;
       return go(k_rb_rows_inv<T, RI_STORE, AX>, axis_info<AX>(a.ax));
     });
-  a.ev = *ev; a.rho = rho; a.vloc = vloc; a.pot = pot; a.partials = partials;
+  a.ev = *ev; a.rho = d.rho; a.vloc = d.vloc; a.pot = d.pot; a.partials = d.partials;
+  a.base = ev->tf || ev->vw || ev->wt || ev->xc || ev->hartree || ev->pp;
+  a.add = d.add;
+  if (d.wgc) {
+    a.wgc = 1;
+    a.wslot = d.wslot;
+    a.two = d.two;
+    a.w_rho0.set(d.wgc->rho0);
+    a.w_inv0.set(1.0 / d.wgc->rho0);
+    a.w_a.set(d.wgc->alpha);
+    a.w_b.set(d.wgc->beta);
+    a.pa = d.pa; a.pb = d.pb;
+    for (int i = 0; i < 6; ++i) a.wstore[i] = d.wstore[i];
+    a.vstore = d.vstore;
+  }
   const double ctf = 2.87123400018819181594;    // (3/10)(3 pi^2)^(2/3)
   a.tf_v.set(5.0 / 3.0 * ctf * ev->tf_x);
   a.tf_e.set(ctf * ev->tf_x);
@@ -1071,24 +1376,26 @@ static int rows_inv(gbofdft_plan* p, const void* spec, int64_t fstride, int ld2,
   return by_axis<T>(a.ax, [&](auto x) {
     using AX = inverse_order<decltype(x)>;
     const AxisInfo xi = axis_info<AX>(a.ax);
-    return calc_e ? go(k_rb_rows_inv<T, RI_EVAL_E, AX>, xi) : go(k_rb_rows_inv<T, RI_EVAL, AX>, xi);
+    return d.calc_e ? go(k_rb_rows_inv<T, RI_EVAL_E, AX>, xi) : go(k_rb_rows_inv<T, RI_EVAL, AX>, xi);
   });
 }
 
-template <typename T>
-static int cols(gbofdft_plan* p, void* spec, int64_t fstride, int ld2, int nf, int axis, int dir, double scale,
-         const KerDesc* kd, cudaStream_t st) {
+// WGC: the WGC kernel on groups of three fields, else plain columns or (kd) the convolution
+template <typename T, bool WGC>
+static int cols(gbofdft_plan* p, const RbCols& d, cudaStream_t st) {
   Cols a;
   memset(&a, 0, sizeof(a));
+  const int axis = d.axis, nf = d.nf, dir = d.dir, ld2 = d.ld2;
+  const KerDesc* kd = d.kd;
   a.ax = p->rb[axis];
   if (a.ax.nst == 0) return 1;
   a.inv = p->rbi[axis];
   const int outer = p->n[axis == 1 ? 0 : 1];
-  a.data = spec; a.fstride = fstride;
+  for (int f = 0; f < nf; ++f) a.data[f] = d.data[f];
   a.stride = axis == 1 ? ld2 : (int64_t)p->n[1] * ld2;
   a.ostride = axis == 1 ? (int64_t)p->n[1] * ld2 : ld2;
   a.ncol = (unsigned)outer * ld2; a.n2h = p->n2h; a.dld.set(ld2);
-  a.tw = p->tw[axis]; a.scale.set(scale);
+  a.tw = p->tw[axis]; a.scale.set(d.scale);
   a.n0 = p->n[0]; a.n1 = p->n[1]; a.n2 = p->n[2]; a.full = p->full;
   for (int i = 0; i < 9; ++i) a.bg[i].set(p->bg[i]);
   if (kd)
@@ -1097,40 +1404,51 @@ static int cols(gbofdft_plan* p, void* spec, int64_t fstride, int ld2, int nf, i
       a.arr[f] = kd->arr[f];
       a.coef[f].set(kd->coef[f]);
     }
+  a.K = d.K;
+  a.kstride = p->NG;
   constexpr int TB = ColTile<T>::TB;
-  const dim3 grid((a.ncol + TB - 1) / TB, nf);
+  const dim3 grid((a.ncol + TB - 1) / TB, WGC ? nf / 3 : nf);
   auto go = [&](auto kern, const AxisInfo& x) -> int {
     // butterflies of a column side by side.  FP64: one per thread of the stage
     // with the most (idle warps cost nothing on the FP64 pipe).  FP32: as many
     // as keep the threads of every stage busy (the last stage counts twice in
     // the convolution, which continues with the inverse's first).
-    const int cap = (sizeof(T) == 4 ? 400 : 256) / TB;
+    auto smem = [&](int fy) {
+      const int nbuf = WGC ? 3 + fy * (x.nst > 2 ? 2 : 1) : x.nst < 2 ? 0 : (kd || x.nst > 2 ? 2 : 1);
+      return nbuf * sizeof(cpx<T>) * (size_t)TB * x.n;
+    };
+    const int fy = WGC && sizeof(T) == 4 && smem(3) <= kMaxSmem ? 3 : 1;
+    const int cap = WGC ? kWgcThreads<T> / (TB * fy) : (sizeof(T) == 4 ? 400 : 256) / TB;
     const int rounds = (x.nbmax + cap - 1) / cap;
     int ni = (x.nbmax + rounds - 1) / rounds;
     if (sizeof(T) == 4) {
       double best = -1.0;
       for (int c = x.nbl < x.nbf ? x.nbl : x.nbf; c <= x.nbmax && c <= cap; ++c) {
         auto busy = [&](int nb) { return nb / (double)((nb + c - 1) / c * c); };
-        const double r = busy(x.nbf) + (kd ? 2.0 : 1.0) * busy(x.nbl) + 1e-3 * c;
+        const double r = busy(x.nbf) + (kd || WGC ? 2.0 : 1.0) * busy(x.nbl) + 1e-3 * c;
         if (r > best) {
           best = r;
           ni = c;
         }
       }
     }
-    const int nbuf = x.nst < 2 ? 0 : (kd || x.nst > 2 ? 2 : 1);
-    const size_t sm = nbuf * sizeof(cpx<T>) * (size_t)TB * x.n;
+    const size_t sm = smem(fy);
     if (sm > kMaxSmem) return 1;
     if (int rc = gbct::ct_smem(kern, sm)) return rc;
-    kern<<<grid, TB * ni, sm, st>>>(a);
+    kern<<<grid, dim3(TB * ni, fy), sm, st>>>(a);
     return launch_check<T>("rb_cols");
   };
   return by_axis<T>(a.ax, [&](auto x) {
     using AX = typename decltype(x)::ax;
     using AXI = typename decltype(x)::inv;
     const AxisInfo xi = axis_info<AX>(a.ax);
-    if (kd) return go(k_rb_cols<T, -1, true, AX, AXI>, xi);
-    return dir < 0 ? go(k_rb_cols<T, -1, false, AX, AXI>, xi) : go(k_rb_cols<T, 1, false, AX, AXI>, xi);
+    if constexpr (WGC) {
+      if (xi.nst < 2) return 1;
+      return go(k_rb_wgc<T, AX, AXI>, xi);
+    } else {
+      if (kd) return go(k_rb_cols<T, -1, true, AX, AXI>, xi);
+      return dir < 0 ? go(k_rb_cols<T, -1, false, AX, AXI>, xi) : go(k_rb_cols<T, 1, false, AX, AXI>, xi);
+    }
   });
 }
 
@@ -1140,21 +1458,18 @@ static int cols(gbofdft_plan* p, void* spec, int64_t fstride, int ld2, int nf, i
 // column passes in translation units of their own: they compile in parallel).
 #define GB_RB_NAME(base, SUF) GB_RB_CAT(GB_RB_CAT(base##_##SUF, _g), GB_RB_GROUP)
 #define GB_RB_DEFINE_FWD(T, SUF)                                                                                \
-  int GB_RB_NAME(gb_rb_rows_fwd, SUF)(gbofdft_plan* p, const void* in, void* spec, int64_t fstride, int ld2,   \
-                                      int nf, const int* ops, double beta, double scale, double rho0,          \
-                                      cudaStream_t st) {                                                       \
-    return gbrb::rows_fwd<T>(p, in, spec, fstride, ld2, nf, ops, beta, scale, rho0, st);                       \
+  int GB_RB_NAME(gb_rb_rows_fwd, SUF)(gbofdft_plan* p, const RbFwd& d, cudaStream_t st) {                      \
+    return gbrb::rows_fwd<T>(p, d, st);                                                                        \
   }
 #define GB_RB_DEFINE_INV(T, SUF)                                                                                \
-  int GB_RB_NAME(gb_rb_rows_inv, SUF)(gbofdft_plan* p, const void* spec, int64_t fstride, int ld2, int nf,     \
-                                      void* out, int64_t ostride, double scale, const EvalDesc* ev,            \
-                                      const void* rho, const void* vloc, void* pot, int calc_e,                \
-                                      double* partials, int64_t* nblk, cudaStream_t st) {                      \
-    return gbrb::rows_inv<T>(p, spec, fstride, ld2, nf, out, ostride, scale, ev, rho, vloc, pot, calc_e,        \
-                             partials, nblk, st);                                                              \
+  int GB_RB_NAME(gb_rb_rows_inv, SUF)(gbofdft_plan* p, const RbInv& d, int64_t* nblk, cudaStream_t st) {       \
+    return gbrb::rows_inv<T>(p, d, nblk, st);                                                                  \
   }
 #define GB_RB_DEFINE_COLS(T, SUF)                                                                               \
-  int GB_RB_NAME(gb_rb_cols, SUF)(gbofdft_plan* p, void* spec, int64_t fstride, int ld2, int nf, int axis,     \
-                                  int dir, double scale, const KerDesc* kd, cudaStream_t st) {                 \
-    return gbrb::cols<T>(p, spec, fstride, ld2, nf, axis, dir, scale, kd, st);                                  \
+  int GB_RB_NAME(gb_rb_cols, SUF)(gbofdft_plan* p, const RbCols& d, cudaStream_t st) {                         \
+    return gbrb::cols<T, false>(p, d, st);                                                                     \
+  }
+#define GB_RB_DEFINE_WGC(T, SUF)                                                                                \
+  int GB_RB_NAME(gb_rb_wgc, SUF)(gbofdft_plan* p, const RbCols& d, cudaStream_t st) {                          \
+    return gbrb::cols<T, true>(p, d, st);                                                                      \
   }

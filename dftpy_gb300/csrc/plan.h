@@ -38,8 +38,6 @@ struct gbofdft_plan {
   int plane_variant;     // radix-schedule variant of the plane pass (autotuned)
   float* wt_pm;          // plane-major copy of the last WT kernel table built on this plan
   const void* wt_pm_src; // the table that copy belongs to
-  float* wgc_pm;         // plane-major copy of the last WGC kernels (4 x NG) built on this plan
-  const void* wgc_pm_src; // the kernels that copy belongs to
   // the buffers the last two TN preconditioners were built into and their
   // mean densities (a rebuild is skipped when both match): the FP32 stage
   // and the refinement's Hessian products keep one each on the same plan
@@ -91,16 +89,48 @@ int gb_cols(gbofdft_plan* p, void* spec, int64_t fstride, int ld2, int nf, int a
 int gb_cols_conv(gbofdft_plan* p, void* spec, int64_t fstride, int ld2, int nf, const KerDesc& kd,
                  double scale, cudaStream_t st);
 // register-blocked passes (passes_rb_*.cu): return 1 when the axis length has a
-// prime factor above 7, 0 on success, an error code otherwise
-#define GB_RB_DECLARE(SUF)                                                                                     \
-  int gb_rb_rows_fwd_##SUF(gbofdft_plan*, const void* in, void* spec, int64_t fstride, int ld2, int nf,        \
-                           const int* ops, double beta, double scale, double rho0, cudaStream_t);              \
-  int gb_rb_rows_inv_##SUF(gbofdft_plan*, const void* spec, int64_t fstride, int ld2, int nf, void* out,       \
-                           int64_t ostride, double scale, const EvalDesc* ev, const void* rho,                 \
-                           const void* vloc, void* pot, int calc_e, double* partials, int64_t* nblk,           \
-                           cudaStream_t);                                                                      \
-  int gb_rb_cols_##SUF(gbofdft_plan*, void* spec, int64_t fstride, int ld2, int nf, int axis, int dir,          \
-                       double scale, const KerDesc* kd, cudaStream_t);
+// prime factor above 7 or its lines do not fit, 0 on success, an error code otherwise
+#define GB_RB_FIELDS 10   // fused terms (GB_MAX_FIELDS - 1) and the six fields of the WGC term
+struct RbFwd {            // forward rows: fields derived from in[0] (OP_RHO alone: in[f]) to spectra out[f]
+  const void* in[GB_RB_FIELDS];
+  void* out[GB_RB_FIELDS];
+  int nf, ld2;
+  int op[GB_RB_FIELDS];
+  double beta, scale, rho0;
+  // OP_WGC0..2 on FP64 plans: store rho^beta (and rho^beta2), or take rho^beta from pw_in
+  double beta2;
+  void *pw_out, *pw2_out;
+  const void* pw_in;
+};
+struct RbInv {            // inverse rows: store real fields (ev null) or the evaluation epilogue
+  const void* in[GB_RB_FIELDS];
+  int nf, ld2;
+  void* out;
+  int64_t ostride;
+  double scale;
+  const EvalDesc* ev;
+  const void *rho, *vloc;
+  void* pot;
+  int calc_e, add;        // add: to pot
+  double* partials;       // GB_NE doubles per CTA
+  const gbofdft_wgc* wgc; // the WGC term from the fields wslot ...
+  int wslot, two;
+  const void *pa, *pb;    // FP64: rho^alpha and rho^beta
+  void* wstore[6];        // with vstore: copies of its fields and potential
+  void* vstore;
+};
+struct RbCols {           // columns of nf spectra: dir, the convolution (kd) or the WGC term (K)
+  void* data[GB_RB_FIELDS];
+  int nf, ld2, axis, dir;
+  double scale;
+  const KerDesc* kd;
+  const void* K;
+};
+#define GB_RB_DECLARE(SUF)                                                                \
+  int gb_rb_rows_fwd_##SUF(gbofdft_plan*, const RbFwd&, cudaStream_t);                    \
+  int gb_rb_rows_inv_##SUF(gbofdft_plan*, const RbInv&, int64_t* nblk, cudaStream_t);     \
+  int gb_rb_cols_##SUF(gbofdft_plan*, const RbCols&, cudaStream_t);                       \
+  int gb_rb_wgc_##SUF(gbofdft_plan*, const RbCols&, cudaStream_t);
 GB_RB_DECLARE(f64_g0)
 GB_RB_DECLARE(f32_g0)
 GB_RB_DECLARE(f32_g1)
@@ -108,6 +138,12 @@ GB_RB_DECLARE(f32_g2)
 GB_RB_DECLARE(f32_g3)
 GB_RB_DECLARE(f32_g4)
 #undef GB_RB_DECLARE
+int gb_rb_rows_fwd(gbofdft_plan*, const RbFwd&, cudaStream_t);
+int gb_rb_rows_inv(gbofdft_plan*, const RbInv&, int64_t* nblk, cudaStream_t);
+int gb_rb_cols(gbofdft_plan*, const RbCols&, cudaStream_t);
+int gb_rb_wgc(gbofdft_plan*, const RbCols&, cudaStream_t);
+// every axis has register-blocked passes, the WGC columns included
+bool gb_rb_wgc_ok(const gbofdft_plan* p);
 void gb_rb_plan(gbofdft_plan* p);   // the plan's rb / rbi from its lengths and precision
 // compile-time-size passes (passes_ct_*.cu): return 1 when the size has no
 // specialisation, 0 on success, an error code otherwise
@@ -171,6 +207,14 @@ int gb_use_ct();  // 0 forces the generic passes (GBOFDFT_GENERIC_FFT=1)
 
 int gb_lwt_eval(gbofdft_plan* p, const void* rho, gbofdft_lwt* d, void* pot, double* energies, int calc_v,
                 int calc_e, cudaStream_t st);
+// the fused terms (ev, kd, nf fields of ops) and the WGC term in one pipeline;
+// 1: an axis has no register-blocked passes
+int gb_wgc_eval_fused(gbofdft_plan* p, const void* rho, int nf, const int* ops, double beta, const KerDesc& kd,
+                      const EvalDesc& ev, const void* vloc, const gbofdft_wgc* d, void* pot, double* energies,
+                      int calc_e, cudaStream_t st);
+// the total of a row pass's energy partials (k_energy_final)
+int gb_energy_final(gbofdft_plan* p, const double* partials, int64_t nblk, double e_ion, double* energies,
+                    cudaStream_t st);
 // store_ref (FP64 plans): keep this evaluation as the reference of gb_wgc_eval_delta
 int gb_wgc_eval(gbofdft_plan* p, const void* rho, const gbofdft_wgc* d, void* pot, double* energies, int calc_v,
                 int calc_e, int store_ref, cudaStream_t st);

@@ -17,6 +17,7 @@
 // inverse transforms and a pointwise pass adding V and reducing E.  With
 // a == b, Y = X and half the transforms are skipped.
 #include <math.h>
+#include <string.h>
 
 #include "gkernels.cuh"
 #include "plan.h"
@@ -34,21 +35,10 @@ struct WgcBufs {
   double* vref;     // FP64 plans: the NL potential of the last reference evaluation [N]
   double* eref;     // FP64 plans: its NL energy [1]
   double* pw[2];    // FP64 plans: rho^a and rho^b of the current evaluation [N] each
-  void* o[6];       // FP32 plane-pipeline plans: the combinations' spectra (plane-major)
 };
-
-// FP32 plans whose grid has the plane pipeline run the WGC transforms there
-bool wgc_plane(const gbofdft_plan* p) { return p->prec == GBOFDFT_F32 && p->plane_ok && gb_use_ct(); }
 
 constexpr int kBlocks = 1216;
 constexpr int kThreads = 256;
-
-// per-CTA energy partials: the grid-stride passes use kBlocks, the fused
-// inverse row pass of the plane pipeline one per pair of rows at most
-int64_t wgc_part_count(const gbofdft_plan* p) {
-  const int64_t rows = (int64_t)p->n[0] * p->n[1] / 2 + 1;
-  return rows > kBlocks ? rows : kBlocks;
-}
 
 WgcBufs wgc_layout(const gbofdft_plan* p, void* work) {
   const size_t fb = r256(gb_elem(p) * (size_t)p->N), sb = r256(2 * gb_elem(p) * (size_t)p->NGld);
@@ -57,11 +47,10 @@ WgcBufs wgc_layout(const gbofdft_plan* p, void* work) {
   for (int i = 0; i < 6; ++i) { W.f[i] = b; b += fb; }
   for (int i = 0; i < 6; ++i) { W.s[i] = b; b += sb; }
   W.part = reinterpret_cast<double*>(b);
-  b += r256(sizeof(double) * (size_t)wgc_part_count(p));
+  b += r256(sizeof(double) * kBlocks);
   W.vref = nullptr;
   W.eref = nullptr;
   W.pw[0] = W.pw[1] = nullptr;
-  for (int i = 0; i < 6; ++i) W.o[i] = nullptr;
   if (p->prec == GBOFDFT_F64) {
     W.vref = reinterpret_cast<double*>(b);
     b += r256(sizeof(double) * (size_t)p->N);
@@ -71,8 +60,6 @@ WgcBufs wgc_layout(const gbofdft_plan* p, void* work) {
       W.pw[i] = reinterpret_cast<double*>(b);
       b += r256(sizeof(double) * (size_t)p->N);
     }
-  } else if (wgc_plane(p)) {
-    for (int i = 0; i < 6; ++i) { W.o[i] = b; b += sb; }
   }
   return W;
 }
@@ -82,9 +69,8 @@ WgcBufs wgc_layout(const gbofdft_plan* p, void* work) {
 // (in f[0..5]), its NL potential and energy
 size_t wgc_bytes(const gbofdft_plan* p) {
   size_t b = 6 * r256(gb_elem(p) * (size_t)p->N) + 6 * r256(2 * gb_elem(p) * (size_t)p->NGld) +
-             r256(sizeof(double) * (size_t)wgc_part_count(p));
+             r256(sizeof(double) * kBlocks);
   if (p->prec == GBOFDFT_F64) b += 3 * r256(sizeof(double) * (size_t)p->N) + 256;
-  else if (wgc_plane(p)) b += 6 * r256(2 * gb_elem(p) * (size_t)p->NGld);
   return b;
 }
 
@@ -126,21 +112,6 @@ __global__ void k_wgc_kernels(GInfo g, double tkf, double C, const double* __res
           g, i0, i1, k2, [&](double gg) { return C * table_at(tab, m, t0, h, c, sqrt(gg) / tkf); });
       out[c * total + id] = (T)v;
     }
-  }
-}
-
-// plane-major copy of the four kernels: element (i0, i1, k2) of kernel c at
-// pm[c NG + (k2 n0 + i0) n1 + i1]
-__global__ void k_wgc_kernels_pm(GInfo g, const float* __restrict__ K, float* __restrict__ pm) {
-  const int64_t total = (int64_t)g.n0 * g.n1 * g.n2h;
-  for (int64_t id = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; id < 4 * total;
-       id += (int64_t)gridDim.x * blockDim.x) {
-    const int c = (int)(id / total);
-    const int64_t r = id - c * total;            // plane-major index within kernel c
-    const int64_t plane = (int64_t)g.n0 * g.n1;
-    const int k2 = (int)(r / plane);
-    const int64_t rr = r - k2 * plane;           // i0 n1 + i1
-    pm[id] = K[c * total + rr * g.n2h + k2];
   }
 }
 
@@ -320,36 +291,129 @@ __global__ void k_wgc_energy(const double* __restrict__ part, int nb, double dV,
   }
 }
 
-// X0..X2 (and Y0..Y2) into W.f[0..5] on the plane pipeline (FP32): the
-// transform inputs are made from rho in the forward row pass (rho given) or
-// read from W.f[0..5] (rho null); K: the plane-major kernels.  pot given
-// (potential-only evaluations): the inverse row pass adds the NL potential
-// to pot directly instead of storing the fields.
-int wgc_xfields_plane(gbofdft_plan* p, const WgcBufs& W, int two, const float* K, const float* rho,
-                      const gbofdft_wgc* d, cudaStream_t st, float* pot = nullptr, double* part = nullptr,
-                      int64_t* nblk = nullptr) {
-  const int nfield = two ? 6 : 3;
-  const int64_t fs = (int64_t)((char*)W.s[1] - (char*)W.s[0]) / (int64_t)sizeof(float2);
-  const int64_t os = (int64_t)((char*)W.o[1] - (char*)W.o[0]) / (int64_t)sizeof(float2);
-  const int64_t rs = (int64_t)((char*)W.f[1] - (char*)W.f[0]) / (int64_t)sizeof(float);
-  int rc = 0;
-  if (rho) {
-    rc = gb_ct_rows_fwd_wgc_pm_f32(p, rho, W.s[0], fs, d->beta, d->rho0, st);
-    if (!rc && two) rc = gb_ct_rows_fwd_wgc_pm_f32(p, rho, W.s[3], fs, d->alpha, d->rho0, st);
-  } else {
-    const int op = OP_RHO;
-    for (int i = 0; i < nfield && !rc; ++i) rc = gb_ct_rows_fwd_pm_f32(p, W.f[i], W.s[i], fs, 1, &op, 1.0, st);
+// The transforms of the WGC fields on the register-blocked passes, from their
+// row spectra in s[0..5] to the combinations' row spectra (axis 1 forward,
+// axis 0 with the kernels, axis 1 inverse), with nb more spectra (the fused
+// terms', convolved by kd) riding in the axis-1 launches
+int wgc_columns(gbofdft_plan* p, void* const* s, int nfield, const void* K, int nb, const KerDesc* kd,
+                cudaStream_t st) {
+  RbCols c;
+  memset(&c, 0, sizeof(c));
+  for (int i = 0; i < nb; ++i) c.data[i] = reinterpret_cast<char*>(p->spec) + 2 * gb_elem(p) * (size_t)(i * p->NGld);
+  for (int i = 0; i < nfield; ++i) c.data[nb + i] = s[i];
+  c.ld2 = p->ld2;
+  c.scale = 1.0;
+  c.nf = nb + nfield; c.axis = 1; c.dir = -1;
+  int rc = gb_rb_cols(p, c, st);
+  const double scale = 0.5 / (double)p->N;   // 1 / N, and the row pass's factor 2
+  if (!rc && nb) {
+    KerDesc k2 = *kd;
+    for (int f = 0; f < nb; ++f) k2.coef[f] = kd->coef[f] * scale;
+    RbCols b = c;
+    b.nf = nb; b.axis = 0; b.kd = &k2;
+    rc = gb_rb_cols(p, b, st);
   }
-  if (!rc) rc = gb_plane_fwd_f32(p, W.s[0], fs, nfield, st);
-  if (!rc) rc = gb_plane_wgc_inv_f32(p, W.s[0], fs, W.o[0], os, two ? 2 : 1, K, 1.0 / (double)p->N, st);
-  if (!rc && pot && rho) {
-    rc = gb_ct_rows_inv_wgc_pm_f32(p, W.o[0], os, two, rho, d->rho0, d->alpha, d->beta, pot, part, nblk, st);
-    if (rc == 1) return gb_set_error(GBOFDFT_ERR_STATE, "wgc: plane size without specialisation");
-    return rc;
+  if (!rc) {
+    RbCols w = c;
+    for (int i = 0; i < nfield; ++i) w.data[i] = s[i];
+    w.nf = nfield; w.axis = 0; w.scale = scale; w.K = K;
+    rc = gb_rb_wgc(p, w, st);
   }
-  for (int h = 0; h < (two ? 2 : 1) && !rc; ++h) rc = gb_ct_rows_inv_store_pm_f32(p, W.o[3 * h], os, 3, W.f[3 * h], rs, st);
-  if (rc == 1) return gb_set_error(GBOFDFT_ERR_STATE, "wgc: plane size without specialisation");
+  c.dir = 1;
+  if (!rc) rc = gb_rb_cols(p, c, st);
   return rc;
+}
+
+// forward rows of the WGC fields: rho^b (then rho^a) times 1, u, u^2
+int wgc_rows_fwd(gbofdft_plan* p, const WgcBufs& W, int two, const void* rho, const gbofdft_wgc* d, cudaStream_t st) {
+  int rc = 0;
+  for (int h = 0; h < (two ? 2 : 1) && !rc; ++h) {
+    RbFwd r;
+    memset(&r, 0, sizeof(r));
+    for (int i = 0; i < 3; ++i) {
+      r.in[i] = rho;
+      r.out[i] = W.s[3 * h + i];
+      r.op[i] = OP_WGC0 + i;
+    }
+    r.nf = 3; r.ld2 = p->ld2; r.scale = 2.0; r.rho0 = d->rho0;
+    r.beta = h == 0 ? d->beta : d->alpha;
+    r.beta2 = d->alpha;
+    if (h == 0) {
+      r.pw_out = W.pw[1];
+      r.pw2_out = two ? W.pw[0] : nullptr;
+    } else {
+      r.pw_in = W.pw[0];
+    }
+    rc = gb_rb_rows_fwd(p, r, st);
+  }
+  return rc;
+}
+
+// inverse rows with the WGC term (and the fused terms ev, nb fields before its)
+RbInv wgc_rows_inv(gbofdft_plan* p, const WgcBufs& W, int two, int nb, const EvalDesc* ev, const void* rho,
+                   const gbofdft_wgc* d, void* pot) {
+  RbInv r;
+  memset(&r, 0, sizeof(r));
+  const int nfield = two ? 6 : 3;
+  for (int i = 0; i < nb; ++i) r.in[i] = reinterpret_cast<char*>(p->spec) + 2 * gb_elem(p) * (size_t)(i * p->NGld);
+  for (int i = 0; i < nfield; ++i) r.in[nb + i] = W.s[i];
+  r.nf = nb + nfield; r.ld2 = p->ld2; r.ev = ev; r.rho = rho; r.pot = pot;
+  r.partials = p->partials;
+  r.wgc = d; r.wslot = nb; r.two = two;
+  r.pa = two ? W.pw[0] : W.pw[1];
+  r.pb = W.pw[1];
+  return r;
+}
+
+// the NL energy slot of the row pass's partials (GB_NE per CTA), as k_wgc_energy
+__global__ void k_wgc_energy_rows(const double* __restrict__ part, int64_t nb, double dV, double* __restrict__ e,
+                                  double* __restrict__ eref) {
+  __shared__ double red[32];
+  KSum s;
+  s.init();
+  for (int64_t i = threadIdx.x; i < nb; i += blockDim.x) s.add(part[i * GB_NE + GB_E_NL]);
+  const double v = warp_sum(s.value());
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    KSum t;
+    t.init();
+    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t.add(red[w]);
+    const double en = t.value() * dV;
+    if (e) {
+      e[GB_E_NL] += en;
+      e[GB_E_TOTAL] += en;
+    }
+    if (eref) *eref = en;
+  }
+}
+
+// the WGC term alone on the register-blocked passes, added to pot / energies
+int wgc_run_rb(gbofdft_plan* p, const void* rho, const gbofdft_wgc* d, void* pot, double* energies, int calc_e,
+               int store_ref, cudaStream_t st) {
+  WgcBufs W = wgc_layout(p, d->work);
+  const int two = fabs(d->alpha - d->beta) > 1e-12;
+  int rc = wgc_rows_fwd(p, W, two, rho, d, st);
+  if (!rc) rc = wgc_columns(p, W.s, two ? 6 : 3, d->kernels, 0, nullptr, st);
+  if (rc) return rc;
+  EvalDesc ev;
+  memset(&ev, 0, sizeof(ev));
+  RbInv r = wgc_rows_inv(p, W, two, 0, &ev, rho, d, pot);
+  r.add = 1;
+  r.calc_e = calc_e || store_ref;
+  if (store_ref) {
+    for (int i = 0; i < 6; ++i) r.wstore[i] = W.f[i];
+    r.vstore = W.vref;
+  }
+  int64_t nblk = 0;
+  if ((rc = gb_rb_rows_inv(p, r, &nblk, st))) return rc;
+  if (r.calc_e) {
+    if (nblk > p->max_partials) return gb_set_error(GBOFDFT_ERR_STATE, "wgc: partials buffer too small");
+    k_wgc_energy_rows<<<1, 256, 0, st>>>(p->partials, nblk, p->dV, calc_e ? energies : nullptr,
+                                         store_ref ? W.eref : nullptr);
+    GB_CHECK_LAUNCH();
+  }
+  return 0;
 }
 
 // X0..X2 (and Y0..Y2) into W.f[0..5] from the transform inputs in W.f[0..5]
@@ -390,30 +454,11 @@ int wgc_run(gbofdft_plan* p, const void* rho, const gbofdft_wgc* d, void* pot, d
   WgcBufs W = wgc_layout(p, d->work);
   const int two = fabs(d->alpha - d->beta) > 1e-12;
   const T* r = reinterpret_cast<const T*>(rho);
-  int rc;
-  if (wgc_plane(p) && p->wgc_pm && p->wgc_pm_src == d->kernels) {
-    if (calc_v && !store_ref) {
-      // the inverse rows add the potential themselves (and sum the energy
-      // integrand per CTA) instead of storing the six fields
-      int64_t nblk = 0;
-      rc = wgc_xfields_plane(p, W, two, p->wgc_pm, reinterpret_cast<const float*>(rho), d, st,
-                             reinterpret_cast<float*>(pot), calc_e ? W.part : nullptr, &nblk);
-      if (rc || !calc_e) return rc;
-      if (nblk > wgc_part_count(p)) return gb_set_error(GBOFDFT_ERR_STATE, "wgc: partials buffer too small");
-      k_wgc_energy<<<1, 256, 0, st>>>(W.part, (int)nblk, p->dV, energies, nullptr, nullptr);
-      GB_CHECK_LAUNCH();
-      gb_count_launch();
-      return 0;
-    }
-    rc = wgc_xfields_plane(p, W, two, p->wgc_pm, reinterpret_cast<const float*>(rho), d, st);
-  } else {
-    k_wgc_prep<T><<<kBlocks, kThreads, 0, st>>>(p->N, r, (T)d->rho0, (T)d->alpha, (T)d->beta, two, (T*)W.f[0],
-                                                (T*)W.f[1], (T*)W.f[2], (T*)W.f[3], (T*)W.f[4], (T*)W.f[5],
-                                                (T*)W.pw[0], (T*)W.pw[1]);
-    GB_CHECK_LAUNCH();
-    gb_count_launch();
-    rc = wgc_xfields<T>(p, W, two, d->kernels, st);
-  }
+  k_wgc_prep<T><<<kBlocks, kThreads, 0, st>>>(p->N, r, (T)d->rho0, (T)d->alpha, (T)d->beta, two, (T*)W.f[0],
+                                              (T*)W.f[1], (T*)W.f[2], (T*)W.f[3], (T*)W.f[4], (T*)W.f[5],
+                                              (T*)W.pw[0], (T*)W.pw[1]);
+  GB_CHECK_LAUNCH();
+  int rc = wgc_xfields<T>(p, W, two, d->kernels, st);
   if (rc) return rc;
   T* vstore = nullptr;
   if (store_ref) {
@@ -583,11 +628,35 @@ static int wgc_check(const gbofdft_plan* p, const gbofdft_wgc* d) {
   return 0;
 }
 
+int gb_wgc_eval_fused(gbofdft_plan* p, const void* rho, int nf, const int* ops, double beta, const KerDesc& kd,
+                      const EvalDesc& ev, const void* vloc, const gbofdft_wgc* d, void* pot, double* energies,
+                      int calc_e, cudaStream_t st) {
+  if (!gb_rb_wgc_ok(p)) return 1;
+  int rc = wgc_check(p, d);
+  if (rc) return rc;
+  WgcBufs W = wgc_layout(p, d->work);
+  const int two = fabs(d->alpha - d->beta) > 1e-12;
+  if (nf > 0) rc = gb_rows_fwd(p, rho, p->spec, p->NGld, p->ld2, nf, ops, beta, 2.0, st);
+  if (!rc) rc = wgc_rows_fwd(p, W, two, rho, d, st);
+  if (!rc) rc = wgc_columns(p, W.s, two ? 6 : 3, d->kernels, nf, &kd, st);
+  if (rc) return rc;
+  RbInv r = wgc_rows_inv(p, W, two, nf, &ev, rho, d, pot);
+  r.vloc = vloc;
+  r.calc_e = calc_e;
+  int64_t nblk = 0;
+  if ((rc = gb_rb_rows_inv(p, r, &nblk, st))) return rc;
+  return calc_e ? gb_energy_final(p, p->partials, nblk, ev.e_ion, energies, st) : 0;
+}
+
 int gb_wgc_eval(gbofdft_plan* p, const void* rho, const gbofdft_wgc* d, void* pot, double* energies, int calc_v,
                 int calc_e, int store_ref, cudaStream_t st) {
   int rc = wgc_check(p, d);
   if (rc) return rc;
   GB_REQUIRE(!store_ref || p->prec == GBOFDFT_F64, "wgc: a delta reference needs an FP64 plan");
+  if (gb_rb_wgc_ok(p) && (calc_v || store_ref)) {
+    rc = wgc_run_rb(p, rho, d, pot, energies, calc_e, store_ref, st);
+    if (rc != 1) return rc;
+  }
   return p->prec == GBOFDFT_F64 ? wgc_run<double>(p, rho, d, pot, energies, calc_v, calc_e, store_ref, st)
                                 : wgc_run<float>(p, rho, d, pot, energies, calc_v, calc_e, 0, st);
 }
@@ -613,10 +682,29 @@ int gb_wgc_eval_delta(gbofdft_plan* p64, gbofdft_plan* p32, const double* rho, c
                                                  f[4], f[5]);
   GB_CHECK_LAUNCH();
   gb_count_launch();
-  if (wgc_plane(p32) && p32->wgc_pm && p32->wgc_pm_src == d32->kernels)
-    rc = wgc_xfields_plane(p32, W32, two, p32->wgc_pm, nullptr, d32, st);
-  else
-    rc = wgc_xfields<float>(p32, W32, two, d32->kernels, st);
+  rc = 1;
+  if (gb_rb_wgc_ok(p32)) {
+    const int nfield = two ? 6 : 3;
+    RbFwd r;
+    memset(&r, 0, sizeof(r));
+    for (int i = 0; i < nfield; ++i) {
+      r.in[i] = W32.f[i];
+      r.out[i] = W32.s[i];
+      r.op[i] = OP_RHO;
+    }
+    r.nf = nfield; r.ld2 = p32->ld2; r.scale = 2.0;
+    rc = gb_rb_rows_fwd(p32, r, st);
+    if (!rc) rc = wgc_columns(p32, W32.s, nfield, d32->kernels, 0, nullptr, st);
+    if (!rc) {
+      RbInv v;
+      memset(&v, 0, sizeof(v));
+      for (int i = 0; i < nfield; ++i) v.in[i] = W32.s[i];
+      v.nf = nfield; v.ld2 = p32->ld2; v.out = W32.f[0]; v.scale = 1.0;
+      v.ostride = (int64_t)((char*)W32.f[1] - (char*)W32.f[0]) / (int64_t)sizeof(float);
+      rc = gb_rb_rows_inv(p32, v, nullptr, st);
+    }
+  }
+  if (rc == 1) rc = wgc_xfields<float>(p32, W32, two, d32->kernels, st);
   if (rc) return rc;
   const double* xr[6];
   for (int i = 0; i < 6; ++i) xr[i] = reinterpret_cast<const double*>(W64.f[two || i < 3 ? i : i - 3]);
@@ -666,23 +754,6 @@ int gbofdft_wgc_kernels(gbofdft_plan* p, double rho0, double alpha, double beta,
     k_wgc_kernels<float><<<nblk, 256, 0, st>>>(p->gi, tkf, C, table, m, t0, h, (float*)out);
   GB_CHECK_LAUNCH();
   gb_count_launch();
-  if (wgc_plane(p)) {
-    // plans with the plane pipeline keep a plane-major copy (allocated with
-    // the first kernels built on the plan)
-    if (!p->wgc_pm) {
-      cudaError_t e = cudaMalloc(&p->wgc_pm, sizeof(float) * 4 * (size_t)p->NG);
-      if (e != cudaSuccess) {
-        p->wgc_pm = nullptr;
-        return gb_set_error(GBOFDFT_ERR_ALLOC, "wgc kernels: plane-major copy: %s", cudaGetErrorString(e));
-      }
-    }
-    const int64_t n4 = 4 * total;
-    k_wgc_kernels_pm<<<(int)((n4 + 255) / 256 > 4096 ? 4096 : (n4 + 255) / 256), 256, 0, st>>>(
-        p->gi, reinterpret_cast<const float*>(out), p->wgc_pm);
-    GB_CHECK_LAUNCH();
-    gb_count_launch();
-    p->wgc_pm_src = out;
-  }
   return GBOFDFT_OK;
 }
 
