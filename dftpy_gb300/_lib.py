@@ -164,6 +164,7 @@ _SIGS = [
     ("gbofdft_dcsrch", ctypes.c_int, [ctypes.POINTER(ctypes.c_double), ctypes.c_int64,
                                       ctypes.POINTER(ctypes.c_double), ctypes.c_double, ctypes.c_double,
                                       ctypes.c_int]),
+    ("gbofdft_spline", ctypes.c_int, [ctypes.c_int64, _P, _P, _P]),
 ]
 
 EXPORTED = [s[0] for s in _SIGS]

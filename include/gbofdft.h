@@ -511,6 +511,15 @@ int gbofdft_optimize_tn_split(gbofdft_plan* plan, const gbofdft_functional* f, g
  */
 int gbofdft_dcsrch(double* state, int64_t state_len, double* stp, double f, double g, int task);
 
+/*
+ * Cubic spline through (x[i], y[i]), i < n, x rising, with not-a-knot ends
+ * (host only; n >= 4): c[4 i .. 4 i + 3] = (a, b, c, d) of
+ * a + b u + c u^2 + d u^3 on [x[i], x[i + 1]], u = t - x[i], n - 1 pieces.
+ * Replaces scipy.interpolate.splrep(x, y, k=3, s=0) as the reference uses it
+ * (functional/pseudo/__init__.py:350-375).
+ */
+int gbofdft_spline(int64_t n, const double* x, const double* y, double* c);
+
 /* ---- evaluation schedules (autotuning) ----------------------------------------
  * No reference counterpart (the reference's only FFT planning is pyFFTW's
  * FFTW_MEASURE, math_utils.py:181-222).  Schedule 0 is the column-pass
