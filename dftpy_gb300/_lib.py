@@ -95,6 +95,7 @@ _SIGS = [
     ("gbofdft_plan_sizes", ctypes.c_int, [_P, ctypes.POINTER(ctypes.c_int64)]),
     ("gbofdft_fft_r2c", ctypes.c_int, [_P, _P, _P, _P]),
     ("gbofdft_fft_c2r", ctypes.c_int, [_P, _P, _P, _P]),
+    ("gbofdft_mean", ctypes.c_int, [_P, ctypes.c_int64, ctypes.c_int, ctypes.POINTER(ctypes.c_double), _P]),
     ("gbofdft_convolve", ctypes.c_int, [_P, _P, _P, ctypes.c_int, _P, ctypes.c_double, _P]),
     ("gbofdft_convolve_noalloc", ctypes.c_int, [ctypes.POINTER(ctypes.c_int), ctypes.POINTER(ctypes.c_double),
                                                 ctypes.c_int, ctypes.c_int, _P, _P, ctypes.c_int, _P,
@@ -230,6 +231,18 @@ def stream_ptr(stream=None):
     import torch
     s = torch.cuda.current_stream() if stream is None else stream
     return ctypes.c_void_p(s.cuda_stream)
+
+
+def mean(t):
+    """Mean of a real CUDA tensor in FP64, as a Python float (``gbofdft_mean``)."""
+    import torch
+    if t.dtype not in (torch.float32, torch.float64) or t.numel() == 0:
+        return float(t.to(torch.float64).mean())
+    t = t.contiguous()
+    out = ctypes.c_double()
+    check(load().gbofdft_mean(ptr(t), t.numel(), F64 if t.dtype == torch.float64 else F32, ctypes.byref(out),
+                              stream_ptr()), "mean")
+    return out.value
 
 
 def ptr(t):

@@ -60,7 +60,7 @@ class KEDF(AbstractFunctional):
         density moves by more than 1e-6 or the grid changes."""
         rho0 = self.options.get("rho0", None)
         if not rho0:
-            rho0 = float(rho.as_subclass(torch.Tensor).to(torch.float64).mean())
+            rho0 = _lib.mean(rho.as_subclass(torch.Tensor))
         s = self._kernels_by_dtype.setdefault(rho.dtype, {"Kernel": None, "rho0": 0.0, "shape": None,
                                                           "dtype": rho.dtype})
         self.ke_kernel_saved = s

@@ -88,6 +88,11 @@ int gbofdft_fft_r2c(gbofdft_plan* plan, const void* in, void* out, void* stream)
  * Replaces ReciprocalField.ifft(force_real=True) (src/dftpy/field.py:739-764). */
 int gbofdft_fft_c2r(gbofdft_plan* plan, const void* in, void* out, void* stream);
 
+/* *mean (host) = mean of the n >= 1 values at x (device, precision
+ * GBOFDFT_F32 or GBOFDFT_F64), summed in double; waits for the stream.
+ * Replaces the mean density of get_ke_kernel_wt (functional/kedf/wt.py:58-73). */
+int gbofdft_mean(const void* x, int64_t n, int precision, double* mean, void* stream);
+
 /* Reciprocal-space kernels for gbofdft_convolve */
 enum gbofdft_kernel { GBOFDFT_KER_NONE = 0, GBOFDFT_KER_HARTREE = 1, GBOFDFT_KER_G2 = 2, GBOFDFT_KER_ARRAY = 3 };
 
