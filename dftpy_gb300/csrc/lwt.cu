@@ -9,7 +9,8 @@
 // [k_i, k_i+1] holding k_F(r) gives the interpolation weights.  The
 // reference's second potential term sum_i K_i fft(rho^alpha w_i) (with masked
 // interval weights) is regrouped by linearity into one forward transform per
-// knot of the accumulated weight field.
+// knot of the accumulated weight field.  Linear interpolation takes the knots in
+// batches (lwt_linear), Hermite interpolation one by one (lwt_knots).
 #include <math.h>
 #include <string.h>
 
@@ -138,6 +139,82 @@ __global__ void k_lwt_acc(GInfo g, BG<T> bg, const cpx<T>* __restrict__ U, int64
   }
 }
 
+// Kernel fields of a batch of knots (linear interpolation): out[q] = scale K(|G| / k_q),
+// out[m + q] = scale K'(|G| / k_q) / k_q.  Bound by the table look-ups (neighbouring
+// |G| are tens of table cells apart, a 32-byte sector for each): this pass has no
+// shared memory to take L1 from them, K and K' of a cell share the sector in FP32
+// (tab: 8 coefficients a cell), and the root is taken once for all knots.  The
+// column passes then read the fields; looked up as they loaded, a field cost them
+// 75 us more at 360^3 FP32, and K is wanted twice.
+struct TabArgs {
+  int m, deriv;
+  double inv_kf[GB_LWT_BATCH];
+  double scale;
+  int64_t stride;
+};
+template <typename T>
+__device__ __forceinline__ void tab_pair(const UTable<T>& tk, const UTable<T>& td, const T* tab, int deriv, T eta, T* v) {
+  v[0] = tk.endval;
+  v[1] = td.endval;
+  if (!(eta < tk.etamax)) return;
+  int j = (int)(eta * tk.inv_deta);
+  j = j > tk.neta - 2 ? tk.neta - 2 : (j < 0 ? 0 : j);
+  const T u = eta - j * tk.deta;
+  if constexpr (sizeof(T) == 4) {
+    const float4* c = reinterpret_cast<const float4*>(tab) + 2 * (size_t)j;
+    const float4 a = __ldg(c);
+    v[0] = a.x + u * (a.y + u * (a.z + u * a.w));
+    if (deriv) {
+      const float4 b = __ldg(c + 1);
+      v[1] = b.x + u * (b.y + u * (b.z + u * b.w));
+    }
+  } else {
+    const T* a = tk.c + 4 * (size_t)j;
+    v[0] = __ldg(a) + u * (__ldg(a + 1) + u * (__ldg(a + 2) + u * __ldg(a + 3)));
+    if (deriv) {
+      const T* b = td.c + 4 * (size_t)j;
+      v[1] = __ldg(b) + u * (__ldg(b + 1) + u * (__ldg(b + 2) + u * __ldg(b + 3)));
+    }
+  }
+}
+template <typename T>
+__global__ void __launch_bounds__(256) k_lwt_tables(GInfo g, BG<T> bg, UTable<T> tk, UTable<T> td,
+                                                    const T* __restrict__ tab, TabArgs a, T* __restrict__ out) {
+  const int nrow = g.n0 * g.n1;
+  for (int row = blockIdx.x; row < nrow; row += gridDim.x) {
+    const int i0 = row / g.n1, i1 = row - i0 * g.n1;
+    for (int k2 = threadIdx.x; k2 < g.n2h; k2 += blockDim.x) {
+      const int m0 = ffreq_l(i0, g.n0), m1 = ffreq_l(i1, g.n1), m2 = g.full ? ffreq_l(k2, g.n2) : k2;
+      const T q = sqrt(gg_a(bg, m0, m1, m2));
+      // the conjugate partner of a Nyquist plane's element
+      const bool nyq = ((g.n0 & 1) == 0 && 2 * i0 == g.n0) || ((g.n1 & 1) == 0 && 2 * i1 == g.n1) ||
+                       (g.full && (g.n2 & 1) == 0 && 2 * k2 == g.n2);
+      const bool pair = nyq && (g.full || k2 == 0 || ((g.n2 & 1) == 0 && 2 * k2 == g.n2));
+      T qp = q;
+      if (pair) {
+        const int p0 = ffreq_l((g.n0 - i0) % g.n0, g.n0), p1 = ffreq_l((g.n1 - i1) % g.n1, g.n1);
+        const int p2 = g.full ? ffreq_l((g.n2 - k2) % g.n2, g.n2) : k2;
+        qp = sqrt(gg_a(bg, p0, p1, p2));
+      }
+      const bool origin = row == 0 && k2 == 0;
+      const int64_t o = (int64_t)row * g.n2h + k2;
+      for (int k = 0; k < a.m; ++k) {
+        const T inv_kf = (T)a.inv_kf[k];
+        T v[2], w[2];
+        tab_pair<T>(tk, td, tab, a.deriv, q * inv_kf, v);
+        if (pair) {
+          tab_pair<T>(tk, td, tab, a.deriv, qp * inv_kf, w);
+          v[0] = (v[0] + w[0]) * (T)0.5;
+          v[1] = (v[1] + w[1]) * (T)0.5;
+        }
+        const T sc = origin ? (T)0 : (T)a.scale;
+        out[k * a.stride + o] = v[0] * sc;
+        if (a.deriv) out[(a.m + k) * a.stride + o] = v[1] * (inv_kf * sc);
+      }
+    }
+  }
+}
+
 __device__ __forceinline__ double kf_of(double rho) { return 2.0 * cbrt(3.0 * 9.86960440108935861883 * rho); }
 __device__ __forceinline__ float kf_of(float rho) { return 2.0f * cbrtf(29.6088132032680758f * rho); }
 
@@ -226,16 +303,16 @@ __global__ void k_lwt_interval(IntervalArgs a) {
 template <typename T>
 __global__ void k_lwt_final(int64_t n, const T* __restrict__ rho, const T* __restrict__ kfp,
                             const T* __restrict__ rap, const T* __restrict__ pot1, const T* __restrict__ pot2,
-                            const T* __restrict__ pot3, double alpha, double beta, double rhov, double ld, int vcalc,
+                            const T* __restrict__ pot3, double alpha, double beta, double inv_rhov, double ld, int vcalc,
                             int have_pot2, T* __restrict__ pot, double* __restrict__ partial) {
-  const T al = (T)alpha, be = (T)beta, ldT = (T)ld, inv_rhov_ld = (T)(1.0 / pow(rhov, ld));
+  const T al = (T)alpha, be = (T)beta, ldT = (T)ld, inv_rhov_ld = (T)inv_rhov;   // rhov^-ld
   const T third = (T)(1.0 / 3.0);
   T es = (T)0;   // per-thread energy sum in the field precision, FP64 above
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     const T r = rho[i];
     T fac = (T)1;
     if (r < (T)1e-6) {
-      if constexpr (sizeof(T) == 8) fac = pow(fabs(r), ld) / pow(rhov, ld);
+      if constexpr (sizeof(T) == 8) fac = pow(fabs(r), ld) * inv_rhov;
       else fac = pow(fabs(r), ldT) * inv_rhov_ld;
     }
     if (r < (T)0) fac = (T)0;
@@ -285,9 +362,12 @@ __global__ void k_lwt_energy(const double* __restrict__ partial, int nb, double 
   }
 }
 
+constexpr int kMinmaxBlocks = 1216;   // eight CTAs per SM
+
 template <typename T>
 __global__ void k_minmax(int64_t n, const T* __restrict__ x, double* __restrict__ part) {
   T mnT = x[0], mxT = x[0];
+#pragma unroll 4
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     const T v = x[i];
     mnT = v < mnT ? v : mnT;
@@ -414,6 +494,16 @@ __global__ void k_to_float(int64_t n, const double* __restrict__ a, float* __res
     b[i] = (float)a[i];
 }
 
+// K and K' coefficients of a cell side by side
+__global__ void k_interleave(int64_t cells, const double* __restrict__ k, const double* __restrict__ d,
+                             float* __restrict__ out) {
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < 8 * cells; i += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t c = i >> 3;
+    const int e = (int)(i & 7);
+    out[i] = (float)(e < 4 ? k[4 * c + e] : d[4 * c + e - 4]);
+  }
+}
+
 template <typename T>
 BG<T> bg_of(const gbofdft_plan* p) {
   BG<T> b;
@@ -439,61 +529,135 @@ int inv3d(gbofdft_plan* p, void* spec, int64_t fstride, int nf, void* out, int64
   return rc;
 }
 
+// Linear interpolation on the register-blocked passes.  The interval weights are
+// hat functions of k_F, so knots go through in batches that need k_F only: kernel
+// fields K_i and K_i', their products with S formed as the inverse axis-0 pass
+// loads it, the inverse passes with pot1 / pot3 in the epilogue of the rows (p_i
+// and m_i never reach memory), the weights of the batch in the prologue of forward
+// rows, and G (+)= K_i fft(w_i) as the forward axis-0 pass ends.  Bound by HBM for
+// grids beyond L2 (360^3 FP32 evaluation, 12 knots: 21.1 -> 15.6 ms), by the FP64
+// pipe below (64x64x80 FP64: 2.53 -> 1.90 ms).  Returns 1 where a length has no
+// such pass.
 template <typename T>
-int lwt_run(gbofdft_plan* p, const void* rho, gbofdft_lwt* d, void* pot, double* energies, int calc_v, int calc_e,
-            cudaStream_t st) {
-  const int64_t N = p->N;
-  LwtBufs L = lwt_layout(p, d->work);
-  const int nb = blocks_for(N);
-  const T* rhoT = reinterpret_cast<const T*>(rho);
-  // rho extrema -> k_F bounds (guess_kf_bound, lwt.py:36-79)
-  k_minmax<T><<<256, 256, 0, st>>>(N, rhoT, L.part);
-  GB_CHECK_LAUNCH();
-  std::vector<double> mm(512);
-  GB_CUDA(cudaMemcpyAsync(mm.data(), L.part, sizeof(double) * 512, cudaMemcpyDeviceToHost, st));
-  GB_CUDA(cudaStreamSynchronize(st));
-  double rmin = 1e300, rmax = -1e300;
-  for (int b = 0; b < 256; ++b) { rmin = fmin(rmin, mm[2 * b]); rmax = fmax(rmax, mm[2 * b + 1]); }
-  const double kf_l = kf_of_host(rmin), kf_r = kf_of_host(rmax);
-  d->nknots = 0;
-  if (fabs(kf_r - kf_l) < 1e-8) return 0;  // homogeneous density: no contribution
-  double kfmin, kfmax;
-  if (d->kfmin_opt > 0 && d->kfmax_opt > 0) {
-    kfmin = d->kfmin_opt;
-    kfmax = d->kfmax_opt;
-  } else {
-    double kfmin_prev = d->kfmin_state, kfmax_prev = d->kfmax_state;
-    kfmin = d->kfmin_opt > 0 ? d->kfmin_opt : -1.0;
-    kfmax = d->kfmax_opt > 0 ? d->kfmax_opt : -1.0;
-    if (!(kfmin_prev > 0)) { kfmin_prev = 10; if (!(kfmin > 0)) kfmin = kf_l; }
-    if (!(kfmax_prev > 0)) { kfmax_prev = 1.0; if (!(kfmax > 0)) kfmax = kf_r; }
-    if (!(kfmin > 0) || kfmin > kfmin_prev) kfmin = kfmin_prev;
-    if (!(kfmax > 0) || kfmax < kfmax_prev) kfmax = kfmax_prev;
-    if (kfmin > kf_l) {
-      const double kfl[] = {1E-5, 1E-4, 5E-3, 1E-3, 5E-3, 1E-2, 5E-2, 0.1, 0.5, 1.0};
-      const double ratio = kf_l / kfmin;
-      for (int i = 9; i > 0; --i)
-        if (ratio > kfl[i]) { kfmin *= kfl[i]; break; }
-    }
-    if (kfmin < 1e-3) kfmin = 1e-3;
-    if (kfmax < kf_r) kfmax += (nearbyint((kf_r - kfmax) / 0.5) + 1) * 0.5;
-    d->kfmin_state = kfmin;
-    d->kfmax_state = kfmax;
+int lwt_linear(gbofdft_plan* p, const void* rho, const gbofdft_lwt* d, const std::vector<double>& kfl, int kdd,
+               const LwtBufs& L, cudaStream_t st) {
+  const int nsp = (int)kfl.size(), nkf = kdd == 3 ? 2 : 1;
+  const size_t fb = lwt_field_bytes(p), sb = lwt_spec_bytes(p);
+  const size_t tb = r256(gb_elem(p) * (size_t)p->NG);
+  if (!gb_use_ct() || p->rb[0].nst < 2 || p->rb[1].nst == 0 || p->rb[2].nst == 0) return 1;
+  // a batch's spectra and kernel fields lie in the knot work slots and in the
+  // fields that this path does not have (T, U: four spectra; p, m, w, wd)
+  const size_t room[2] = {4 * sb, 8 * fb};
+  char* at[2] = {(char*)L.T, (char*)L.p[0]};
+  int m = GB_LWT_BATCH;
+  void *spec[GB_RB_FIELDS], *ker[GB_RB_FIELDS];
+  for (; m > 0; --m) {
+    size_t used[2] = {0, 0};
+    auto take = [&](size_t bytes) -> void* {
+      for (int r = 0; r < 2; ++r)
+        if (used[r] + bytes <= room[r]) {
+          used[r] += bytes;
+          return at[r] + used[r] - bytes;
+        }
+      return nullptr;
+    };
+    bool fits = true;
+    for (int f = 0; f < nkf * m; ++f) fits = (spec[f] = take(sb)) && fits;
+    if (fits && (ker[0] = take(nkf * m * tb))) break;
   }
-  const int nsp = (int)ceil(log(kfmax / kfmin) / log(d->ratio)) + 1;
-  GB_REQUIRE(nsp >= 2 && nsp <= 4096, "lwt: %d knots from kf range [%g, %g]", nsp, kfmin, kfmax);
-  std::vector<double> kfl(nsp);
-  for (int i = 0; i < nsp; ++i) kfl[i] = kfmin * pow(d->ratio, (double)i);
-  kfl[0] -= 1e-16;
-  kfl[nsp - 1] += 1e-16;
-  d->nknots = nsp;
-  const int kdd = calc_v ? d->kdd : 1;
+  if (m < 1) return 1;
+  const int nbatch = (nsp + m - 1) / m;
+  UTable<T> tk = utab<T>(d, 0, nullptr), td = utab<T>(d, 1, nullptr);
+  const T* tab = nullptr;
+  if constexpr (sizeof(T) == 4) {
+    // the two FP32 table slots are adjacent
+    k_interleave<<<blocks_for(8 * (int64_t)(d->neta - 1)), 256, 0, st>>>(d->neta - 1, d->ktab_c, d->dtab_c, L.ktab_f);
+    GB_CHECK_LAUNCH();
+    tab = L.ktab_f;
+  }
+  const BG<T> bg = bg_of<T>(p);
+  const RowLaunch rl = row_launch(p);
+  const double invN = 0.5 / (double)p->N;   // 1 / N of the inverse transforms, 1/2 of fwd3d
+  int rc = fwd3d(p, rho, L.S, OP_POWB, d->beta, st);
+  for (int b = 0; b < nbatch && !rc; ++b) {
+    const int k0 = (int)((int64_t)nsp * b / nbatch), mb = (int)((int64_t)nsp * (b + 1) / nbatch) - k0;
+    LwtKnots kn;
+    kn.m = mb;
+    kn.below = k0 == 0;
+    kn.kl = kfl[0];
+    kn.kl_e = kfl[0] + 1e-18;
+    kn.inv_kl = 1.0 / kfl[0];
+    for (int e = 0; e <= mb; ++e) {
+      const int l = k0 + e - 1;
+      const bool in = l >= 0 && l + 1 < nsp;
+      kn.lo[e] = in ? kfl[l] : HUGE_VAL;
+      kn.hi[e] = in ? kfl[l + 1] + 1e-18 : HUGE_VAL;
+      kn.inv[e] = in ? 1.0 / (kfl[l + 1] - kfl[l]) : 0.0;
+    }
+    TabArgs ta;
+    ta.m = mb;
+    ta.deriv = nkf == 2;
+    ta.scale = invN;
+    ta.stride = (int64_t)(tb / gb_elem(p));
+    for (int q = 0; q < mb; ++q) ta.inv_kf[q] = 1.0 / kfl[k0 + q];
+    k_lwt_tables<T><<<rl.blocks, rl.threads, 0, st>>>(p->gi, bg, tk, td, tab, ta, reinterpret_cast<T*>(ker[0]));
+    GB_CHECK_LAUNCH();
+    RbLwt c;
+    RbCols ax1;
+    RbLwtRows rows;
+    memset(&c, 0, sizeof(c));
+    memset(&ax1, 0, sizeof(ax1));
+    memset(&rows, 0, sizeof(rows));
+    c.dir = 1;
+    c.nf = nkf * mb;
+    c.in[0] = L.S;
+    c.ld2 = ax1.ld2 = rows.ld2 = p->ld2;
+    for (int f = 0; f < c.nf; ++f) {
+      c.out[f] = spec[f];
+      c.K[f] = reinterpret_cast<T*>(ker[0]) + f * ta.stride;
+      ax1.data[f] = spec[f];
+      rows.in[f] = spec[f];
+    }
+    ax1.axis = 1; ax1.scale = 1.0; ax1.nf = c.nf; ax1.dir = 1;
+    rows.knots = &kn; rows.kf = L.kf;
+    rows.out1 = L.pot1;
+    rows.out3 = kdd == 3 ? L.pot3 : nullptr;
+    rows.first = b == 0;
+    rc = gb_rb_lwt(p, c, st);
+    if (!rc) rc = gb_rb_cols(p, ax1, st);
+    if (!rc) rc = gb_rb_lwt_rows(p, rows, st);
+    if (rc || kdd == 1) continue;
+    rows.out1 = nullptr;
+    rows.ra = L.ra;
+    rows.scale = 2.0;
+    c.dir = -1;
+    c.nf = ax1.nf = mb;
+    c.first = b == 0;
+    c.out[0] = L.G;
+    ax1.dir = -1;
+    for (int f = 0; f < mb; ++f) {
+      rows.out[f] = spec[f];
+      c.in[f] = spec[f];
+    }
+    rc = gb_rb_lwt_rows(p, rows, st);
+    if (!rc) rc = gb_rb_cols(p, ax1, st);
+    if (!rc) rc = gb_rb_lwt(p, c, st);
+  }
+  if (!rc && kdd < 3) GB_CUDA(cudaMemsetAsync(L.pot3, 0, fb, st));
+  return rc;
+}
+
+// One knot at a time with its fields in memory: Hermite interpolation, and
+// lengths without register-blocked passes.
+template <typename T>
+int lwt_knots(gbofdft_plan* p, const void* rho, const gbofdft_lwt* d, const std::vector<double>& kfl, double kfmax,
+              int kdd, const LwtBufs& L, cudaStream_t st) {
+  const int64_t N = p->N;
+  const int nb = blocks_for(N), nsp = (int)kfl.size();
   const int hermite = d->interp == 1;
   const int mcalc = kdd > 1 || hermite;
   const int nkf = mcalc ? 2 : 1;
   if constexpr (sizeof(T) == 4) {
-    GB_REQUIRE(d->neta <= kMaxNetaF32, "lwt: FP32 plans take at most %d table points (neta %d)", kMaxNetaF32,
-               d->neta);
     const int64_t nc = 4 * (int64_t)(d->neta - 1);
     k_to_float<<<blocks_for(nc), 256, 0, st>>>(nc, d->ktab_c, L.ktab_f);
     k_to_float<<<blocks_for(nc), 256, 0, st>>>(nc, d->dtab_c, L.dtab_f);
@@ -501,8 +665,6 @@ int lwt_run(gbofdft_plan* p, const void* rho, gbofdft_lwt* d, void* pot, double*
   }
   const UTable<T> tk = utab<T>(d, 0, L.ktab_f), td = utab<T>(d, 1, L.dtab_f);
   const BG<T> bg = bg_of<T>(p);
-  k_lwt_pre<T><<<nb, 256, 0, st>>>(N, rhoT, kfmax, d->alpha, reinterpret_cast<T*>(L.kf), reinterpret_cast<T*>(L.ra));
-  GB_CHECK_LAUNCH();
   const double invN = 0.5 / (double)N;   // 1 / N of the inverse transforms, 1/2 of fwd3d
   const RowLaunch rl = row_launch(p);
   const size_t fb = lwt_field_bytes(p), sb = lwt_spec_bytes(p);
@@ -555,13 +717,76 @@ int lwt_run(gbofdft_plan* p, const void* rho, gbofdft_lwt* d, void* pot, double*
     cur ^= 1;
   }
   const int last = cur ^ 1;
+  if (kdd > 1) return accumulate(nsp - 1, L.w[last], L.wd[last], 0);
+  return 0;
+}
+
+template <typename T>
+int lwt_run(gbofdft_plan* p, const void* rho, gbofdft_lwt* d, void* pot, double* energies, int calc_v, int calc_e,
+            cudaStream_t st) {
+  const int64_t N = p->N;
+  LwtBufs L = lwt_layout(p, d->work);
+  const int nb = blocks_for(N);
+  const T* rhoT = reinterpret_cast<const T*>(rho);
+  // rho extrema -> k_F bounds (guess_kf_bound, lwt.py:36-79)
+  k_minmax<T><<<kMinmaxBlocks, 256, 0, st>>>(N, rhoT, L.part);
+  GB_CHECK_LAUNCH();
+  std::vector<double> mm(2 * kMinmaxBlocks);
+  GB_CUDA(cudaMemcpyAsync(mm.data(), L.part, sizeof(double) * 2 * kMinmaxBlocks, cudaMemcpyDeviceToHost, st));
+  GB_CUDA(cudaStreamSynchronize(st));
+  double rmin = 1e300, rmax = -1e300;
+  for (int b = 0; b < kMinmaxBlocks; ++b) { rmin = fmin(rmin, mm[2 * b]); rmax = fmax(rmax, mm[2 * b + 1]); }
+  const double kf_l = kf_of_host(rmin), kf_r = kf_of_host(rmax);
+  d->nknots = 0;
+  if (fabs(kf_r - kf_l) < 1e-8) return 0;  // homogeneous density: no contribution
+  double kfmin, kfmax;
+  if (d->kfmin_opt > 0 && d->kfmax_opt > 0) {
+    kfmin = d->kfmin_opt;
+    kfmax = d->kfmax_opt;
+  } else {
+    double kfmin_prev = d->kfmin_state, kfmax_prev = d->kfmax_state;
+    kfmin = d->kfmin_opt > 0 ? d->kfmin_opt : -1.0;
+    kfmax = d->kfmax_opt > 0 ? d->kfmax_opt : -1.0;
+    if (!(kfmin_prev > 0)) { kfmin_prev = 10; if (!(kfmin > 0)) kfmin = kf_l; }
+    if (!(kfmax_prev > 0)) { kfmax_prev = 1.0; if (!(kfmax > 0)) kfmax = kf_r; }
+    if (!(kfmin > 0) || kfmin > kfmin_prev) kfmin = kfmin_prev;
+    if (!(kfmax > 0) || kfmax < kfmax_prev) kfmax = kfmax_prev;
+    if (kfmin > kf_l) {
+      const double kfl[] = {1E-5, 1E-4, 5E-3, 1E-3, 5E-3, 1E-2, 5E-2, 0.1, 0.5, 1.0};
+      const double ratio = kf_l / kfmin;
+      for (int i = 9; i > 0; --i)
+        if (ratio > kfl[i]) { kfmin *= kfl[i]; break; }
+    }
+    if (kfmin < 1e-3) kfmin = 1e-3;
+    if (kfmax < kf_r) kfmax += (nearbyint((kf_r - kfmax) / 0.5) + 1) * 0.5;
+    d->kfmin_state = kfmin;
+    d->kfmax_state = kfmax;
+  }
+  const int nsp = (int)ceil(log(kfmax / kfmin) / log(d->ratio)) + 1;
+  GB_REQUIRE(nsp >= 2 && nsp <= 4096, "lwt: %d knots from kf range [%g, %g]", nsp, kfmin, kfmax);
+  std::vector<double> kfl(nsp);
+  for (int i = 0; i < nsp; ++i) kfl[i] = kfmin * pow(d->ratio, (double)i);
+  kfl[0] -= 1e-16;
+  kfl[nsp - 1] += 1e-16;
+  d->nknots = nsp;
+  const int kdd = calc_v ? d->kdd : 1;
+  const int hermite = d->interp == 1;
+  if constexpr (sizeof(T) == 4) {
+    GB_REQUIRE(d->neta <= kMaxNetaF32, "lwt: FP32 plans take at most %d table points (neta %d)", kMaxNetaF32,
+               d->neta);
+  }
+  k_lwt_pre<T><<<nb, 256, 0, st>>>(N, rhoT, kfmax, d->alpha, reinterpret_cast<T*>(L.kf), reinterpret_cast<T*>(L.ra));
+  GB_CHECK_LAUNCH();
+  int rc = hermite ? 1 : lwt_linear<T>(p, rho, d, kfl, kdd, L, st);
+  if (rc == 1) rc = lwt_knots<T>(p, rho, d, kfl, kfmax, kdd, L, st);
+  if (rc) return rc;
   if (kdd > 1) {
-    if ((rc = accumulate(nsp - 1, L.w[last], L.wd[last], 0))) return rc;
+    const int64_t sfs = (int64_t)(lwt_spec_bytes(p) / (2 * gb_elem(p)));
     if (calc_v && (rc = inv3d(p, L.G, sfs, 1, L.pot2, 0, st))) return rc;
   }
   const double ld = fmax(0.1, d->ldw > 0 ? d->ldw : 1.0 / 6.0);
   k_lwt_final<T><<<nb, 256, 0, st>>>(N, rhoT, (const T*)L.kf, (const T*)L.ra, (const T*)L.pot1, (const T*)L.pot2,
-                                      (const T*)L.pot3, d->alpha, d->beta, rmax, ld, calc_v, kdd > 1,
+                                      (const T*)L.pot3, d->alpha, d->beta, 1.0 / pow(rmax, ld), ld, calc_v, kdd > 1,
                                       reinterpret_cast<T*>(pot), L.part);
   GB_CHECK_LAUNCH();
   if (calc_e && energies) {

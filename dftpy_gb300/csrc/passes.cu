@@ -518,6 +518,8 @@ int gb_rb_rows_inv(gbofdft_plan* p, const RbInv& d, int64_t* nblk, cudaStream_t 
 }
 int gb_rb_cols(gbofdft_plan* p, const RbCols& d, cudaStream_t st) { GB_RB_CALL(gb_rb_cols, d, st); }
 int gb_rb_wgc(gbofdft_plan* p, const RbCols& d, cudaStream_t st) { GB_RB_CALL(gb_rb_wgc, d, st); }
+int gb_rb_lwt(gbofdft_plan* p, const RbLwt& d, cudaStream_t st) { GB_RB_CALL(gb_rb_lwt, d, st); }
+int gb_rb_lwt_rows(gbofdft_plan* p, const RbLwtRows& d, cudaStream_t st) { GB_RB_CALL(gb_rb_lwt_rows, d, st); }
 
 bool gb_rb_wgc_ok(const gbofdft_plan* p) {
   if (!gb_use_ct()) return false;

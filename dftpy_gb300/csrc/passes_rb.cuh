@@ -601,6 +601,31 @@ __device__ __forceinline__ T wgc_point(const RowsInv& a, T rho, T A, T B, T X0, 
   return v;
 }
 
+// inputs i + t nb of a row pair's inverse transform from its two half spectra
+template <int R, typename T>
+__device__ __forceinline__ void inverse_row_inputs(cpx<T>* u, const cpx<T>* pa, int ld2, bool ok0, bool ok1, int i,
+                                                   int nb, int n) {
+#pragma unroll
+  for (int t = 0; t < R; ++t) {
+    const int j = i + t * nb;
+    // j > n/2, and j in {0, n/2}, whose imaginary parts do not count
+    bool up, edge;
+    if constexpr (R % 2 == 0) {
+      up = t > R / 2 || (t == R / 2 && i > 0);
+      edge = t % (R / 2) == 0 && i == 0;
+    } else {
+      up = 2 * j > n;
+      edge = j == 0 || 2 * j == n;
+    }
+    const int k = up ? n - j : j;
+    cpx<T> va = {(T)0, (T)0}, vb = {(T)0, (T)0};
+    if (ok0) va = pa[k];
+    if (ok1) vb = pa[ld2 + k];
+    if (edge) { va.y = (T)0; vb.y = (T)0; }
+    u[t] = up ? cpx<T>{va.x + vb.y, vb.x - va.y} : cpx<T>{va.x - vb.y, va.y + vb.x};
+  }
+}
+
 enum { RI_STORE = 0, RI_EVAL = 1, RI_EVAL_E = 2 };
 
 template <typename T, int MODE, typename AX>
@@ -625,25 +650,7 @@ __global__ void __launch_bounds__(RowCta<T>::NT, (RowCta<T, AX>::MINB)) k_rb_row
       cpx<T> u[R];
       const cpx<T>* pa = reinterpret_cast<const cpx<T>*>(a.in[f]) + (int64_t)ra * a.ld2;
       const bool ok0 = ra < a.nrows, ok1 = ra + 1 < a.nrows;
-#pragma unroll
-      for (int t = 0; t < R; ++t) {
-        const int j = i + t * nb;
-        // j > n/2, and j in {0, n/2}, whose imaginary parts do not count
-        bool up, edge;
-        if constexpr (R % 2 == 0) {
-          up = t > R / 2 || (t == R / 2 && i > 0);
-          edge = t % (R / 2) == 0 && i == 0;
-        } else {
-          up = 2 * j > n;
-          edge = j == 0 || 2 * j == n;
-        }
-        const int k = up ? n - j : j;
-        cpx<T> va = {(T)0, (T)0}, vb = {(T)0, (T)0};
-        if (ok0) va = pa[k];
-        if (ok1) vb = pa[a.ld2 + k];
-        if (edge) { va.y = (T)0; vb.y = (T)0; }
-        u[t] = up ? cpx<T>{va.x + vb.y, vb.x - va.y} : cpx<T>{va.x - vb.y, va.y + vb.x};
-      }
+      inverse_row_inputs<R, T>(u, pa, a.ld2, ok0, ok1, i, nb, n);
       stage_first<1, T>(rc, u, tw, n);
       cpx<T>* dst = A + line * ls;
 #pragma unroll
@@ -880,6 +887,317 @@ template <typename T> struct ColKernel {
     return k;
   }
 };
+
+// ---- LWT --------------------------------------------------------------------------
+// Linear interpolation between the knots k_i of the kernel: a point with k_F in
+// interval e has weight t at the interval's right knot and 1 - t at its left one.
+// The passes take a batch of knots and run through them with the shared memory of
+// one: all knots of a batch at once left four row CTAs (one column CTA) on an SM
+// (360^3 FP32, per knot: inverse rows 363 -> 292 us, forward rows 180 -> 131 us,
+// forward columns 274 -> 128 us).
+struct LwtRows {
+  const void* in[GB_RB_FIELDS];
+  void* out[GB_RB_FIELDS];
+  const void *kf, *ra;
+  void *out1, *out3;
+  int first, m, below;
+  int nrows, n2h, ld2, lp;
+  RbAxis ax;
+  FastDiv dn, dnh;
+  const void* tw;
+  Sc half;
+  Sc lo[GB_LWT_BATCH + 1], hi[GB_LWT_BATCH + 1], inv[GB_LWT_BATCH + 1];
+  Sc kl, kl_e, inv_kl;
+};
+
+// weights of one knot of the batch, without branches (the loads of k_F around them
+// stay in flight together)
+template <typename T> struct LwtWeight {
+  T lo0, hi0, inv0, lo1, hi1, inv1, kl, kl_e, inv_kl;
+  __device__ __forceinline__ LwtWeight(const LwtRows& a, int q) {
+    lo0 = sc<T>(a.lo[q]); hi0 = sc<T>(a.hi[q]); inv0 = sc<T>(a.inv[q]);
+    lo1 = sc<T>(a.lo[q + 1]); hi1 = sc<T>(a.hi[q + 1]); inv1 = sc<T>(a.inv[q + 1]);
+    kl = sc<T>(a.kl); inv_kl = sc<T>(a.inv_kl);
+    kl_e = q == 0 && a.below ? sc<T>(a.kl_e) : -(T)HUGE_VAL;
+  }
+  // low: count the points below the first knot
+  __device__ __forceinline__ T at(T kf, bool low) const {
+    T w = low && kf < kl_e ? (kf - kl) * inv_kl : (T)0;
+    w = kf > lo1 && kf < hi1 ? (T)1 - (kf - lo1) * inv1 : w;
+    return kf > lo0 && kf < hi0 ? (kf - lo0) * inv0 : w;
+  }
+};
+
+// out1 (out3) (+)= sum over the batch of weight x inverse rows of the knot's field
+// (its derivative field).  The transformed fields never reach memory; a point has
+// its interval's two knots only, so the sums are added in memory where the weight is
+// not zero (from the batch's second knot on, in L2).
+template <typename T, typename AX>
+__global__ void __launch_bounds__(RowCta<T>::NT, (RowCta<T, AX>::MINB)) k_rb_lwt_rows_inv(const __grid_constant__ LwtRows a) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const AX ax(a.ax);
+  const int n = ax.n(), lp = a.lp, ls = line_pitch<T>(n), nk = a.out3 ? 2 : 1, nl = nk * lp;
+  cpx<T>* A = reinterpret_cast<cpx<T>*>(smem_raw);
+  cpx<T>* B = A + nl * ls;                               // three or more stages
+  const int tid = threadIdx.x, nthr = blockDim.x;
+  const int base = blockIdx.x * 2 * lp;
+  const cpx<T>* tw = reinterpret_cast<const cpx<T>*>(a.tw);
+  const int nb = ax.nbl(), rl = ax.rl();
+#pragma unroll 1
+  for (int q = 0; q < a.m; ++q) {
+    const LwtWeight<T> wq(a, q);
+    ax.first([&](auto rc) {
+      constexpr int R = decltype(rc)::R;
+      const int nbf = ax.nbf();
+      for (int t0 = tid; t0 < nl * nbf; t0 += nthr) {
+        const int line = ax.div_nbf(t0), i = t0 - line * nbf;
+        const int f = line >= lp, l = line - f * lp;
+        const int ra = base + 2 * l;
+        cpx<T> u[R];
+        const cpx<T>* pa = reinterpret_cast<const cpx<T>*>(a.in[q + f * a.m]) + (int64_t)ra * a.ld2;
+        inverse_row_inputs<R, T>(u, pa, a.ld2, ra < a.nrows, ra + 1 < a.nrows, i, nbf, n);
+        stage_first<1, T>(rc, u, tw, n);
+        cpx<T>* dst = A + line * ls;
+#pragma unroll
+        for (int t = 0; t < R; ++t) dst[sidx<T>(i * R + t)] = u[t];
+      }
+    });
+    __syncthreads();
+    cpx<T>* cur = A;
+    cpx<T>* oth = B;
+    ax.middle([&](auto rc, auto nbm, auto p, auto div_nb, auto div_p) {
+      constexpr int R = decltype(rc)::R;
+      for (int t0 = tid; t0 < nl * nbm; t0 += nthr) {
+        const int line = div_nb(t0), i = t0 - line * nbm;
+        const int k = i - p * div_p(i);
+        cpx<T> u[R];
+        load_stage<1, T>(rc, u, cur + line * ls, tw, i, k, nbm, p, n, sidx<T>);
+        cpx<T>* dst = oth + line * ls;
+        const int j0 = (i - k) * R + k;
+#pragma unroll
+        for (int t = 0; t < R; ++t) dst[sidx<T>(j0 + t * p)] = u[t];
+      }
+      __syncthreads();
+      cpx<T>* x = cur;
+      cur = oth;
+      oth = x;
+    });
+    for (int t0 = tid; t0 < lp * nb; t0 += nthr) {
+      const int l = ax.div_nbl(t0), i = t0 - l * nb;
+      const int ra = base + 2 * l;
+      if (ra >= a.nrows) continue;
+      const bool ok1 = ra + 1 < a.nrows;
+      const T* kp = reinterpret_cast<const T*>(a.kf) + (int64_t)ra * n + i;
+      const int second = ok1 ? n : 0;
+      const bool store = a.first && q == 0;
+      // C points t, t + 1, .. of field f: every load before the first store
+      auto add = [&](auto cc, int t, int f, auto&& z) {
+        constexpr int C = decltype(cc)::value;
+        T* o = reinterpret_cast<T*>(f ? a.out3 : a.out1) + (int64_t)ra * n + i;
+        T w0[C], w1[C], s0[C], s1[C];
+#pragma unroll
+        for (int c = 0; c < C; ++c) {
+          // below the knots there is no derivative term
+          w0[c] = wq.at(__ldg(kp + (t + c) * nb), f == 0);
+          w1[c] = wq.at(__ldg(kp + (t + c) * nb + second), f == 0);
+        }
+#pragma unroll
+        for (int c = 0; c < C; ++c) {
+          s0[c] = !store && w0[c] != (T)0 ? o[(t + c) * nb] : (T)0;
+          s1[c] = !store && w1[c] != (T)0 ? o[(t + c) * nb + second] : (T)0;
+        }
+#pragma unroll
+        for (int c = 0; c < C; ++c) {
+          const cpx<T> v = z(t + c);
+          if (store || w0[c] != (T)0) o[(t + c) * nb] = s0[c] + w0[c] * v.x;
+          if (ok1 && (store || w1[c] != (T)0)) o[(t + c) * nb + n] = s1[c] + w1[c] * v.y;
+        }
+      };
+      if (ax.nst() > 1) {
+        ax.last([&](auto rc) {
+          constexpr int R = decltype(rc)::R;
+          // 4 or so: 360^3 FP32, three knots 877 us, 904 with 2 (registers for 7 CTAs;
+          // without spills, at 5 CTAs, 1026)
+          constexpr int C = R % 4 == 0 ? 4 : R % 3 == 0 ? 3 : R % 5 == 0 ? 5 : R % 7 == 0 ? 7 : 2;
+          for (int f = 0; f < nk; ++f) {
+            cpx<T> u[R];
+            load_stage<1, T>(rc, u, cur + (f * lp + l) * ls, tw, i, i, nb, nb, n, sidx<T>);
+#pragma unroll
+            for (int t = 0; t < R; t += C) add(std::integral_constant<int, C>{}, t, f, [&](int k) { return u[k]; });
+          }
+        });
+      } else {
+        for (int f = 0; f < nk; ++f)
+          for (int t = 0; t < rl; ++t)
+            add(std::integral_constant<int, 1>{}, t, f,
+                [&](int k) { return cur[(f * lp + l) * ls + sidx<T>(i + k * nb)]; });
+      }
+    }
+    __syncthreads();                                     // the next knot overwrites the buffers
+  }
+}
+
+// spectra along axis 2 of weight x ra for every knot of the batch
+template <typename T, typename AX>
+__global__ void __launch_bounds__(RowCta<T>::NT, (RowCta<T, AX>::MINB)) k_rb_lwt_rows_fwd(const __grid_constant__ LwtRows a) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const AX ax(a.ax);
+  const int n = ax.n(), lp = a.lp, ls = line_pitch<T>(n);
+  cpx<T>* A = reinterpret_cast<cpx<T>*>(smem_raw);
+  cpx<T>* B = ax.nst() > 2 ? A + lp * ls : A;
+  const int tid = threadIdx.x, nthr = blockDim.x;
+  const int base = blockIdx.x * 2 * lp;
+  const cpx<T>* tw = reinterpret_cast<const cpx<T>*>(a.tw);
+  const T* kf = reinterpret_cast<const T*>(a.kf);
+  const T* fac = reinterpret_cast<const T*>(a.ra);
+  const int nh = AX::kFixed ? n / 2 + 1 : a.n2h;
+#pragma unroll 1
+  for (int q = 0; q < a.m; ++q) {
+    const LwtWeight<T> wq(a, q);
+    ax.first([&](auto rc) {
+      constexpr int R = decltype(rc)::R;
+      const int nb = ax.nbf();
+      for (int t0 = tid; t0 < lp * nb; t0 += nthr) {
+        const int l = ax.div_nbf(t0), i = t0 - l * nb;
+        const int ra = base + 2 * l;
+        const bool ok0 = ra < a.nrows, ok1 = ra + 1 < a.nrows;
+        const int64_t off = (int64_t)ra * n + i;
+        cpx<T> u[R];
+#pragma unroll
+        for (int t = 0; t < R; ++t) u[t] = cpx<T>{ok0 ? __ldg(kf + off + t * nb) : (T)0, ok1 ? __ldg(kf + off + n + t * nb) : (T)0};
+#pragma unroll
+        for (int t = 0; t < R; ++t) {
+          const T w0 = ok0 ? wq.at(u[t].x, true) : (T)0, w1 = ok1 ? wq.at(u[t].y, true) : (T)0;
+          u[t].x = w0 != (T)0 ? w0 * __ldg(fac + off + t * nb) : (T)0;
+          u[t].y = w1 != (T)0 ? w1 * __ldg(fac + off + n + t * nb) : (T)0;
+        }
+        stage_first<-1, T>(rc, u, tw, n);
+        cpx<T>* dst = B + l * ls;
+#pragma unroll
+        for (int t = 0; t < R; ++t) dst[sidx<T>(i * R + t)] = u[t];
+      }
+    });
+    const cpx<T>* res = lines<-1, false, T>(A, B, ls, lp, ax, tw);
+    const T half = sc<T>(a.half);
+    cpx<T>* o = reinterpret_cast<cpx<T>*>(a.out[q]);
+    for (int idx = tid; idx < lp * nh; idx += nthr) {
+      const int l = AX::kFixed ? idx / nh : (int)a.dnh.div(idx), k = idx - l * nh;
+      const int ra = base + 2 * l;
+      if (ra >= a.nrows) continue;
+      const cpx<T> Z = res[l * ls + sidx<T>(k)];
+      const cpx<T> Zc = res[l * ls + sidx<T>(k == 0 ? 0 : n - k)];
+      cpx<T>* w = o + (int64_t)ra * a.ld2 + k;
+      w[0] = c_scale(cpx<T>{Z.x + Zc.x, Z.y - Zc.y}, half);
+      if (ra + 1 < a.nrows) w[a.ld2] = c_scale(cpx<T>{Z.y + Zc.y, Zc.x - Z.x}, half);
+    }
+    __syncthreads();                                     // the next knot overwrites the buffers
+  }
+}
+
+// Columns along axis 0.  Inverse: field f = ifft(K_f S), the product formed as the
+// pass loads S (the fields of one column tile are neighbouring CTAs: the tile
+// comes from HBM once).  Forward: out (+)= sum_f K_f fft(in_f), added through L2 as
+// each field's last stage ends.
+struct LwtCols {
+  const void* in[GB_RB_FIELDS];
+  void* out[GB_RB_FIELDS];
+  const void* K[GB_RB_FIELDS];
+  int64_t stride, ostride, kst;
+  unsigned ncol;
+  int n2h, nf, first;
+  FastDiv dld;
+  RbAxis ax;
+  const void* tw;
+};
+
+// columns of a tile.  The sums read and write memory field after field: half the
+// tile, and twice the CTAs on an SM, for three-stage lines (360^3 FP32, three
+// fields: 466 -> 385 us; the inverse pass 549 -> 573 us, so it keeps the whole one)
+template <typename T, int DIR, typename AX> constexpr int lwt_tb() {
+  if constexpr (sizeof(T) == 4 && AX::kFixed && DIR < 0) return AX::nst() > 2 ? 8 : ColTile<T>::TB;
+  else return ColTile<T>::TB;
+}
+
+template <typename T, int DIR, typename AX>
+__global__ void __launch_bounds__(sizeof(T) == 4 ? 400 : 256) k_rb_lwt(const __grid_constant__ LwtCols a) {
+  constexpr int TB = lwt_tb<T, DIR, AX>();
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const AX ax(a.ax);
+  const int n = ax.n();
+  cpx<T>* A = reinterpret_cast<cpx<T>*>(smem_raw);
+  const int c = threadIdx.x % TB, i0 = threadIdx.x / TB, ni = blockDim.x / TB;
+  const unsigned tile = DIR > 0 ? blockIdx.x / a.nf : blockIdx.x;
+  const unsigned col = tile * TB + c;
+  const int outer = a.dld.div(col), k2 = col - outer * a.dld.d;
+  const bool ok = col < a.ncol && k2 < a.n2h;
+  const int64_t off = outer * a.ostride + k2, koff = (int64_t)outer * a.n2h + k2;
+  const cpx<T>* tw = reinterpret_cast<const cpx<T>*>(a.tw);
+  const int64_t st = a.stride, kst = a.kst;
+  auto sx = [&](int j) { return j * TB + c; };
+  const int f_lo = DIR > 0 ? blockIdx.x - tile * a.nf : 0, f_hi = DIR > 0 ? f_lo + 1 : a.nf;
+#pragma unroll 1
+  for (int f = f_lo; f < f_hi; ++f) {
+    const cpx<T>* g = reinterpret_cast<const cpx<T>*>(a.in[DIR > 0 ? 0 : f]) + off;
+    const T* K = reinterpret_cast<const T*>(a.K[f]) + koff;
+    ax.first([&](auto rc) {
+      constexpr int R = decltype(rc)::R;
+      const int nb = ax.nbf();
+      for (int i = i0; i < nb; i += ni) {
+        cpx<T> u[R];
+#pragma unroll
+        for (int t = 0; t < R; ++t) {
+          const int j = i + t * nb;
+          u[t] = ok ? g[j * st] : cpx<T>{(T)0, (T)0};
+          if (DIR > 0) u[t] = c_scale(u[t], ok ? __ldg(K + j * kst) : (T)0);
+        }
+        stage_first<DIR, T>(rc, u, tw, n);
+#pragma unroll
+        for (int t = 0; t < R; ++t) A[sx(i * R + t)] = u[t];
+      }
+    });
+    __syncthreads();
+    cpx<T>* cur = A;
+    cpx<T>* oth = A + n * TB;
+    ax.middle([&](auto rc, auto nb, auto p, auto, auto div_p) {
+      constexpr int R = decltype(rc)::R;
+      for (int i = i0; i < nb; i += ni) {
+        const int k = i - p * div_p(i);
+        cpx<T> u[R];
+        load_stage<DIR, T>(rc, u, cur, tw, i, k, nb, p, n, sx);
+        const int j0 = (i - k) * R + k;
+#pragma unroll
+        for (int t = 0; t < R; ++t) oth[sx(j0 + t * p)] = u[t];
+      }
+      __syncthreads();
+      cpx<T>* y = cur;
+      cur = oth;
+      oth = y;
+    });
+    cpx<T>* o = reinterpret_cast<cpx<T>*>(a.out[DIR > 0 ? f : 0]) + off;
+    ax.last([&](auto rc) {
+      constexpr int R = decltype(rc)::R;
+      const int nb = ax.nbl();
+      for (int i = i0; i < nb; i += ni) {
+        cpx<T> u[R];
+        load_stage<DIR, T>(rc, u, cur, tw, i, i, nb, nb, n, sx);
+        if (!ok) continue;
+#pragma unroll
+        for (int t = 0; t < R; ++t) {
+          const int j = i + t * nb;
+          if (DIR < 0) {
+            u[t] = c_scale(u[t], __ldg(K + j * kst));
+            if (f > 0 || !a.first) {
+              const cpx<T> s = o[j * st];
+              u[t] = cpx<T>{s.x + u[t].x, s.y + u[t].y};
+            }
+          }
+          o[j * st] = u[t];
+        }
+      }
+    });
+    if (DIR < 0) __syncthreads();                        // the next field overwrites the buffers
+  }
+}
 
 template <typename T, int DIR, bool CONV, typename AX, typename AXI>
 __global__ void __launch_bounds__(sizeof(T) == 4 ? 400 : 256) k_rb_cols(const __grid_constant__ Cols a) {
@@ -1380,6 +1698,102 @@ static int rows_inv(gbofdft_plan* p, const RbInv& d, int64_t* nblk_out, cudaStre
   });
 }
 
+// Butterflies of a column side by side.  FP64: one per thread of the stage with
+// the most (idle warps cost nothing on the FP64 pipe).  FP32: as many as keep
+// the threads of every stage busy, the last stage weighed with wl.
+template <typename T> inline int column_threads(const AxisInfo& x, int cap, double wl) {
+  const int rounds = (x.nbmax + cap - 1) / cap;
+  int ni = (x.nbmax + rounds - 1) / rounds;
+  if (sizeof(T) == 4) {
+    double best = -1.0;
+    for (int c = x.nbl < x.nbf ? x.nbl : x.nbf; c <= x.nbmax && c <= cap; ++c) {
+      auto busy = [&](int nb) { return nb / (double)((nb + c - 1) / c * c); };
+      const double r = busy(x.nbf) + wl * busy(x.nbl) + 1e-3 * c;
+      if (r > best) {
+        best = r;
+        ni = c;
+      }
+    }
+  }
+  return ni;
+}
+
+// LWT columns along axis 0
+template <typename T>
+static int lwt_cols(gbofdft_plan* p, const RbLwt& d, cudaStream_t st) {
+  LwtCols a;
+  memset(&a, 0, sizeof(a));
+  a.ax = p->rb[0];
+  if (a.ax.nst < 2) return 1;
+  for (int f = 0; f < d.nf; ++f) {
+    a.in[f] = d.in[f];
+    a.out[f] = d.out[f];
+    a.K[f] = d.K[f];
+  }
+  a.stride = (int64_t)p->n[1] * d.ld2;
+  a.kst = (int64_t)p->n[1] * p->n2h;
+  a.ostride = d.ld2;
+  a.ncol = (unsigned)p->n[1] * d.ld2; a.n2h = p->n2h; a.nf = d.nf; a.first = d.first;
+  a.dld.set(d.ld2);
+  a.tw = p->tw[0];
+  return by_axis<T>(a.ax, [&](auto x) {
+    using AX = typename decltype(x)::ax;
+    const AxisInfo xi = axis_info<AX>(a.ax);
+    auto go = [&](auto kern, auto tb, unsigned nf) -> int {
+      constexpr int TB = decltype(tb)::value;
+      const size_t sm = (xi.nst > 2 ? 2 : 1) * sizeof(cpx<T>) * (size_t)TB * xi.n;
+      if (sm > kMaxSmem) return 1;
+      if (int rc = gbct::ct_smem(kern, sm)) return rc;
+      const int threads = TB * column_threads<T>(xi, (sizeof(T) == 4 ? 400 : 256) / TB, 1.0);
+      kern<<<(a.ncol + TB - 1) / TB * nf, threads, sm, st>>>(a);
+      return launch_check<T>("rb_lwt");
+    };
+    if (d.dir > 0) return go(k_rb_lwt<T, 1, AX>, std::integral_constant<int, lwt_tb<T, 1, AX>()>{}, d.nf);
+    return go(k_rb_lwt<T, -1, AX>, std::integral_constant<int, lwt_tb<T, -1, AX>()>{}, 1);
+  });
+}
+
+// LWT rows: inverse (d.out1) or forward
+template <typename T>
+static int lwt_rows(gbofdft_plan* p, const RbLwtRows& d, cudaStream_t st) {
+  LwtRows a;
+  memset(&a, 0, sizeof(a));
+  a.ax = p->rb[2];
+  if (a.ax.nst == 0) return 1;
+  const LwtKnots& k = *d.knots;
+  const int inverse = d.out1 != nullptr, nk = inverse && d.out3 ? 2 : 1;
+  for (int f = 0; f < (inverse ? nk : 0) * k.m; ++f) a.in[f] = d.in[f];
+  for (int f = 0; f < (inverse ? 0 : k.m); ++f) a.out[f] = d.out[f];
+  a.kf = d.kf; a.ra = d.ra; a.out1 = d.out1; a.out3 = d.out3; a.first = d.first;
+  a.m = k.m; a.below = k.below;
+  a.nrows = p->n[0] * p->n[1]; a.n2h = p->n2h; a.ld2 = d.ld2;
+  a.dn.set(p->n[2]);
+  a.dnh.set(p->n2h);
+  a.tw = p->tw[2];
+  a.half.set(0.5 * d.scale);
+  for (int e = 0; e <= k.m; ++e) {
+    a.lo[e].set(k.lo[e]);
+    a.hi[e].set(k.hi[e]);
+    a.inv[e].set(k.inv[e]);
+  }
+  a.kl.set(k.kl); a.kl_e.set(k.kl_e); a.inv_kl.set(k.inv_kl);
+  auto go = [&](auto kern, const AxisInfo& x) -> int {
+    const int nbuf = x.nst > 2 ? 2 : 1;
+    const RowShape sh = row_shape<T>(x, nk, nbuf, a.nrows);
+    a.lp = sh.lp;
+    const size_t sm = nbuf * sizeof(cpx<T>) * (size_t)nk * a.lp * line_pitch<T>(x.n);
+    if (sm > kMaxSmem) return 1;
+    if (int rc = gbct::ct_smem(kern, sm)) return rc;
+    kern<<<(a.nrows + 2 * a.lp - 1) / (2 * a.lp), sh.threads, sm, st>>>(a);
+    return launch_check<T>("rb_lwt_rows");
+  };
+  return by_axis<T>(a.ax, [&](auto x) {
+    using P = decltype(x);
+    if (inverse) return go(k_rb_lwt_rows_inv<T, inverse_order<P>>, axis_info<inverse_order<P>>(a.ax));
+    return go(k_rb_lwt_rows_fwd<T, typename P::ax>, axis_info<typename P::ax>(a.ax));
+  });
+}
+
 // WGC: the WGC kernel on groups of three fields, else plain columns or (kd) the convolution
 template <typename T, bool WGC>
 static int cols(gbofdft_plan* p, const RbCols& d, cudaStream_t st) {
@@ -1409,29 +1823,14 @@ static int cols(gbofdft_plan* p, const RbCols& d, cudaStream_t st) {
   constexpr int TB = ColTile<T>::TB;
   const dim3 grid((a.ncol + TB - 1) / TB, WGC ? nf / 3 : nf);
   auto go = [&](auto kern, const AxisInfo& x) -> int {
-    // butterflies of a column side by side.  FP64: one per thread of the stage
-    // with the most (idle warps cost nothing on the FP64 pipe).  FP32: as many
-    // as keep the threads of every stage busy (the last stage counts twice in
-    // the convolution, which continues with the inverse's first).
     auto smem = [&](int fy) {
       const int nbuf = WGC ? 3 + fy * (x.nst > 2 ? 2 : 1) : x.nst < 2 ? 0 : (kd || x.nst > 2 ? 2 : 1);
       return nbuf * sizeof(cpx<T>) * (size_t)TB * x.n;
     };
     const int fy = WGC && sizeof(T) == 4 && smem(3) <= kMaxSmem ? 3 : 1;
     const int cap = WGC ? kWgcThreads<T> / (TB * fy) : (sizeof(T) == 4 ? 400 : 256) / TB;
-    const int rounds = (x.nbmax + cap - 1) / cap;
-    int ni = (x.nbmax + rounds - 1) / rounds;
-    if (sizeof(T) == 4) {
-      double best = -1.0;
-      for (int c = x.nbl < x.nbf ? x.nbl : x.nbf; c <= x.nbmax && c <= cap; ++c) {
-        auto busy = [&](int nb) { return nb / (double)((nb + c - 1) / c * c); };
-        const double r = busy(x.nbf) + (kd || WGC ? 2.0 : 1.0) * busy(x.nbl) + 1e-3 * c;
-        if (r > best) {
-          best = r;
-          ni = c;
-        }
-      }
-    }
+    // the last stage of the convolution continues with the inverse's first
+    const int ni = column_threads<T>(x, cap, kd || WGC ? 2.0 : 1.0);
     const size_t sm = smem(fy);
     if (sm > kMaxSmem) return 1;
     if (int rc = gbct::ct_smem(kern, sm)) return rc;
@@ -1472,4 +1871,11 @@ static int cols(gbofdft_plan* p, const RbCols& d, cudaStream_t st) {
 #define GB_RB_DEFINE_WGC(T, SUF)                                                                                \
   int GB_RB_NAME(gb_rb_wgc, SUF)(gbofdft_plan* p, const RbCols& d, cudaStream_t st) {                          \
     return gbrb::cols<T, true>(p, d, st);                                                                      \
+  }
+#define GB_RB_DEFINE_LWT(T, SUF)                                                                                \
+  int GB_RB_NAME(gb_rb_lwt, SUF)(gbofdft_plan* p, const RbLwt& d, cudaStream_t st) {                           \
+    return gbrb::lwt_cols<T>(p, d, st);                                                                        \
+  }                                                                                                             \
+  int GB_RB_NAME(gb_rb_lwt_rows, SUF)(gbofdft_plan* p, const RbLwtRows& d, cudaStream_t st) {                  \
+    return gbrb::lwt_rows<T>(p, d, st);                                                                        \
   }

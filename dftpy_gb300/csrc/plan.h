@@ -91,6 +91,35 @@ int gb_cols_conv(gbofdft_plan* p, void* spec, int64_t fstride, int ld2, int nf, 
 // register-blocked passes (passes_rb_*.cu): return 1 when the axis length has a
 // prime factor above 7 or its lines do not fit, 0 on success, an error code otherwise
 #define GB_RB_FIELDS 10   // fused terms (GB_MAX_FIELDS - 1) and the six fields of the WGC term
+#define GB_LWT_BATCH 4     // knots of one launch, at most
+// The knot intervals of the knots k0 .. k0 + m - 1 of a LWT batch: interval e
+// (lo, hi) lies left of knot k0 + e; lo = HUGE_VAL: none there.  below: k0 is the
+// first knot, and its weight also holds (kf - kl) / kl at kf < kl_e.
+struct LwtKnots {
+  int m, below;
+  double lo[GB_LWT_BATCH + 1], hi[GB_LWT_BATCH + 1], inv[GB_LWT_BATCH + 1];
+  double kl, kl_e, inv_kl;
+};
+struct RbLwt {            // LWT columns along axis 0
+  const void* in[GB_RB_FIELDS];   // inverse: in[0] = S for every field; accumulation: field f
+  void* out[GB_RB_FIELDS];        // inverse: field f; accumulation: out[0] (+)= sum_f K_f in[f]
+  const void* K[GB_RB_FIELDS];    // kernel fields [n0][n1][n2h]
+  int nf, ld2, dir, first;
+};
+struct RbLwtRows {        // LWT rows of a batch of knots
+  const LwtKnots* knots;
+  const void* kf;         // k_F
+  int ld2;
+  // inverse: spectra p_i (0 .. m - 1) and, with out3, those of the derivative kernels (m .. 2 m - 1):
+  // out1, out3 (+)= weights x fields
+  const void* in[GB_RB_FIELDS];
+  void *out1, *out3;
+  int first;
+  // forward: spectra of the weights times ra, scaled by scale
+  const void* ra;
+  void* out[GB_RB_FIELDS];
+  double scale;
+};
 struct RbFwd {            // forward rows: fields derived from in[0] (OP_RHO alone: in[f]) to spectra out[f]
   const void* in[GB_RB_FIELDS];
   void* out[GB_RB_FIELDS];
@@ -130,7 +159,9 @@ struct RbCols {           // columns of nf spectra: dir, the convolution (kd) or
   int gb_rb_rows_fwd_##SUF(gbofdft_plan*, const RbFwd&, cudaStream_t);                    \
   int gb_rb_rows_inv_##SUF(gbofdft_plan*, const RbInv&, int64_t* nblk, cudaStream_t);     \
   int gb_rb_cols_##SUF(gbofdft_plan*, const RbCols&, cudaStream_t);                       \
-  int gb_rb_wgc_##SUF(gbofdft_plan*, const RbCols&, cudaStream_t);
+  int gb_rb_wgc_##SUF(gbofdft_plan*, const RbCols&, cudaStream_t);                        \
+  int gb_rb_lwt_##SUF(gbofdft_plan*, const RbLwt&, cudaStream_t);                         \
+  int gb_rb_lwt_rows_##SUF(gbofdft_plan*, const RbLwtRows&, cudaStream_t);
 GB_RB_DECLARE(f64_g0)
 GB_RB_DECLARE(f32_g0)
 GB_RB_DECLARE(f32_g1)
@@ -142,6 +173,8 @@ int gb_rb_rows_fwd(gbofdft_plan*, const RbFwd&, cudaStream_t);
 int gb_rb_rows_inv(gbofdft_plan*, const RbInv&, int64_t* nblk, cudaStream_t);
 int gb_rb_cols(gbofdft_plan*, const RbCols&, cudaStream_t);
 int gb_rb_wgc(gbofdft_plan*, const RbCols&, cudaStream_t);
+int gb_rb_lwt(gbofdft_plan*, const RbLwt&, cudaStream_t);
+int gb_rb_lwt_rows(gbofdft_plan*, const RbLwtRows&, cudaStream_t);
 // every axis has register-blocked passes, the WGC columns included
 bool gb_rb_wgc_ok(const gbofdft_plan* p);
 void gb_rb_plan(gbofdft_plan* p);   // the plan's rb / rbi from its lengths and precision
