@@ -33,6 +33,7 @@ template <typename T>
 __global__ void k_force_field(GInfo g, int mode, const cpx<T>* __restrict__ in, const double2* __restrict__ bm0,
                               const double2* __restrict__ bm1, const double2* __restrict__ bm2, gbofdft_vtable vt,
                               double eta, cpx<T>* __restrict__ out) {
+  const double ie = -1.0 / (4.0 * eta);                  // mode 1
   const int64_t total = (int64_t)g.n0 * g.n1 * g.n2h;
   for (int64_t id = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; id < total;
        id += (int64_t)gridDim.x * blockDim.x) {
@@ -42,12 +43,12 @@ __global__ void k_force_field(GInfo g, int mode, const cpx<T>* __restrict__ in, 
     const double2 b = bprod(bm0, bm1, bm2, i0, i1, k2);
     const cpx<T> v = in[id];
     if (mode == 0) {
-      const double kv = gbk::sym_kernel<double>(g, i0, i1, k2, [&](double gg) { return vline_eval(vt, sqrt(gg)); });
+      const double kv = gbk::sym_kernel<double>(g, i0, i1, k2, [&](double gg) { return vline_eval(vt, sqrt_nr(gg)); });
       out[id] = cpx<T>{(T)(((double)v.x * b.x + (double)v.y * b.y) * kv),
                        (T)(((double)v.y * b.x - (double)v.x * b.y) * kv)};
     } else {
       const double kv = gbk::sym_kernel<double>(
-          g, i0, i1, k2, [&](double gg) { return gg > 0.0 ? exp(-gg / (4.0 * eta)) / gg : 0.0; });
+          g, i0, i1, k2, [&](double gg) { return gg > 0.0 ? exp(gg * ie) * rcp_nr(gg) : 0.0; });
       const double bb = (b.x * b.x + b.y * b.y) * kv;
       out[id] = cpx<T>{(T)((double)v.x * bb), (T)((double)v.y * bb)};
     }
@@ -120,9 +121,12 @@ __global__ void k_ewald_real_forces(const double* __restrict__ pos, const double
   const double xi = pos[3 * i], yi = pos[3 * i + 1], zi = pos[3 * i + 2];
   const double c2 = 2.0 / sqrt(3.14159265358979323846);
   double f0 = 0.0, f1 = 0.0, f2 = 0.0;
-  const int64_t tot = (int64_t)nimg * nat;
-  for (int64_t t = threadIdx.x; t < tot; t += blockDim.x) {
-    const int im = (int)(t / nat), j = (int)(t % nat);
+  int im = 0, j = threadIdx.x;
+  for (;; j += blockDim.x) {
+    while (j >= nat) { j -= nat; ++im; }
+    if (im >= nimg) break;
+    if (ewald_far((float)xi, (float)yi, (float)zi, (float)pos[3 * j], (float)pos[3 * j + 1], (float)pos[3 * j + 2],
+                  (float)img[3 * im], (float)img[3 * im + 1], (float)img[3 * im + 2], (float)rmax)) continue;
     const double dx = xi - (pos[3 * j] - img[3 * im]);
     const double dy = yi - (pos[3 * j + 1] - img[3 * im + 1]);
     const double dz = zi - (pos[3 * j + 2] - img[3 * im + 2]);

@@ -28,10 +28,10 @@ __global__ void k_pme_vloc_acc(GInfo g, gbofdft_vtable vt, const cpx<T>* __restr
     int i0, i1, k2;
     decode(g, id, i0, i1, k2);
     const int m0 = ffreq(i0, g.n0), m1 = ffreq(i1, g.n1);
-    double vl = vline_eval(vt, sqrt(gg_at(g, m0, m1, m2_of(g, k2))));
+    double vl = vline_eval(vt, sqrt_nr(gg_at(g, m0, m1, m2_of(g, k2))));
     if (needs_sym(g, i0, i1, k2)) {
       const int p0 = ffreq((g.n0 - i0) % g.n0, g.n0), p1 = ffreq((g.n1 - i1) % g.n1, g.n1);
-      vl = 0.5 * (vl + vline_eval(vt, sqrt(gg_at(g, p0, p1, m2_partner(g, k2)))));
+      vl = 0.5 * (vl + vline_eval(vt, sqrt_nr(gg_at(g, p0, p1, m2_partner(g, k2)))));
     }
     const double2 b = bprod(bm0, bm1, bm2, i0, i1, k2);
     const cpx<T> q = fq[id];
@@ -95,9 +95,12 @@ __global__ void k_ewald_real(const double* __restrict__ pos, const double* __res
   KSum s;
   s.init();
   const double xi = pos[3 * i], yi = pos[3 * i + 1], zi = pos[3 * i + 2];
-  const int64_t tot = (int64_t)nimg * nat;
-  for (int64_t t = threadIdx.x; t < tot; t += blockDim.x) {
-    const int im = (int)(t / nat), j = (int)(t % nat);
+  int im = 0, j = threadIdx.x;
+  for (;; j += blockDim.x) {
+    while (j >= nat) { j -= nat; ++im; }
+    if (im >= nimg) break;
+    if (ewald_far((float)xi, (float)yi, (float)zi, (float)pos[3 * j], (float)pos[3 * j + 1], (float)pos[3 * j + 2],
+                  (float)img[3 * im], (float)img[3 * im + 1], (float)img[3 * im + 2], (float)rmax)) continue;
     const double dx = xi - (pos[3 * j] - img[3 * im]);
     const double dy = yi - (pos[3 * j + 1] - img[3 * im + 1]);
     const double dz = zi - (pos[3 * j + 2] - img[3 * im + 2]);
@@ -137,6 +140,7 @@ __global__ void __launch_bounds__(256) k_ewald_rec_pme(GInfo g, const cpx<T>* __
                                                        const double2* __restrict__ bm2, double eta,
                                                        double* __restrict__ partial) {
   const int64_t total = (int64_t)g.n0 * g.n1 * g.n2h;
+  const double ie = -1.0 / (4.0 * eta);
   KSum s;
   s.init();
   for (int64_t id = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; id < total;
@@ -149,7 +153,7 @@ __global__ void __launch_bounds__(256) k_ewald_rec_pme(GInfo g, const cpx<T>* __
     const double2 b0 = bm0[i0], b1 = bm1[i1], b2 = bm2[k2];
     const double bb = (b0.x * b0.x + b0.y * b0.y) * (b1.x * b1.x + b1.y * b1.y) * (b2.x * b2.x + b2.y * b2.y);
     const cpx<T> q = fq[id];
-    s.add(((double)q.x * q.x + (double)q.y * q.y) * bb * exp(-gg / (4.0 * eta)) / gg);
+    s.add(((double)q.x * q.x + (double)q.y * q.y) * bb * exp(gg * ie) * rcp_nr(gg));
   }
   block_partial<256>(s, partial);
 }
