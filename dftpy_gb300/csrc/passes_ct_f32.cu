@@ -1,5 +1,4 @@
-// FP32 instantiations of the compile-time-size passes.
+// The FP32 plane pipeline: row passes of compile-time length, plane convolution.
 #include "passes_ct.cuh"
 
-GB_CT_DEFINE(float, f32)
 GB_CT_DEFINE_PLANE()

@@ -178,44 +178,20 @@ int gb_rb_lwt_rows(gbofdft_plan*, const RbLwtRows&, cudaStream_t);
 // every axis has register-blocked passes, the WGC columns included
 bool gb_rb_wgc_ok(const gbofdft_plan* p);
 void gb_rb_plan(gbofdft_plan* p);   // the plan's rb / rbi from its lengths and precision
-// compile-time-size passes (passes_ct_*.cu): return 1 when the size has no
+// plane-major FP32 pipeline (passes_ct_f32.cu): return 1 when the size has no
 // specialisation, 0 on success, an error code otherwise
-int gb_ct_rows_fwd_f32(gbofdft_plan*, const void*, void*, int64_t, int, int, const int*, double, double, cudaStream_t);
-int gb_ct_rows_fwd_f64(gbofdft_plan*, const void*, void*, int64_t, int, int, const int*, double, double, cudaStream_t);
-int gb_ct_rows_inv_f32(gbofdft_plan*, const void*, int64_t, int, int, void*, int64_t, double, const EvalDesc*,
-                       const void*, const void*, void*, int, double*, int64_t*, cudaStream_t);
-int gb_ct_rows_inv_f64(gbofdft_plan*, const void*, int64_t, int, int, void*, int64_t, double, const EvalDesc*,
-                       const void*, const void*, void*, int, double*, int64_t*, cudaStream_t);
-int gb_ct_cols_f32(gbofdft_plan*, void*, int64_t, int, int, int, int, double, const KerDesc*, cudaStream_t);
-// plane-major FP32 pipeline (passes_ct_f32.cu)
 int gb_ct_rows_fwd_pm_f32(gbofdft_plan*, const void*, void*, int64_t, int, const int*, double, cudaStream_t);
 int gb_ct_rows_inv_eval_pm_f32(gbofdft_plan*, const void*, int64_t, int, const EvalDesc*, const void*, const void*,
                                void*, int, double*, int64_t*, cudaStream_t);
 int gb_plane_conv_f32(gbofdft_plan*, void*, int64_t, int, const KerDesc*, const float* const*, double, cudaStream_t);
 int gb_plane_supported_f32(int n0, int n1, int n2);
-// WGC fields on the plane pipeline (FP32): the forward rows with the WGC
-// prologues (3 fields rho^e u^k from rho), the forward plane transforms of
-// nf fields (in place), the kernel combination and inverse plane transforms
-// of ngroups groups of three fields (K: the plane-major kernels K0, K1, Kq,
-// Kx), and the inverse rows storing real fields
-int gb_ct_rows_fwd_wgc_pm_f32(gbofdft_plan*, const void* rho, void* spec, int64_t fstride, double e, double rho0,
-                              cudaStream_t);
-int gb_plane_fwd_f32(gbofdft_plan*, void* spec, int64_t fstride, int nf, cudaStream_t);
-int gb_plane_wgc_inv_f32(gbofdft_plan*, const void* spec, int64_t fstride, void* out, int64_t ostride, int ngroups,
-                         const float* K, double scale, cudaStream_t);
 int gb_ct_rows_inv_store_pm_f32(gbofdft_plan*, const void* spec, int64_t fstride, int nf, void* out, int64_t ostride,
                                 cudaStream_t);
-// the inverse rows of the six (three when a == b) combined WGC spectra with
-// the NL potential added to pot (FP32 evaluations); part non-null: per-CTA
-// partial sums of the NL energy integrand, *nblk of them
-int gb_ct_rows_inv_wgc_pm_f32(gbofdft_plan*, const void* spec, int64_t fstride, int two, const float* rho, double rho0,
-                              double ea, double eb, float* pot, double* part, int64_t* nblk, cudaStream_t);
 int gb_plane_variants_f32(int n0, int n1);
 // the plane-major evaluation (returns 1 when the plan has no plane pipeline
 // or a kernel table has no plane-major copy)
 int gb_eval_plane(gbofdft_plan* p, const void* rho, int nf, const int* ops, double beta, const KerDesc& kd,
                   const EvalDesc& ev, const void* vloc, void* pot, int calc_e, double* energies, cudaStream_t st);
-int gb_ct_cols_f64(gbofdft_plan*, void*, int64_t, int, int, int, int, double, const KerDesc*, cudaStream_t);
 // delta evaluation (passes_delta.cu): FP32 transforms of the change of the
 // derived fields against a reference density, FP64 pointwise work
 int gb_delta_rows_fwd(gbofdft_plan* p32, const double* rho, const double* rho_ref, void* spec, int64_t fstride,
