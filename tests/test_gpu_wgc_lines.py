@@ -102,3 +102,45 @@ def test_wgc_on_lines(nr, base, two, prec):
     assert np.abs(pv.double().cpu().numpy() - ref).max() <= tol * scale
     assert abs(float(en[lib.E_NL]) - e_nl) <= tol * e_size
     assert abs(float(en[lib.E_TOTAL]) - e_tot) <= tol * e_size
+
+
+def test_wgc_beside_the_plane_pipeline():
+    """A plan set to the plane schedule: the other terms on planes, the WGC term on
+    lines, added; the same potential and energies as on lines alone within the FP32
+    bound above."""
+    import torch
+    from dftpy_gb300 import _lib as lib
+    from dftpy_gb300.functional.wgc import kernel_table
+    lib.require_cuda()
+    nr, N = (64, 64, 32), 64 * 64 * 32
+    L, s = lib.load(), lib.stream_ptr()
+    plan = lib.Plan(nr, np.diag([0.4 * k for k in nr]), precision=0)
+    rho = 0.03 + 0.01 * np.random.default_rng(1).random(nr)
+    r0 = float(rho.mean())
+    nb = ctypes.c_int64()
+    lib.check(L.gbofdft_wgc_workspace_bytes(plan.handle, ctypes.byref(nb)))
+    buf = torch.empty(int(nb.value) // 8 + 64, dtype=torch.float64, device="cuda")
+    K = torch.empty((4, 64, 64, 17), dtype=torch.float32, device="cuda")
+    t0, h, cols = kernel_table(1.2, 0.47, 2.7, 1.0, 2)
+    tab = torch.tensor(np.ascontiguousarray(cols), dtype=torch.float64, device="cuda")
+    lib.check(L.gbofdft_wgc_kernels(plan.handle, r0, 1.2, 0.47, lib.ptr(tab), int(cols.shape[1]), t0, h, lib.ptr(K), s))
+    d = lib.Wgc()
+    d.alpha, d.beta, d.gamma, d.rho0, d.order = 1.2, 0.47, 2.7, r0, 2
+    d.kernels, d.work, d.work_bytes = K.data_ptr(), lib.aligned_ptr(buf, 256), int(nb.value)
+    f = lib.Functional()
+    f.wgc = ctypes.pointer(d)
+    f.tf, f.tf_x, f.hartree = 1, 1.0, 1
+    rd = torch.tensor(rho, dtype=torch.float32, device="cuda")
+    res = []
+    for sched in (0, 1):
+        lib.check(L.gbofdft_plan_set_schedule(plan.handle, sched))
+        pot = torch.full(nr, float("nan"), dtype=torch.float32, device="cuda")
+        en = torch.zeros(lib.NE, dtype=torch.float64, device="cuda")
+        lib.check(L.gbofdft_eval(plan.handle, lib.ptr(rd), f, lib.ptr(pot), lib.ptr(en), lib.CALC_E | lib.CALC_V, s))
+        res.append((pot.double().cpu().numpy(), en.cpu().numpy()))
+    tol = (8 * np.log2(N) + 16) * 2.0 ** -24
+    (p0, e0), (p1, e1) = res
+    # |4 pi / G^2| rho is the largest term
+    scale = 4 * np.pi / (2 * np.pi / (0.4 * 64)) ** 2 * rho.max()
+    assert np.abs(p0 - p1).max() <= tol * scale
+    assert np.abs(e0 - e1).max() <= tol * scale * rho.sum() * 0.4 ** 3
