@@ -843,6 +843,8 @@ struct Cols {
   int n0, n1, n2, full;
   const void* K;          // WGC: K0, K1, Kq, Kx (API layout), kstride values each
   int64_t kstride;
+  const void* src;        // inverse: read one field from here instead
+  int64_t sstride, sostride;
 };
 
 template <typename T> struct ColTile { static constexpr int TB = 128 / (2 * (int)sizeof(T)); };
@@ -1216,6 +1218,12 @@ __global__ void __launch_bounds__(sizeof(T) == 4 ? 400 : 256) k_rb_cols(const __
   cpx<T>* g = reinterpret_cast<cpx<T>*>(a.data[f]) + outer * a.ostride + k2;
   const cpx<T>* tw = reinterpret_cast<const cpx<T>*>(a.tw);
   const int64_t st = a.stride;
+  const cpx<T>* gs = g;
+  int64_t ss = st;
+  if (DIR > 0 && !CONV && a.src) {
+    gs = reinterpret_cast<const cpx<T>*>(a.src) + outer * a.sostride + k2;
+    ss = a.sstride;
+  }
   ColKernel<T> ker;
   int type = KER_NONE;
   T coef = (T)1;
@@ -1242,7 +1250,7 @@ __global__ void __launch_bounds__(sizeof(T) == 4 ? 400 : 256) k_rb_cols(const __
       constexpr int R = decltype(rc)::R;
       cpx<T> u[R];
 #pragma unroll
-      for (int t = 0; t < R; ++t) u[t] = ok ? g[t * st] : cpx<T>{(T)0, (T)0};
+      for (int t = 0; t < R; ++t) u[t] = ok ? gs[t * ss] : cpx<T>{(T)0, (T)0};
       stage_first<D0, T>(rc, u, tw, n);
       if constexpr (CONV) {
 #pragma unroll
@@ -1263,7 +1271,7 @@ __global__ void __launch_bounds__(sizeof(T) == 4 ? 400 : 256) k_rb_cols(const __
     for (int i = i0; i < nb; i += ni) {
       cpx<T> u[R];
 #pragma unroll
-      for (int t = 0; t < R; ++t) u[t] = ok ? g[(i + t * nb) * st] : cpx<T>{(T)0, (T)0};
+      for (int t = 0; t < R; ++t) u[t] = ok ? gs[(i + t * nb) * ss] : cpx<T>{(T)0, (T)0};
       stage_first<D0, T>(rc, u, tw, n);
 #pragma unroll
       for (int t = 0; t < R; ++t) A[sx(i * R + t)] = u[t];
@@ -1820,6 +1828,9 @@ static int cols(gbofdft_plan* p, const RbCols& d, cudaStream_t st) {
     }
   a.K = d.K;
   a.kstride = p->NG;
+  a.src = d.src;
+  a.sstride = axis == 1 ? d.src_ld : (int64_t)p->n[1] * d.src_ld;
+  a.sostride = axis == 1 ? (int64_t)p->n[1] * d.src_ld : d.src_ld;
   constexpr int TB = ColTile<T>::TB;
   const dim3 grid((a.ncol + TB - 1) / TB, WGC ? nf / 3 : nf);
   auto go = [&](auto kern, const AxisInfo& x) -> int {

@@ -154,6 +154,8 @@ struct RbCols {           // columns of nf spectra: dir, the convolution (kd) or
   double scale;
   const KerDesc* kd;
   const void* K;
+  const void* src;        // dir 1, nf = 1: the field is read from here (row pitch src_ld)
+  int src_ld;
 };
 #define GB_RB_DECLARE(SUF)                                                                \
   int gb_rb_rows_fwd_##SUF(gbofdft_plan*, const RbFwd&, cudaStream_t);                    \

@@ -59,3 +59,30 @@ def test_line_lengths(lib, n, axis, prec):
                                  lib.stream_ptr()))
     want = np.fft.irfftn(np.fft.rfftn(x) * K, s=nr, axes=(0, 1, 2))
     assert np.abs(conv.cpu().numpy() - want).max() <= 4 * tol * np.abs(want).max()
+
+
+@pytest.mark.parametrize("prec", [1, 0])
+@pytest.mark.parametrize("nr", [(12, 10, 14), (9, 15, 7), (22, 6, 8), (8, 7, 5)])
+def test_c2r_input_alignment(lib, nr, prec):
+    """The first inverse pass reads the caller's spectrum where it is aligned to a
+    complex value (else a copy of it): the same values, and the input is left alone."""
+    import torch
+    dt = torch.float64 if prec else torch.float32
+    plan = lib.Plan(nr, np.diag([float(k) for k in nr]), precision=prec)
+    L = lib.load()
+    X = np.fft.rfftn(np.random.default_rng(3).standard_normal(nr))
+    flat = torch.tensor(np.ascontiguousarray(X).view(np.float64).reshape(-1), dtype=dt, device="cuda")
+    res = []
+    for off in (0, 1, 2):
+        buf = torch.zeros(flat.numel() + 4, dtype=dt, device="cuda")
+        buf[off:off + flat.numel()] = flat
+        keep = buf.clone()
+        out = torch.full(nr, float("nan"), dtype=dt, device="cuda")
+        p = buf.data_ptr() + off * buf.element_size()
+        lib.check(L.gbofdft_fft_c2r(plan.handle, p, lib.ptr(out), lib.stream_ptr()))
+        assert torch.equal(buf, keep)
+        res.append(out)
+    assert torch.equal(res[0], res[1]) and torch.equal(res[0], res[2])
+    want = np.fft.irfftn(X, s=nr, axes=(0, 1, 2))
+    tol = 8 * (2.0 ** -53 if prec else 2.0 ** -24) * np.log2(np.prod(nr))
+    assert np.abs(res[0].cpu().numpy() - want).max() <= tol * np.abs(want).max()
