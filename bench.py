@@ -718,7 +718,7 @@ def main():
         traffic = profile_traffic()
         roofline = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                     "peak_kind": peak_kind, "traffic": traffic.get("bytes_per_eval") if traffic else None,
-                    "kernel": "FP32 potential evaluation (rows / plane-convolution / rows pipeline), 128^3, "
+                    "kernel": "FP32 potential evaluation (the schedule that the autotuner picked), 128^3, "
                               "WT + LDA + Hartree + PP",
                     "t_eval_us": t_eval * 1e6, "n_evals_timed": live[1],
                     "timing": "CUDA events around each FP32 potential evaluation inside the al256 timed solves "
