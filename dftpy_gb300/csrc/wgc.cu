@@ -12,10 +12,12 @@
 // (A = rho^a, B = rho^b; Y0..Y2 the same with A):
 //   E = int A (X0 + u X1 + u^2 X2),
 //   V = A'(X0 + u X1 + u^2 X2) + (A/rho*)(X1 + 2u X2) + B'(Y0 + u Y1 + u^2 Y2) + (B/rho*)(Y1 + 2u Y2).
-// One evaluation: a pointwise pass (the 3 or 6 transformed fields), their
-// forward transforms, one reciprocal-space pass forming X and Y, the
-// inverse transforms and a pointwise pass adding V and reducing E.  With
-// a == b, Y = X and half the transforms are skipped.
+// One evaluation: the 3 or 6 transformed fields out of the row prologue, axis 1
+// together with the other terms' fields, X and Y formed along axis 0 between the
+// forward and inverse transforms, V and E in the epilogue of the inverse rows
+// (gb_wgc_eval_fused).  Lines of one stage or with a prime factor above 7: a
+// pointwise pass, the transforms, a reciprocal-space pass, the inverse transforms
+// and a pointwise pass.  With a == b, Y = X and half the transforms are skipped.
 #include <math.h>
 #include <string.h>
 
