@@ -264,11 +264,13 @@ int gbofdft_fft_r2c(gbofdft_plan* p, const void* in, void* out, void* stream) {
   GB_REQUIRE(p && in && out, "fft_r2c: null argument");
   cudaStream_t st = (cudaStream_t)stream;
   const int op = OP_RHO;
-  // the row pass writes twice the spectra (scale 2: separating a row pair then
-  // needs no multiplication); the factor is undone in the last pass
-  int rc = gb_rows_fwd(p, in, out, 0, p->n2h, 1, &op, 1.0, 2.0, st);
+  // FP64: the row pass writes twice the spectra (scale 2: separating a row pair
+  // then needs no multiplication) and the last pass undoes it; FP32, not bound by
+  // its operations, scales once, in the rows
+  const bool late = p->prec == GBOFDFT_F64;
+  int rc = gb_rows_fwd(p, in, out, 0, p->n2h, 1, &op, 1.0, late ? 2.0 : p->dV, st);
   if (!rc) rc = gb_cols(p, out, 0, p->n2h, 1, 1, -1, 1.0, st);
-  if (!rc) rc = gb_cols(p, out, 0, p->n2h, 1, 0, -1, 0.5 * p->dV, st);
+  if (!rc) rc = gb_cols(p, out, 0, p->n2h, 1, 0, -1, late ? 0.5 * p->dV : 1.0, st);
   return rc;
 }
 
