@@ -169,11 +169,11 @@ __device__ __forceinline__ Derived<T> derived(const RowsFwd& a, T rho) {
     }
   } else if constexpr (KIND != PK_PLAIN) {
     const T kz = (T)kZero;
-    const T rc = rho > kz ? rho : kz;
+    const T rc = rho < kz ? kz : rho;                    // a NaN stays one in the powers
     const Roots<T> r = roots(rc);
     d.sq = sqrt_of(rc, r);
     if (sizeof(T) == 4 && !a.rsq) d.sq = sqrt(rc);
-    if (rho > (T)0 && rho < kz) d.sq = sqrt_call<T>(rho);
+    if (!(rho >= kz)) d.sq = sqrt_call<T>(rho > (T)0 ? rho : kz);
     if constexpr (KIND == PK_ROOTS) d.b = pow56(rc, r);
     else d.b = pow_general<T>(rc, sc<T>(a.beta));
   }

@@ -1,0 +1,54 @@
+"""Pointwise terms of the evaluation's row passes (GPU): densities that the
+clamps meet, against the clamps written out in numpy."""
+import ctypes
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+KZ = 1e-30
+# rows of kernels of one length, of run-time lengths (odd, above 400), of a prime factor above 7
+LENGTHS = [36, 128, 105, 486, 22]
+
+
+@pytest.fixture(scope="module")
+def lib():
+    from dftpy_gb300 import _lib
+    _lib.require_cuda()
+    return _lib
+
+
+def _plan(lib, nr, prec):
+    return lib.Plan(nr, np.diag([0.4 * k for k in nr]), precision=prec)
+
+
+def _eval(lib, plan, f, rho, energies=True):
+    """Potential and energies of the functional ``f`` at ``rho`` (numpy)."""
+    import torch
+    r = torch.tensor(rho, dtype=torch.float64 if plan.precision == lib.F64 else torch.float32, device="cuda")
+    pot = torch.full_like(r, 7.0)
+    en = torch.zeros(lib.NE, dtype=torch.float64, device="cuda")
+    lib.check(lib.load().gbofdft_eval(plan.handle, lib.ptr(r), ctypes.byref(f), lib.ptr(pot), lib.ptr(en),
+                                      lib.CALC_V | (lib.CALC_E if energies else 0), lib.stream_ptr()))
+    torch.cuda.synchronize()
+    return pot.cpu().numpy(), en.cpu().numpy()
+
+
+@pytest.mark.parametrize("prec", [1, 0])
+@pytest.mark.parametrize("beta", [5 / 6, 0.7])
+@pytest.mark.parametrize("n2", LENGTHS)
+def test_nan_density_reaches_the_power(lib, n2, beta, prec):
+    """A NaN of the density is one of rho^beta, and the convolution carries it to every
+    point of the Wang-Teter potential: a broken density must not look like a good one."""
+    import torch
+    nr = (6, 5, n2)
+    plan = _plan(lib, nr, prec)
+    kern = torch.ones((6, 5, n2 // 2 + 1), dtype=torch.float64 if prec else torch.float32, device="cuda")
+    f = lib.Functional()
+    f.wt, f.wt_alpha, f.wt_beta, f.wt_kernel = 1, beta, beta, kern.data_ptr()
+    rho = np.full(nr, 0.03)
+    assert np.isfinite(_eval(lib, plan, f, rho)[0]).all()
+    rho[3, 2, n2 // 3] = np.nan
+    pot, en = _eval(lib, plan, f, rho)
+    assert np.isnan(pot).all() and np.isnan(en[lib.E_NL])
