@@ -475,10 +475,45 @@ __device__ __forceinline__ void pz_lda(T rho, const Roots<T>& r, T& eps, T& pot,
   }
 }
 
+// A thread's sum of one energy term over its points (the 2 rl points of a row
+// pair's butterfly, up to 32, rarely of a second one), in double across threads.
+// FP32: the running sum and the sum of its rounding errors, and products of two
+// fields with theirs, so that n points add an error of n^2 2^-49 at most where
+// 24-bit sums had n 2^-24 (measured: 1e-9 of the total); doubles would take the
+// FP64 pipe 12 operations a point.
+template <typename T> struct ESum;
+template <> struct ESum<double> {
+  double s;
+  __device__ __forceinline__ void init() { s = 0.0; }
+  __device__ __forceinline__ void add(double x) { s += x; }
+  __device__ __forceinline__ void add_product(double x, double y) { s += x * y; }
+  __device__ __forceinline__ void add(const ESum& o) { s += o.s; }
+  __device__ __forceinline__ double value() const { return s; }
+};
+template <> struct ESum<float> {
+  float s, c;
+  __device__ __forceinline__ void init() { s = c = 0.0f; }
+  __device__ __forceinline__ void add(float x) {
+    const float t = __fadd_rn(s, x), z = __fsub_rn(t, s);
+    c += __fsub_rn(s, __fsub_rn(t, z)) + __fsub_rn(x, z);
+    s = t;
+  }
+  __device__ __forceinline__ void add_product(float x, float y) {
+    const float p = __fmul_rn(x, y);
+    add(p);
+    c += __fmaf_rn(x, y, -p);
+  }
+  __device__ __forceinline__ void add(const ESum& o) {
+    add(o.s);
+    c += o.c;
+  }
+  __device__ __forceinline__ double value() const { return (double)s + (double)c; }
+};
+
 // the pointwise terms at rho <= 1e-30 (the reference's clamps), out of line
 template <typename T>
 __device__ __noinline__ void point_tiny(const RowsInv& a, T rho, T w, T kc, T vh, T vl, bool want_e, T* pot_out,
-                                        T* es) {
+                                        ESum<T>* es) {
   const EvalDesc& ev = a.ev;
   T pot = (T)0;
   const T kz = (T)kZero;
@@ -487,19 +522,19 @@ __device__ __noinline__ void point_tiny(const RowsInv& a, T rho, T w, T kc, T vh
     if (want_e) {
       T r5 = rho * rho;
       r5 = r5 * rho; r5 = r5 * rho; r5 = r5 * rho;
-      es[0] += cbrt(r5) * sc<T>(a.tf_e);
+      es[0].add(cbrt(r5) * sc<T>(a.tf_e));
     }
   }
   if (ev.vw) {
     const T v = (T)0.5 * w * (rho > (T)0 ? (T)1 / fmax(sqrt(rho), kz) : (T)1e15);
     pot += v * sc<T>(a.vw_y);
-    if (want_e && rho > (T)0) es[1] += rho * v * sc<T>(a.vw_y);
+    if (want_e && rho > (T)0) es[1].add(rho * v * sc<T>(a.vw_y));
   }
   if (ev.wt) {
     const T rb = a.b56 ? sqrt(kz) * cbrt(kz) / kz : pow(kz, sc<T>(a.wt_beta)) / kz;
     const T v = sc<T>(a.two_alpha) * rb * kc;
     pot += v;
-    if (want_e) es[2] += v * rho * sc<T>(a.inv_two_alpha);
+    if (want_e) es[2].add(v * rho * sc<T>(a.inv_two_alpha));
   }
   if (ev.xc) {
     const T cx = (T)0.98474502184269654115;
@@ -516,15 +551,15 @@ __device__ __noinline__ void point_tiny(const RowsInv& a, T rho, T w, T kc, T vh
     vx += cx * (rc * rc * rc * inv * inv) - cx * rc;
     eps += (T)0.75 * cx * (rc * rc * rc * inv * inv) - (T)0.75 * cx * rc;
     pot += vx;
-    if (want_e) es[3] += eps * rho;
+    if (want_e) es[3].add(eps * rho);
   }
   if (ev.hartree) {
     pot += vh;
-    if (want_e) es[4] += (T)0.5 * vh * rho;
+    if (want_e) es[4].add_product((T)0.5 * vh, rho);
   }
   if (ev.pp) {
     pot += vl;
-    if (want_e) es[5] += vl * rho;
+    if (want_e) es[5].add_product(vl, rho);
   }
   *pot_out = pot;
 }
@@ -532,15 +567,17 @@ __device__ __noinline__ void point_tiny(const RowsInv& a, T rho, T w, T kc, T vh
 // potential at one point from its density and convolution results; energy
 // densities added to es
 template <typename T, bool WANT_E>
-__device__ __forceinline__ T point(const RowsInv& a, T rho, T w, T kc, T vh, T vl, T* es) {
+__device__ __forceinline__ T point(const RowsInv& a, T rho, T w, T kc, T vh, T vl, ESum<T>* es) {
   const EvalDesc& ev = a.ev;
   if (!(rho > (T)kZero)) {
     T p;
-    T e6[6] = {0, 0, 0, 0, 0, 0};
+    ESum<T> e6[6];
+#pragma unroll
+    for (int q = 0; q < 6; ++q) e6[q].init();
     point_tiny<T>(a, rho, w, kc, vh, vl, WANT_E, &p, e6);
     if constexpr (WANT_E) {
 #pragma unroll
-      for (int q = 0; q < 6; ++q) es[q] += e6[q];
+      for (int q = 0; q < 6; ++q) es[q].add(e6[q]);
     }
     return p;
   }
@@ -549,33 +586,33 @@ __device__ __forceinline__ T point(const RowsInv& a, T rho, T w, T kc, T vh, T v
   if (ev.tf) {
     const T r23 = rho * r.z3;                           // rho^(2/3)
     pot += sc<T>(a.tf_v) * r23;
-    if (WANT_E) es[0] += rho * r23 * sc<T>(a.tf_e);
+    if (WANT_E) es[0].add(rho * r23 * sc<T>(a.tf_e));
   }
   if (ev.vw) {
     const T v = (T)0.5 * w * r.z2 * sc<T>(a.vw_y);
     pot += v;
-    if (WANT_E) es[1] += rho * v;
+    if (WANT_E) es[1].add(rho * v);
   }
   if (ev.wt) {
     // rho^(beta - 1)
     const T rb = a.b56 ? (sizeof(T) == 8 ? r.y : rho * r.z3 * r.z3 * r.z2) : pow_general<T>(rho, sc<T>(a.wt_beta)) / rho;
     const T v = sc<T>(a.two_alpha) * rb * kc;
     pot += v;
-    if (WANT_E) es[2] += v * rho * sc<T>(a.inv_two_alpha);
+    if (WANT_E) es[2].add(v * rho * sc<T>(a.inv_two_alpha));
   }
   if (ev.xc) {
     T eps, vx;
     pz_lda<T>(rho, r, eps, vx, WANT_E);
     pot += vx;
-    if (WANT_E) es[3] += eps * rho;
+    if (WANT_E) es[3].add(eps * rho);
   }
   if (ev.hartree) {
     pot += vh;
-    if (WANT_E) es[4] += (T)0.5 * vh * rho;
+    if (WANT_E) es[4].add_product((T)0.5 * vh, rho);
   }
   if (ev.pp) {
     pot += vl;
-    if (WANT_E) es[5] += vl * rho;
+    if (WANT_E) es[5].add_product(vl, rho);
   }
   return pot;
 }
@@ -583,13 +620,14 @@ __device__ __forceinline__ T point(const RowsInv& a, T rho, T w, T kc, T vh, T v
 // the WGC term at one point from its six fields (FP64: and the powers A, B of
 // the forward rows): potential; energy density added to es[2]
 template <typename T, bool WANT_E>
-__device__ __forceinline__ T wgc_point(const RowsInv& a, T rho, T A, T B, T X0, T X1, T X2, T Y0, T Y1, T Y2, T* es) {
+__device__ __forceinline__ T wgc_point(const RowsInv& a, T rho, T A, T B, T X0, T X1, T X2, T Y0, T Y1, T Y2,
+                                       ESum<T>* es) {
   const T rc = rho > (T)kZero ? rho : (T)kZero;
   const T inv0 = sc<T>(a.w_inv0), u = (rc - sc<T>(a.w_rho0)) * inv0;
   if constexpr (sizeof(T) == 4) A = pow_of(rc, sc<T>(a.w_a));
   const T ir = rcp_nr(rc);
   const T sx = X0 + u * X1 + u * u * X2, tx = X1 + (T)2 * u * X2;
-  if (WANT_E) es[2] += A * sx;
+  if (WANT_E) es[2].add(A * sx);
   T v = A * (sc<T>(a.w_a) * ir * sx + inv0 * tx);
   if (a.two) {
     if constexpr (sizeof(T) == 4) B = pow_of(rc, sc<T>(a.w_b));
@@ -680,7 +718,9 @@ __global__ void __launch_bounds__(RowCta<T>::NT, (RowCta<T, AX>::MINB)) k_rb_row
   // last stage: a thread transforms butterfly i of every field of a row pair
   // in place (its own elements), so the points i + t nb are complete in it
   const int nb = ax.nbl(), rl = ax.rl();
-  T es[6] = {0, 0, 0, 0, 0, 0};
+  ESum<T> es[6];
+#pragma unroll
+  for (int c = 0; c < 6; ++c) es[c].init();
   for (int t0 = tid; t0 < lp * nb; t0 += nthr) {
     const int l = ax.div_nbl(t0), i = t0 - l * nb;
     const int ra = base + 2 * l;
@@ -814,7 +854,7 @@ __global__ void __launch_bounds__(RowCta<T>::NT, (RowCta<T, AX>::MINB)) k_rb_row
   const int lane = tid & 31, warp = tid >> 5;
 #pragma unroll
   for (int c = 0; c < 6; ++c) {
-    const double v = warp_sum((double)es[c]);
+    const double v = warp_sum(es[c].value());
     if (lane == 0) red[warp][c] = v;
   }
   __syncthreads();

@@ -52,3 +52,37 @@ def test_nan_density_reaches_the_power(lib, n2, beta, prec):
     rho[3, 2, n2 // 3] = np.nan
     pot, en = _eval(lib, plan, f, rho)
     assert np.isnan(pot).all() and np.isnan(en[lib.E_NL])
+
+
+@pytest.mark.parametrize("prec", [1, 0])
+@pytest.mark.parametrize("rows", [(2, 3), (1, 1), (12, 10)])
+@pytest.mark.parametrize("n2", LENGTHS[:4] + [84, 400, 8])
+def test_energy_sums(lib, n2, rows, prec):
+    """Energies that are sums of products of two fields of the plan's precision.
+
+    Tolerance: the products are exact to twice the precision and a thread's n <= 64
+    points add an error below n^2 2^-49 = 8e-12 of the magnitudes' sum (FP32), n 2^-53
+    (FP64); the additions above are FP64, below 64 2^-53."""
+    import math
+    import torch
+    nr = rows + (n2,)
+    plan = _plan(lib, nr, prec)
+    dt = np.float64 if prec else np.float32
+    rng = np.random.default_rng(n2)
+    rho = (0.03 + 0.02 * rng.random(nr)).astype(dt)
+    vloc = (1.0 + rng.random(nr)).astype(dt)
+    dV = 0.4 ** 3
+    tol = 128 * 2.0 ** -53 if prec else 1e-11
+    vd = torch.tensor(vloc, device="cuda")
+    f = lib.Functional()
+    f.vloc = vd.data_ptr()
+    pot, en = _eval(lib, plan, f, rho)
+    assert np.array_equal(pot, vloc)
+    terms = (rho.astype(float) * vloc.astype(float)).ravel()       # exact in FP32's case
+    want = math.fsum(terms) * dV
+    assert abs(en[lib.E_PSEUDO] - want) <= tol * want
+    f = lib.Functional()
+    f.hartree = 1
+    pot, en = _eval(lib, plan, f, rho)
+    terms = (0.5 * rho.astype(float) * pot.astype(float)).ravel()
+    assert abs(en[lib.E_HARTREE] - math.fsum(terms) * dV) <= tol * np.abs(terms).sum() * dV
