@@ -89,9 +89,7 @@ __device__ __forceinline__ float rcp_nr(float x) { return 1.0f / x; }
 
 // x^(-1/6), x in the float range: one third-order (Halley-type) step on the
 // seed, y (1 + r/6 + 7 r^2/72) with r = 1 - x y^6 (|r| < 1e-5, so the next term
-// is below 1e-16).  x^(-1/3) and x^(-1/2) are its square and cube: 9 FP64
-// operations for all of them, where separate Newton iterations for the two
-// took 25 (the FP64 pipe bounds the FP64 row passes).
+// is below 1e-16)
 __device__ __forceinline__ double rroot6(double x) {
   const double y = (double)rsqrtf(cbrtf((float)x));
   const double y2 = y * y;
@@ -99,22 +97,48 @@ __device__ __forceinline__ double rroot6(double x) {
   return fma(y * r, fma(r, 7.0 / 72.0, 1.0 / 6.0), y);
 }
 
-// rho^(-1/3), rho^(-1/2) and (FP64) rho^(-1/6) of a positive density
-template <typename T> struct Roots { T z3, z2, y; };
-__device__ __forceinline__ Roots<float> roots(float x) { return Roots<float>{rcbrtf(x), rsqrtf(x), 0.0f}; }
+// The roots of a positive density that the terms are made of: x^(1/3), x^(-1/3),
+// x^(-1/2) and (FP64) x^(-1/6), from single-precision seeds.  Each ends in one
+// correction by a residual that one or two roundings separate from the exact one,
+// so the first three are good to about one rounding themselves, and the terms to
+// no more than library calls of cbrt, sqrt and division gave them (rms error of
+// the potentials in 2^-53, 24 x 20 x 84: Thomas-Fermi 1.0, LDA 0.6; library 1.2,
+// 0.7; the powers of one x^(-1/6), 13 FP64 operations against 20, 1.6, 1.7).
+template <typename T> struct Roots { T c, z3, z2, y; };
 __device__ __forceinline__ Roots<double> roots(double x) {
-  const double y = rroot6(x), y2 = y * y;
-  return Roots<double>{y2, y2 * y, y};
+  const float f = (float)x;
+  const double a = (double)rcbrtf(f), b = (double)rsqrtf(f);
+  // squares of FP32 numbers are exact; r = 1 - x a^3, e = 1 - x b^2
+  const double a2 = a * a, r = fma(-x, a2 * a, 1.0), e = fma(-x, b * b, 1.0);
+  Roots<double> q;
+  q.z3 = fma(a * r, fma(r, 2.0 / 9.0, 1.0 / 3.0), a);
+  q.z2 = fma(b * e, fma(e, 0.375, 0.5), b);
+  const double c = x * q.z3 * q.z3;
+  q.c = fma(fma(-(c * c), c, x), a2 * (1.0 / 3.0), c);
+  q.y = q.c * q.z2;
+  return q;
 }
-__device__ __forceinline__ float sqrt_of(float x, const Roots<float>& r) { return x * r.z2; }
-// one more Newton step: the rounding of sqrt(rho) is what the G^2 kernel amplifies
-__device__ __forceinline__ double sqrt_of(double x, const Roots<double>& r) {
-  const double s = x * r.z2;
-  return fma(0.5 * r.z2, fma(-s, s, x), s);
+__device__ __forceinline__ Roots<float> roots(float x) {
+  const float a = rcbrtf(x), b = rsqrtf(x);
+  const float a2 = a * a, c = x * a2, s = x * b;
+  Roots<float> q;
+  q.z3 = a;
+  q.z2 = fmaf(b * fmaf(-s, b, 1.0f), 0.5f, b);
+  q.c = fmaf(fmaf(-(c * c), c, x), a2 * (1.0f / 3.0f), c);
+  q.y = 0.0f;
+  return q;
 }
-// x^(5/6)
-__device__ __forceinline__ float pow56(float x, const Roots<float>& r) { return (x * r.z2) * (x * r.z3 * r.z3); }
-__device__ __forceinline__ double pow56(double x, const Roots<double>& r) { return x * r.y; }
+// x^(1/2) and x^(5/6) of the forward rows.  FP64: from x^(-1/6); one more Newton
+// step for the square root, whose rounding the G^2 kernel amplifies.
+template <typename T> struct Powers { T sq, p56; };
+__device__ __forceinline__ Powers<double> powers(double x) {
+  const double y = rroot6(x), z2 = y * y * y, s = x * z2;
+  return Powers<double>{fma(0.5 * z2, fma(-s, s, x), s), x * y};
+}
+__device__ __forceinline__ Powers<float> powers(float x) {
+  const Roots<float> r = roots(x);
+  return Powers<float>{x * rsqrtf(x), x * r.z2 * r.c};
+}
 
 // ---- forward rows ---------------------------------------------------------------
 struct RowsFwd {
@@ -170,11 +194,11 @@ __device__ __forceinline__ Derived<T> derived(const RowsFwd& a, T rho) {
   } else if constexpr (KIND != PK_PLAIN) {
     const T kz = (T)kZero;
     const T rc = rho < kz ? kz : rho;                    // a NaN stays one in the powers
-    const Roots<T> r = roots(rc);
-    d.sq = sqrt_of(rc, r);
+    const Powers<T> r = powers(rc);
+    d.sq = r.sq;
     if (sizeof(T) == 4 && !a.rsq) d.sq = sqrt(rc);
     if (!(rho >= kz)) d.sq = sqrt_call<T>(rho > (T)0 ? rho : kz);
-    if constexpr (KIND == PK_ROOTS) d.b = pow56(rc, r);
+    if constexpr (KIND == PK_ROOTS) d.b = r.p56;
     else d.b = pow_general<T>(rc, sc<T>(a.beta));
   }
   return d;
@@ -199,7 +223,7 @@ __device__ __forceinline__ T field_direct(int op, T rho, bool rsq) {
   }
   if (op == OP_POWB) {
     const T rc = rho < kz ? kz : rho;
-    return pow56(rc, roots(rc));
+    return powers(rc).p56;
   }
   return rho;
 }
@@ -429,7 +453,7 @@ struct RowsInv {
   int64_t ostride;
   Sc scale;
   EvalDesc ev;
-  Sc tf_v, tf_e, vw_y, two_alpha, inv_two_alpha, wt_beta;
+  Sc tf_v, tf_vl, tf_e, vw_y, half_vw, two_alpha, inv_two_alpha, wt_beta;
   int b56;
   const void* rho;
   const void* vloc;
@@ -450,14 +474,14 @@ struct RowsInv {
 static __device__ __noinline__ double log_call(double x) { return log(x); }
 static __device__ __forceinline__ float log_call(float x) { return logf(x); }
 
-// Perdew-Zunger 1981 LDA at rho > 0 given its roots: potential and (want_e)
+// Perdew-Zunger 1981 LDA given the density's roots: potential and (want_e)
 // energy per particle
 template <typename T>
-__device__ __forceinline__ void pz_lda(T rho, const Roots<T>& r, T& eps, T& pot, bool want_e) {
+__device__ __forceinline__ void pz_lda(const Roots<T>& r, T& eps, T& pot, bool want_e) {
   const T a = (T)0.0311, b = (T)-0.048, c = (T)0.0020, d = (T)-0.0116;
   const T g = (T)-0.1423, b1 = (T)1.0529, b2 = (T)0.3334;
   const T cx = (T)0.98474502184269654115;                 // (3/pi)^(1/3)
-  const T rc = rho * r.z3 * r.z3;
+  const T rc = r.c;
   const T rs = (T)0.62035049089940001667 * r.z3;          // (3/(4 pi))^(1/3) / rho^(1/3)
   pot = -cx * rc;
   eps = (T)(-0.75) * cx * rc;
@@ -537,19 +561,16 @@ __device__ __noinline__ void point_tiny(const RowsInv& a, T rho, T w, T kc, T vh
     if (want_e) es[2].add(v * rho * sc<T>(a.inv_two_alpha));
   }
   if (ev.xc) {
-    const T cx = (T)0.98474502184269654115;
     T rc = cbrt(rho);
     if (rc < kz) rc = kz;
     const T inv = (T)1 / rc;
     T vx, eps;
     Roots<T> r;
+    r.c = rc;
     r.z3 = inv;
     r.z2 = (T)0;
     r.y = sqrt(inv);
-    // pz_lda forms rho^(1/3) as rho z3^2; here it is the clamped rc
-    pz_lda<T>(rc * rc * rc, r, eps, vx, want_e);
-    vx += cx * (rc * rc * rc * inv * inv) - cx * rc;
-    eps += (T)0.75 * cx * (rc * rc * rc * inv * inv) - (T)0.75 * cx * rc;
+    pz_lda<T>(r, eps, vx, want_e);
     pot += vx;
     if (want_e) es[3].add(eps * rho);
   }
@@ -585,24 +606,25 @@ __device__ __forceinline__ T point(const RowsInv& a, T rho, T w, T kc, T vh, T v
   T pot = (T)0;
   if (ev.tf) {
     const T r23 = rho * r.z3;                           // rho^(2/3)
-    pot += sc<T>(a.tf_v) * r23;
+    if constexpr (sizeof(T) == 4) pot = fma(sc<T>(a.tf_v), r23, sc<T>(a.tf_vl) * r23);
+    else pot += sc<T>(a.tf_v) * r23;
     if (WANT_E) es[0].add(rho * r23 * sc<T>(a.tf_e));
   }
   if (ev.vw) {
-    const T v = (T)0.5 * w * r.z2 * sc<T>(a.vw_y);
+    const T v = w * r.z2 * sc<T>(a.half_vw);
     pot += v;
     if (WANT_E) es[1].add(rho * v);
   }
   if (ev.wt) {
     // rho^(beta - 1)
-    const T rb = a.b56 ? (sizeof(T) == 8 ? r.y : rho * r.z3 * r.z3 * r.z2) : pow_general<T>(rho, sc<T>(a.wt_beta)) / rho;
+    const T rb = a.b56 ? (sizeof(T) == 8 ? r.y : r.c * r.z2) : pow_general<T>(rho, sc<T>(a.wt_beta)) / rho;
     const T v = sc<T>(a.two_alpha) * rb * kc;
     pot += v;
     if (WANT_E) es[2].add(v * rho * sc<T>(a.inv_two_alpha));
   }
   if (ev.xc) {
     T eps, vx;
-    pz_lda<T>(rho, r, eps, vx, WANT_E);
+    pz_lda<T>(r, eps, vx, WANT_E);
     pot += vx;
     if (WANT_E) es[3].add(eps * rho);
   }
@@ -1732,9 +1754,11 @@ static int rows_inv(gbofdft_plan* p, const RbInv& d, int64_t* nblk_out, cudaStre
     a.vstore = d.vstore;
   }
   const double ctf = 2.87123400018819181594;    // (3/10)(3 pi^2)^(2/3)
-  a.tf_v.set(5.0 / 3.0 * ctf * ev->tf_x);
+  a.tf_v.set(4.78539000031365302657 * ev->tf_x);   // (5/3) ctf
+  a.tf_vl.set(a.tf_v.d - (double)a.tf_v.f);        // (FP32: the rest of it)
   a.tf_e.set(ctf * ev->tf_x);
   a.vw_y.set(ev->vw_y);
+  a.half_vw.set(0.5 * ev->vw_y);
   a.two_alpha.set(2.0 * ev->wt_alpha);
   a.inv_two_alpha.set(ev->wt_alpha != 0.0 ? 1.0 / (2.0 * ev->wt_alpha) : 0.0);
   a.wt_beta.set(ev->wt_beta);
