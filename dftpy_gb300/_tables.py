@@ -23,9 +23,41 @@ def spline_notaknot(x, y):
         raise ValueError("spline needs >= 4 points")
     if x.shape != y.shape or x.ndim != 1:
         raise ValueError("spline points have shapes %s and %s" % (x.shape, y.shape))
+    try:
+        L = _lib.load()
+    except _lib.GbofdftError:                   # not built: tables need no GPU, and no library either
+        return x, _spline_numpy(x, y)
     c = np.empty((x.size - 1, 4))
-    _lib.check(_lib.load().gbofdft_spline(x.size, x.ctypes.data, y.ctypes.data, c.ctypes.data), "spline")
+    _lib.check(L.gbofdft_spline(x.size, x.ctypes.data, y.ctypes.data, c.ctypes.data), "spline")
     return x, c
+
+
+def _spline_numpy(x, y):
+    """``gbofdft_spline``'s elimination in Python: a loop of 8 ms for 10,000 points
+    where the library takes 0.1 to 0.3."""
+    n = x.size
+    m = n - 2                                   # unknowns M[1..n-2], the second derivatives
+    h = np.diff(x)
+    delta = np.diff(y) / h
+    lo, up = h[:-1].copy(), h[1:].copy()        # row j: lo M[j] + di M[j+1] + up M[j+2]
+    di = 2.0 * (lo + up)
+    r = 6.0 * (delta[1:] - delta[:-1])
+    # third derivative continuous at x[1]: M0 = ((h0 + h1) M1 - h0 M2) / h1; at x[n-2] likewise
+    di[0] += h[0] * (h[0] + h[1]) / h[1]
+    up[0] -= h[0] * h[0] / h[1]
+    di[-1] += h[-1] * (h[-2] + h[-1]) / h[-2]
+    lo[-1] -= h[-1] * h[-1] / h[-2]
+    for i in range(1, m):
+        w = lo[i] / di[i - 1]
+        di[i] -= w * up[i - 1]
+        r[i] -= w * r[i - 1]
+    M = np.zeros(n)
+    for i in range(m - 1, -1, -1):
+        M[i + 1] = (r[i] - (up[i] * M[i + 2] if i < m - 1 else 0.0)) / di[i]
+    M[0] = ((h[0] + h[1]) * M[1] - h[0] * M[2]) / h[1]
+    M[-1] = ((h[-2] + h[-1]) * M[-2] - h[-1] * M[-3]) / h[-2]
+    return np.stack([y[:-1], delta - h * (2.0 * M[:-1] + M[1:]) / 6.0, M[:-1] / 2.0,
+                     (M[1:] - M[:-1]) / (6.0 * h)], axis=1)
 
 
 def quartic_coefficients(vp):
