@@ -15,6 +15,7 @@
 #include <string.h>
 
 #include <chrono>
+#include <exception>
 #include <mutex>
 #include <vector>
 
@@ -942,7 +943,13 @@ int gbofdft_spline(int64_t n, const double* x, const double* y, double* c) {
   // through their neighbours.  A serial chain of 2 n divisions: 10,000 points
   // take 0.1 ms here, 8 ms as a Python loop.
   const int64_t m = n - 2;
-  std::vector<double> cp(m), M(n);
+  std::vector<double> cp, M;
+  try {
+    cp.resize(m);
+    M.resize(n);
+  } catch (const std::exception&) {              // no exception leaves a C entry
+    return gb_set_error(GBOFDFT_ERR_ALLOC, "spline: no memory for %lld points", (long long)n);
+  }
   const double h0 = x[1] - x[0], h1 = x[2] - x[1], ha = x[n - 2] - x[n - 3], hb = x[n - 1] - x[n - 2];
   double hl = h0, dl = (y[1] - y[0]) / h0;
   for (int64_t i = 0; i < m; ++i) {

@@ -28,3 +28,13 @@ def test_spline_without_library(n, tmp_path):
     got = np.load(tmp_path / "out.npz")["c"]
     assert got.shape == c.shape
     np.testing.assert_allclose(got, c, rtol=0, atol=256 * 2.0 ** -53 * np.abs(c).max())
+
+
+def test_spline_that_does_not_fit_in_memory():
+    """A status, no exception through the C entry (which would end the process)."""
+    code = ("import ctypes\nfrom dftpy_gb300 import _lib\nx = (ctypes.c_double * 4)(0, 1, 2, 3)\n"
+            "p = ctypes.cast(x, ctypes.c_void_p)\nrc = _lib.load().gbofdft_spline(1 << 60, p, p, p)\n"
+            "assert rc == 4 and 'memory' in _lib.last_error(), rc\n")
+    env = dict(os.environ, PYTHONPATH=ROOT + os.pathsep + os.environ.get("PYTHONPATH", ""))
+    r = subprocess.run([sys.executable, "-c", code], cwd=ROOT, env=env, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr
