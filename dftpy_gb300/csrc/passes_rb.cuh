@@ -1590,10 +1590,14 @@ template <typename P> struct InverseOrder<P, true> {
 template <typename P> using inverse_order = typename InverseOrder<P, P::ax::kFixed>::type;
 #define GB_RB_G(...) Rad<__VA_ARGS__>
 template <typename T, typename F> static int by_axis(const RbAxis& ax, F&& f) {
-#define GB_RB_TWO(N, A, B) \
-  case N: return f(AxPair<Ax2<A, B>, Ax2<B, A>>{});
-#define GB_RB_THREE(N, A, B, C) \
-  case N: return f(AxPair<Ax3<A, B, C>, Ax3<C, B, A>>{});
+#define GB_RB_TWO(LEN, A, B)                                                \
+  case LEN:                                                                 \
+    static_assert(Ax2<A, B>::N == LEN, "the radices make another length");  \
+    return f(AxPair<Ax2<A, B>, Ax2<B, A>>{});
+#define GB_RB_THREE(LEN, A, B, C)                                              \
+  case LEN:                                                                    \
+    static_assert(Ax3<A, B, C>::N == LEN, "the radices make another length");  \
+    return f(AxPair<Ax3<A, B, C>, Ax3<C, B, A>>{});
 #define GB_RB_OTHER(N, ...) case N: return 1;
   if constexpr (sizeof(T) == 4) {
     switch (ax.n) {
