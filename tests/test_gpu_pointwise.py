@@ -124,3 +124,77 @@ def test_pointwise_rounding(lib, n2, prec):
     want = vc - k(0.98474502184269654115) * c
     err = ((pot - want) / want).astype(float) / u
     assert np.sqrt((err * err).mean()) <= 1.2
+
+
+@pytest.mark.parametrize("prec", [1, 0])
+@pytest.mark.parametrize("beta", [5 / 6, 0.7])
+@pytest.mark.parametrize("n2", LENGTHS)
+def test_densities_that_are_clamped(lib, n2, beta, prec):
+    """Zero, negative and tiny densities: the terms written out with their clamps.
+
+    Tolerance: a convolution with kernel K of a field x errs below 16 eps log2 N max|K|
+    rms(x); the factors around it and the local terms make a dozen roundings, their
+    products with the convolution included (32 eps of the value).  rho^2 under
+    Thomas-Fermi's cube root loses what lies below the smallest normal FP32 number, and
+    LDA's correlation, 0.19 / den, is lost where den^2 is above the largest one."""
+    import torch
+    nr = (6, 4, n2)
+    plan = _plan(lib, nr, prec)
+    dt = np.float64 if prec else np.float32
+    eps = 2.0 ** -53 if prec else 2.0 ** -24
+    rng = np.random.default_rng(n2)
+    rho = (0.03 + 0.02 * rng.random(nr)).astype(dt)
+    odd = np.array([0.0, -0.0, -1e-3, -1e-31, 1e-31, 5e-31, 1e-30, 2e-30, 1e-24, 1e-12, 1e-7], dtype=dt)
+    where = rng.choice(rho.size, 3 * odd.size, replace=False)
+    rho.reshape(-1)[where] = np.tile(odd, 3)
+    r = rho.astype(float)
+    kz = float(dt(KZ))
+    N, dV = rho.size, 0.4 ** 3
+    log2n = np.log2(N)
+    m = np.meshgrid(*[np.fft.fftfreq(n, 1.0 / n) for n in nr[:2]], np.arange(n2 // 2 + 1), indexing="ij")
+    gg = sum((2 * np.pi * mi / (0.4 * n)) ** 2 for mi, n in zip(m, nr))
+
+    def conv(K, x):
+        return (np.fft.irfftn(K * np.fft.rfftn(x), s=nr, axes=(0, 1, 2)),
+                16 * eps * log2n * np.abs(K).max() * np.sqrt((x * x).mean()))
+
+    def check(f, slot, pot, terms, err):
+        """err: the potential's error at each point, beside 32 eps of its value."""
+        got, en = _eval(lib, plan, f, rho)
+        bound = err + 32 * eps * np.abs(pot) + 1e-37
+        assert (np.abs(got - pot) <= bound).all()
+        assert abs(en[slot] - terms.sum() * dV) <= 2 * (np.abs(r) * bound + 32 * eps * np.abs(terms)).sum() * dV
+
+    f = lib.Functional()
+    f.tf, f.tf_x = 1, 1.0
+    c = np.cbrt(r)
+    check(f, lib.E_TF, 4.78539000031365302657 * c * c, 2.87123400018819181594 * c ** 5,
+          np.full(nr, 0.0 if prec else 5.0 * np.cbrt(2.0 ** -126)))
+    f = lib.Functional()
+    f.vw, f.vw_y = 1, 1.0
+    rm = np.where(r > 0, r, kz)
+    sq = np.sqrt(rm)
+    w, e = conv(gg, sq)
+    v = 0.5 * w / sq
+    check(f, lib.E_VW, v, np.where(r > 0, r * v, 0.0), 0.5 * e / sq)
+    f = lib.Functional()
+    K = 1.0 / (1.0 + gg)
+    kd = torch.tensor(K.astype(dt), device="cuda")
+    f.wt, f.wt_alpha, f.wt_beta, f.wt_kernel = 1, beta, beta, kd.data_ptr()
+    rc = np.where(r < kz, kz, r)
+    kc, e = conv(K.astype(dt).astype(float), rc ** beta)
+    v = 2 * beta * rc ** (beta - 1) * kc
+    # rc^(beta - 1): the exponent's rounding is one of |ln rc| roundings
+    check(f, lib.E_NL, v, v * r / (2 * beta), 2 * beta * rc ** (beta - 1) * e + 70 * eps * np.abs(v))
+    f = lib.Functional()
+    f.xc = 1
+    c = np.maximum(np.cbrt(r), kz)
+    rs = 0.62035049089940001667 / c
+    sq, lr = np.sqrt(rs), np.log(rs)
+    den = 1 + 1.0529 * sq + 0.3334 * rs
+    cx = 0.98474502184269654115
+    low = rs >= 1
+    vx = -cx * c + np.where(low, (-0.1423 - 0.1423 * (7 / 6 * 1.0529 * sq + 4 / 3 * 0.3334 * rs)) / den ** 2,
+                            lr * (0.0311 + 2 / 3 * 0.002 * rs) - 0.048 - 0.0311 / 3 + (2 * -0.0116 - 0.002) * rs / 3)
+    ex = -0.75 * cx * c + np.where(low, -0.1423 / den, 0.0311 * lr - 0.048 + 0.002 * rs * lr - 0.0116 * rs)
+    check(f, lib.E_XC, vx, ex * r, np.full(nr, 0.0 if prec else 0.19 * 2.0 ** -63))
