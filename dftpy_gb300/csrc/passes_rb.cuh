@@ -79,14 +79,6 @@ template <typename T> __host__ __device__ inline int line_pitch(int n) {
 }
 
 // ---- FP64 elementary functions from single-precision seeds -------------------
-// 1/x by two Newton steps (seed error 1e-7 -> 1e-14 -> below 1 ulp)
-__device__ __forceinline__ double rcp_nr(double x) {
-  double r = (double)(1.0f / (float)x);
-  r = fma(r, fma(-x, r, 1.0), r);
-  return fma(r, fma(-x, r, 1.0), r);
-}
-__device__ __forceinline__ float rcp_nr(float x) { return 1.0f / x; }
-
 // x^(-1/6), x in the float range: one third-order (Halley-type) step on the
 // seed, y (1 + r/6 + 7 r^2/72) with r = 1 - x y^6 (|r| < 1e-5, so the next term
 // is below 1e-16)

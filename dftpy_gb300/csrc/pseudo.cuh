@@ -17,25 +17,6 @@ __device__ __forceinline__ double gg_at(const GInfo& g, int m0, int m1, int m2) 
   return gx * gx + gy * gy + gz * gz;
 }
 
-// sqrt(x) and 1/x by Newton steps from single-precision seeds (error 1e-7 -> 1e-14
-// -> rounding): the spectrum kernels are bound by the FP64 pipe, where these are 8
-// and 4 operations (160^3: v_loc 312 -> 271 us a species, force fields 282 -> 254 us)
-__device__ __forceinline__ double sqrt_nr(double x) {
-  const float f = (float)x;
-  if (!(f > 1e-30f && f < 1e30f)) return sqrt(x);
-  double y = (double)rsqrtf(f);
-  y = fma(0.5 * y, fma(-x * y, y, 1.0), y);
-  const double s = x * y;
-  return fma(0.5 * y, fma(-s, s, x), s);
-}
-__device__ __forceinline__ double rcp_nr(double x) {
-  const float f = (float)x;
-  if (!(f > 1e-30f && f < 1e30f)) return 1.0 / x;
-  double r = (double)(1.0f / f);
-  r = fma(r, fma(-x, r, 1.0), r);
-  return fma(r, fma(-x, r, 1.0), r);
-}
-
 struct VTabs {
   gbofdft_vtable t[GBOFDFT_MAX_SPECIES];
   int n;

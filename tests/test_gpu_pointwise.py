@@ -198,3 +198,18 @@ def test_densities_that_are_clamped(lib, n2, beta, prec):
                             lr * (0.0311 + 2 / 3 * 0.002 * rs) - 0.048 - 0.0311 / 3 + (2 * -0.0116 - 0.002) * rs / 3)
     ex = -0.75 * cx * c + np.where(low, -0.1423 / den, 0.0311 * lr - 0.048 + 0.002 * rs * lr - 0.0116 * rs)
     check(f, lib.E_XC, vx, ex * r, np.full(nr, 0.0 if prec else 0.19 * 2.0 ** -63))
+
+
+@pytest.mark.parametrize("power", [-70, -40, 40, 70])
+def test_hartree_of_any_cell_size(lib, power):
+    """The Hartree potential of a cell scaled by s is s^2 times the cell's, also where
+    |G|^2 and its reciprocal leave the FP32 range."""
+    nr = (12, 10, 14)
+    rho = 0.03 + 0.02 * np.random.default_rng(1).random(nr)
+    f = lib.Functional()
+    f.hartree = 1
+    s = 2.0 ** power
+    want = _eval(lib, _plan(lib, nr, 1), f, rho, energies=False)[0] * s * s
+    plan = lib.Plan(nr, np.diag([0.4 * s * k for k in nr]), precision=1)
+    got = _eval(lib, plan, f, rho, energies=False)[0]
+    assert np.abs(got - want).max() <= 1e-13 * np.abs(want).max()
