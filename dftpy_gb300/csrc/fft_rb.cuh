@@ -8,7 +8,7 @@
 // the host (RbAxis) and selected in the kernel by a branch that is uniform
 // over the CTA, so one kernel serves every length.
 //
-// Composite radices whose factors are coprime (6, 10, 12, 14, 15, 18, 20) use
+// Composite radices whose factors are coprime (6, 10, 12, 14, 15) use
 // the Good-Thomas prime-factor index maps: no twiddle factors inside.
 //
 // Stage s (radix r, p = product of the radices before it), butterfly i in
@@ -213,8 +213,6 @@ __device__ __forceinline__ void dft(cpx<T>* u) {
   else if constexpr (R == 14) dft_pfa<DIR, T, 2, 7>(u);
   else if constexpr (R == 15) dft_pfa<DIR, T, 3, 5>(u);
   else if constexpr (R == 16) dft16<DIR, T>(u);
-  else if constexpr (R == 18) dft_pfa<DIR, T, 2, 9>(u);
-  else if constexpr (R == 20) dft_pfa<DIR, T, 4, 5>(u);
   else static_assert(R == 2, "radix not implemented");
 }
 
@@ -230,7 +228,8 @@ __device__ __forceinline__ void dft(cpx<T>* u) {
 // large as their variation, every partial sum carries it, its rounding is the
 // noise of all high-G coefficients, and the G^2 kernel makes that noise the
 // error of the potential.  A length's radices therefore stay what they are
-// (8, 4, 2, 3, 5, 7 from large to small, with the exceptions in rb_axis).
+// (8, 4, 2, 3, 5, 7; the lists of passes_rb.cuh have 128 as 8, 4, 4 and 360 as
+// 8, 5, 3, 3).
 template <int R_> struct Pfa { static constexpr int R = R_; };
 template <int Q, int... Qs> struct Rad {
   static constexpr int R = Q * Rad<Qs...>::R;
@@ -260,7 +259,9 @@ __device__ __forceinline__ float2 tw_mul(float2 a, float2 b) {
 }
 
 // Radix 7 as the plain sum over its inputs in order, the stage's twiddle (step
-// e) and the DFT's (step n / 7) looked up together
+// e) and the DFT's (step n / 7) looked up together.  Forward transforms keep it with
+// their radices, for the rounding of the mean; inverse ones take the cheaper codelet,
+// since nothing amplifies their rounding.
 template <int DIR, typename T>
 __device__ __forceinline__ void dft7_direct(cpx<T>* u, const cpx<T>* __restrict__ tw, int e, int n) {
   cpx<T> o[7];
@@ -284,7 +285,7 @@ __device__ __forceinline__ void dft7_direct(cpx<T>* u, const cpx<T>* __restrict_
 template <int DIR, typename T, bool ONE, int Q, int... Qs>
 __device__ __forceinline__ void rad_dft(Rad<Q, Qs...>, cpx<T>* u, const cpx<T>* __restrict__ tw, int k, int p, int n) {
   constexpr int M = Rad<Q, Qs...>::R / Q;
-  if constexpr (Q == 7 && M == 1 && DIR < 0) {   // (inverse inputs carry no mean)
+  if constexpr (Q == 7 && M == 1 && DIR < 0) {
     dft7_direct<DIR, T>(u, tw, ONE ? 0 : k * (n / (p * Q)), n);
     return;
   }

@@ -1,7 +1,8 @@
-// Row passes of compile-time length for the plane pipeline (plane-major
-// spectra) and the delta evaluations, for the grid sizes of the workloads; a
-// launcher returns 1 when the size has no specialisation, 0 on success, or an
-// error.
+// FP32 row passes of compile-time length for the plane pipeline and the delta
+// evaluations, for the grid sizes of the workloads; a launcher returns 1 when the
+// size has no specialisation, 0 on success, or an error.  Spectra are plane-major:
+// element k2 of row r at k2 * nrows + r, consecutive threads on consecutive rows of
+// one k2.
 #pragma once
 #include <math.h>
 #include <string.h>
@@ -39,27 +40,25 @@ __host__ inline bool ct_dispatch(int n, F&& f) {
 #define GB_CT_PF_F32 4      // density / v_loc values prefetched per thread in the FP32 evaluation epilogue (measured best)
 #endif
 
-template <typename T> struct RowsCfg;            // row pairs per CTA (per field)
-template <> struct RowsCfg<float> { static constexpr int RP = GB_CT_RP_F32; };
-template <> struct RowsCfg<double> { static constexpr int RP = 4; };
+constexpr int kRowPairs = GB_CT_RP_F32;         // row pairs per CTA (per field)
 // threads of a row-pass CTA: TPL per line, one line per (field, row pair)
-template <typename T, int N> constexpr int rows_threads_max() { return Tpl<N>::value * RowsCfg<T>::RP * GB_MAX_FIELDS; }
+template <int N> constexpr int rows_threads_max() { return Tpl<N>::value * kRowPairs * GB_MAX_FIELDS; }
+
 // ---- pointwise functions -----------------------------------------------------
 // x^(1/2), x^(5/6) and friends for x >= 1e-30 (the reference's clamps)
-template <typename T> __device__ __forceinline__ T sqrt_pos(T x) { return x * rsqrt_d(x); }
+__device__ __forceinline__ float sqrt_pos(float x) { return x * rsqrtf(x); }
 
-template <typename T> __device__ __forceinline__ T pow_beta_ct(T x, bool b56, T beta) {
+__device__ __forceinline__ float pow_beta_ct(float x, bool b56, float beta) {
   if (b56) {
-    const T z3 = rcbrt_d(x), z2 = rsqrt_d(x);
+    const float z3 = rcbrtf(x), z2 = rsqrtf(x);
     return (x * z2) * (x * z3 * z3);         // x^(1/2) x^(1/3)
   }
-  return pow(x, beta);
+  return powf(x, beta);
 }
 
-template <typename T>
-__device__ __forceinline__ T prologue_ct(int op, T rho, bool b56, T beta) {
-  if (op == OP_SQRT) return sqrt_pos<T>(rho > (T)0 ? rho : (T)kZero);
-  if (op == OP_POWB) return pow_beta_ct<T>(rho < (T)kZero ? (T)kZero : rho, b56, beta);
+__device__ __forceinline__ float prologue_ct(int op, float rho, bool b56, float beta) {
+  if (op == OP_SQRT) return sqrt_pos(rho > 0.0f ? rho : (float)kZero);
+  if (op == OP_POWB) return pow_beta_ct(rho < (float)kZero ? (float)kZero : rho, b56, beta);
   return rho;
 }
 
@@ -70,39 +69,37 @@ struct CtRowsFwd {
   const void* in;
   void* out;
   int64_t fstride;
-  int nrows, ld2, nf;
+  int nrows, nf;
   int op[GB_MAX_FIELDS];
   int b56;            // beta == 5/6
-  Sc beta, half;      // half = scale / 2
+  Sc beta;
   const void* tw;
 };
 
-// PM: write plane-major spectra (k2 * nrows + row) for the plane pass;
-// consecutive threads then take consecutive rows of one k2.
-template <typename T, int N, bool PM>
-__global__ void __launch_bounds__(rows_threads_max<T, N>(), GB_CT_ROWS_MINB) k_ct_rows_fwd(CtRowsFwd a) {
-  constexpr int RP = RowsCfg<T>::RP, TPL = Tpl<N>::value, NP = Pad<T, N>::NP, NH = N / 2 + 1;
+template <int N>
+__global__ void __launch_bounds__(rows_threads_max<N>(), GB_CT_ROWS_MINB) k_ct_rows_fwd(CtRowsFwd a) {
+  constexpr int RP = kRowPairs, TPL = Tpl<N>::value, NP = Pad<float, N>::NP, NH = N / 2 + 1;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int nl = a.nf * RP;
-  cpx<T>* tw = reinterpret_cast<cpx<T>*>(smem_raw);
-  cpx<T>* A = tw + N;
-  cpx<T>* B = A + nl * NP;
-  T* R = reinterpret_cast<T*>(B + nl * NP);      // [2 RP][N] real input rows
+  cpx<float>* tw = reinterpret_cast<cpx<float>*>(smem_raw);
+  cpx<float>* A = tw + N;
+  cpx<float>* B = A + nl * NP;
+  float* R = reinterpret_cast<float*>(B + nl * NP);      // [2 RP][N] real input rows
   const int tid = threadIdx.x, l = tid / TPL, lane = tid % TPL;
   const int64_t base = (int64_t)blockIdx.x * 2 * RP;
-  const cpx<T>* twg = reinterpret_cast<const cpx<T>*>(a.tw);
+  const cpx<float>* twg = reinterpret_cast<const cpx<float>*>(a.tw);
   for (int i = tid; i < N; i += blockDim.x) tw[i] = twg[i];
-  const T* in = reinterpret_cast<const T*>(a.in);
+  const float* in = reinterpret_cast<const float*>(a.in);
   // input rows: batches of independent loads ahead of their stores
   constexpr int NE = 2 * RP * N, UNR = 4;
 #pragma unroll 1
   for (int b0 = 0; b0 < NE; b0 += UNR * (int)blockDim.x) {
-    T v[UNR];
+    float v[UNR];
 #pragma unroll
     for (int u = 0; u < UNR; ++u) {
       const int idx = b0 + u * (int)blockDim.x + tid;
       const int64_t row = base + idx / N;
-      v[u] = (idx < NE && row < a.nrows) ? __ldg(in + row * N + idx % N) : (T)0;
+      v[u] = (idx < NE && row < a.nrows) ? __ldg(in + row * N + idx % N) : 0.0f;
     }
 #pragma unroll
     for (int u = 0; u < UNR; ++u) {
@@ -112,7 +109,7 @@ __global__ void __launch_bounds__(rows_threads_max<T, N>(), GB_CT_ROWS_MINB) k_c
   }
   __syncthreads();
   const bool b56 = a.b56 != 0;
-  const T beta = sc<T>(a.beta);
+  const float beta = sc<float>(a.beta);
   // fields in an unrolled outer loop: the field's prologue op is a
   // compile-time parameter index, and every index split below is by a
   // compile-time constant
@@ -123,31 +120,28 @@ __global__ void __launch_bounds__(rows_threads_max<T, N>(), GB_CT_ROWS_MINB) k_c
     for (int idx = tid; idx < RP * N; idx += blockDim.x) {
       const int l2 = idx / N, j = idx % N;
       const int64_t ra = base + 2 * l2;
-      const T x0 = ra < a.nrows ? prologue_ct<T>(op, R[(2 * l2) * N + j], b56, beta) : (T)0;
-      const T x1 = ra + 1 < a.nrows ? prologue_ct<T>(op, R[(2 * l2 + 1) * N + j], b56, beta) : (T)0;
-      A[sw<T, NP>(f * RP + l2, j)] = cpx<T>{x0, x1};
+      const float x0 = ra < a.nrows ? prologue_ct(op, R[(2 * l2) * N + j], b56, beta) : 0.0f;
+      const float x1 = ra + 1 < a.nrows ? prologue_ct(op, R[(2 * l2 + 1) * N + j], b56, beta) : 0.0f;
+      A[sw<float, NP>(f * RP + l2, j)] = cpx<float>{x0, x1};
     }
   }
   __syncthreads();
-  cpx<T>* res = fft<-1, T, N>(A, B, tw, l, lane, true);
-  cpx<T>* out = reinterpret_cast<cpx<T>*>(a.out);
-  const T half = sc<T>(a.half);
+  cpx<float>* res = fft<-1, float, N>(A, B, tw, l, lane, true);
+  cpx<float>* out = reinterpret_cast<cpx<float>*>(a.out);
 #pragma unroll
   for (int f = 0; f < GB_MAX_FIELDS; ++f) {
     if (f >= a.nf) break;
-    cpx<T>* o = out + f * a.fstride;
+    cpx<float>* o = out + f * a.fstride;
     for (int idx = tid; idx < RP * NH; idx += blockDim.x) {
-      // plane-major: consecutive threads take consecutive row pairs of one k
-      const int l2 = PM ? idx % RP : idx / NH, k = PM ? idx / RP : idx % NH;
+      const int l2 = idx % RP, k = idx / RP;
       const int line = f * RP + l2;
       const int64_t ra = base + 2 * l2, rb = ra + 1;
       if (ra >= a.nrows) continue;
-      const cpx<T> Z = res[sw<T, NP>(line, k)];
-      const cpx<T> Zc = res[sw<T, NP>(line, k == 0 ? 0 : N - k)];
-      const int64_t ia = PM ? (int64_t)k * a.nrows + ra : ra * a.ld2 + k;
-      const int64_t ib = PM ? ia + 1 : ia + a.ld2;
-      o[ia] = cpx<T>{(Z.x + Zc.x) * half, (Z.y - Zc.y) * half};
-      if (rb < a.nrows) o[ib] = cpx<T>{(Z.y + Zc.y) * half, (Zc.x - Z.x) * half};
+      const cpx<float> Z = res[sw<float, NP>(line, k)];
+      const cpx<float> Zc = res[sw<float, NP>(line, k == 0 ? 0 : N - k)];
+      const int64_t ia = (int64_t)k * a.nrows + ra;
+      o[ia] = cpx<float>{(Z.x + Zc.x) * 0.5f, (Z.y - Zc.y) * 0.5f};
+      if (rb < a.nrows) o[ia + 1] = cpx<float>{(Z.y + Zc.y) * 0.5f, (Zc.x - Z.x) * 0.5f};
     }
   }
 }
@@ -156,11 +150,10 @@ __global__ void __launch_bounds__(rows_threads_max<T, N>(), GB_CT_ROWS_MINB) k_c
 struct CtRowsInv {
   const void* in;
   int64_t fstride;
-  int nrows, ld2, nf;
+  int nrows, nf;
   const void* tw;
   void* out;
   int64_t ostride;
-  Sc scale;
   EvalDesc ev;
   Sc tf_v, tf_e, vw_y, two_alpha, inv_two_alpha, wt_beta;  // evaluation constants
   int b56;
@@ -173,57 +166,55 @@ struct CtRowsInv {
 
 // irfftn line build (all fields) + inverse FFT; result line (f * RP + pair)
 // holds row 2 pair in .x and row 2 pair + 1 in .y.
-template <typename T, int N, bool PM = false, int NFMAX = GB_MAX_FIELDS>
-__device__ __forceinline__ cpx<T>* ct_rows_inv_lines(const CtRowsInv& a, int64_t base, cpx<T>* tw, cpx<T>* A,
-                                                     cpx<T>* B) {
-  constexpr int RP = RowsCfg<T>::RP, TPL = Tpl<N>::value, NP = Pad<T, N>::NP, NH = N / 2 + 1;
+template <int N>
+__device__ __forceinline__ cpx<float>* ct_rows_inv_lines(const CtRowsInv& a, int64_t base, cpx<float>* tw,
+                                                         cpx<float>* A, cpx<float>* B) {
+  constexpr int RP = kRowPairs, TPL = Tpl<N>::value, NP = Pad<float, N>::NP, NH = N / 2 + 1;
   const int tid = threadIdx.x, l = tid / TPL, lane = tid % TPL;
   const int nl = a.nf * RP;
-  const cpx<T>* src0 = reinterpret_cast<const cpx<T>*>(a.in);
+  const cpx<float>* src0 = reinterpret_cast<const cpx<float>*>(a.in);
 #pragma unroll
-  for (int f = 0; f < NFMAX; ++f) {
+  for (int f = 0; f < GB_MAX_FIELDS; ++f) {
     if (f >= a.nf) break;
-    const cpx<T>* src = src0 + f * a.fstride;
+    const cpx<float>* src = src0 + f * a.fstride;
     for (int idx = tid; idx < RP * NH; idx += blockDim.x) {
-      const int l2 = PM ? idx % RP : idx / NH, k = PM ? idx / RP : idx % NH;
+      const int l2 = idx % RP, k = idx / RP;
       const int line = f * RP + l2;
       const int64_t ra = base + 2 * l2, rb = ra + 1;
-      const int64_t ia = PM ? (int64_t)k * a.nrows + ra : ra * a.ld2 + k;
-      const int64_t ib = PM ? ia + 1 : ia + a.ld2;
-      cpx<T> va = {(T)0, (T)0}, vb = {(T)0, (T)0};
+      const int64_t ia = (int64_t)k * a.nrows + ra;
+      cpx<float> va = {0.0f, 0.0f}, vb = {0.0f, 0.0f};
       if (ra < a.nrows) va = src[ia];
-      if (rb < a.nrows) vb = src[ib];
-      if (k == 0 || 2 * k == N) { va.y = (T)0; vb.y = (T)0; }
-      A[sw<T, NP>(line, k)] = cpx<T>{va.x - vb.y, va.y + vb.x};
-      if (k > 0 && 2 * k < N) A[sw<T, NP>(line, N - k)] = cpx<T>{va.x + vb.y, vb.x - va.y};
+      if (rb < a.nrows) vb = src[ia + 1];
+      if (k == 0 || 2 * k == N) { va.y = 0.0f; vb.y = 0.0f; }
+      A[sw<float, NP>(line, k)] = cpx<float>{va.x - vb.y, va.y + vb.x};
+      if (k > 0 && 2 * k < N) A[sw<float, NP>(line, N - k)] = cpx<float>{va.x + vb.y, vb.x - va.y};
     }
   }
   __syncthreads();
-  return fft<1, T, N>(A, B, tw, l, lane, true);
+  return fft<1, float, N>(A, B, tw, l, lane, true);
 }
 
-template <typename T, int N, bool PM = false>
-__global__ void __launch_bounds__(rows_threads_max<T, N>()) k_ct_rows_inv_store(CtRowsInv a) {
-  constexpr int RP = RowsCfg<T>::RP, NP = Pad<T, N>::NP;
+template <int N>
+__global__ void __launch_bounds__(rows_threads_max<N>()) k_ct_rows_inv_store(CtRowsInv a) {
+  constexpr int RP = kRowPairs, NP = Pad<float, N>::NP;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int nl = a.nf * RP;
-  cpx<T>* tw = reinterpret_cast<cpx<T>*>(smem_raw);
-  cpx<T>* A = tw + N;
-  cpx<T>* B = A + nl * NP;
+  cpx<float>* tw = reinterpret_cast<cpx<float>*>(smem_raw);
+  cpx<float>* A = tw + N;
+  cpx<float>* B = A + nl * NP;
   const int tid = threadIdx.x;
   const int64_t base = (int64_t)blockIdx.x * 2 * RP;
-  const cpx<T>* twg = reinterpret_cast<const cpx<T>*>(a.tw);
+  const cpx<float>* twg = reinterpret_cast<const cpx<float>*>(a.tw);
   for (int i = tid; i < N; i += blockDim.x) tw[i] = twg[i];
-  cpx<T>* res = ct_rows_inv_lines<T, N, PM>(a, base, tw, A, B);
-  T* out = reinterpret_cast<T*>(a.out);
-  const T s = sc<T>(a.scale);
+  cpx<float>* res = ct_rows_inv_lines<N>(a, base, tw, A, B);
+  float* out = reinterpret_cast<float*>(a.out);
   for (int idx = tid; idx < a.nf * 2 * RP * N; idx += blockDim.x) {
     const int f = idx / (2 * RP * N), r = idx % (2 * RP * N);
     const int rr = r / N, j = r % N;
     const int64_t row = base + rr;
     if (row >= a.nrows) continue;
-    const cpx<T> z = res[sw<T, NP>(f * RP + (rr >> 1), j)];
-    out[f * a.ostride + row * N + j] = ((rr & 1) ? z.y : z.x) * s;
+    const cpx<float> z = res[sw<float, NP>(f * RP + (rr >> 1), j)];
+    out[f * a.ostride + row * N + j] = (rr & 1) ? z.y : z.x;
   }
 }
 
@@ -259,116 +250,110 @@ __device__ __forceinline__ void pz_lda_ct(T rho, T& eps, T& pot, bool want_e) {
 // WANT_E is a template parameter so the potential-only instantiation holds no
 // FP64 accumulation at all (if-converted, never-taken FP64 code still
 // occupies the FP64 pipe).
-template <typename T, int N, bool WANT_E, bool PM = false>
-__global__ void __launch_bounds__(rows_threads_max<T, N>(), GB_CT_ROWS_MINB) k_ct_rows_inv_eval(CtRowsInv a) {
-  constexpr int RP = RowsCfg<T>::RP, NP = Pad<T, N>::NP;
+template <int N, bool WANT_E>
+__global__ void __launch_bounds__(rows_threads_max<N>(), GB_CT_ROWS_MINB) k_ct_rows_inv_eval(CtRowsInv a) {
+  constexpr int RP = kRowPairs, NP = Pad<float, N>::NP;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int nl = (a.nf > 0 ? a.nf : 1) * RP;
-  cpx<T>* tw = reinterpret_cast<cpx<T>*>(smem_raw);
-  cpx<T>* A = tw + N;
-  cpx<T>* B = A + nl * NP;
+  cpx<float>* tw = reinterpret_cast<cpx<float>*>(smem_raw);
+  cpx<float>* A = tw + N;
+  cpx<float>* B = A + nl * NP;
   const int tid = threadIdx.x;
   const int64_t base = (int64_t)blockIdx.x * 2 * RP;
-  const cpx<T>* twg = reinterpret_cast<const cpx<T>*>(a.tw);
+  const cpx<float>* twg = reinterpret_cast<const cpx<float>*>(a.tw);
   for (int i = tid; i < N; i += blockDim.x) tw[i] = twg[i];
   const EvalDesc& ev = a.ev;
-  const T* rhop = reinterpret_cast<const T*>(a.rho);
-  const T* vlocp = reinterpret_cast<const T*>(a.vloc);
+  const float* rhop = reinterpret_cast<const float*>(a.rho);
+  const float* vlocp = reinterpret_cast<const float*>(a.vloc);
   // the density and v_loc of this thread's first PF elements, loaded before
   // the transforms so their latency is hidden behind them
-  constexpr int PF = sizeof(T) == 4 ? GB_CT_PF_F32 : 4;
-  T pre_rho[PF], pre_vl[PF];
+  constexpr int PF = GB_CT_PF_F32;
+  float pre_rho[PF], pre_vl[PF];
 #pragma unroll
   for (int m = 0; m < PF; ++m) {
     const int idx = tid + m * (int)blockDim.x;
     const int64_t row = base + idx / N;
     const bool ok = idx < 2 * RP * N && row < a.nrows;
     const int64_t gidx = row * N + idx % N;
-    pre_rho[m] = ok ? __ldg(rhop + gidx) : (T)0;
-    pre_vl[m] = (ok && ev.pp) ? __ldg(vlocp + gidx) : (T)0;
+    pre_rho[m] = ok ? __ldg(rhop + gidx) : 0.0f;
+    pre_vl[m] = (ok && ev.pp) ? __ldg(vlocp + gidx) : 0.0f;
   }
-  cpx<T>* res = A;
-  if (a.nf > 0) res = ct_rows_inv_lines<T, N, PM>(a, base, tw, A, B);
-  T* potp = reinterpret_cast<T*>(a.pot);
+  cpx<float>* res = A;
+  if (a.nf > 0) res = ct_rows_inv_lines<N>(a, base, tw, A, B);
+  float* potp = reinterpret_cast<float*>(a.pot);
   constexpr bool want_e = WANT_E;
-  const T tf_v = sc<T>(a.tf_v);             // (5/3) C_TF x
-  const T tf_e = sc<T>(a.tf_e);             // C_TF x
-  const T vw_y = sc<T>(a.vw_y);
-  const T two_alpha = sc<T>(a.two_alpha);
-  const T inv_two_alpha = sc<T>(a.inv_two_alpha);
-  const T wt_beta = sc<T>(a.wt_beta);
+  const float tf_v = sc<float>(a.tf_v);             // (5/3) C_TF x
+  const float tf_e = sc<float>(a.tf_e);             // C_TF x
+  const float vw_y = sc<float>(a.vw_y);
+  const float two_alpha = sc<float>(a.two_alpha);
+  const float inv_two_alpha = sc<float>(a.inv_two_alpha);
+  const float wt_beta = sc<float>(a.wt_beta);
   const bool b56 = a.b56 != 0;
   // per-thread energy sums in the field precision (a handful of elements per
   // thread); combined in FP64 across threads and CTAs
-  T es[6] = {0, 0, 0, 0, 0, 0};
-  // FP64 only: optional copy of the convolution results (delta-evaluation reference)
-  T* coutp = nullptr;
-  if constexpr (sizeof(T) == 8) coutp = reinterpret_cast<T*>(ev.cout);
-  auto point = [&](int idx, T rho, T vl_pre) {
+  float es[6] = {0, 0, 0, 0, 0, 0};
+  auto point = [&](int idx, float rho, float vl_pre) {
     const int rr = idx / N, j = idx % N;
     const int64_t row = base + rr;
     if (row >= a.nrows) return;
     const int64_t gidx = row * N + j;
     const int pr = rr >> 1;
     const bool odd = rr & 1;
-    const bool pos = rho > (T)kZero;
+    const bool pos = rho > (float)kZero;
     // rho^(-1/3) and rho^(-1/2) for positive densities (shared by TF, vW, WT)
-    T z3 = (T)0, z2 = (T)0;
+    float z3 = 0.0f, z2 = 0.0f;
     if (pos) { z3 = rcbrt_d(rho); z2 = rsqrt_d(rho); }
-    T pot = (T)0;
+    float pot = 0.0f;
     if (ev.tf) {
-      T r23;                                              // cbrt(rho^2)
+      float r23;                                              // cbrt(rho^2)
       if (pos) r23 = rho * z3;
       else r23 = cbrt(rho * rho);
       pot += tf_v * r23;
       if (want_e) {
-        T r53;                                            // cbrt(rho^5)
+        float r53;                                            // cbrt(rho^5)
         if (pos) r53 = rho * rho * z3;
-        else { T r5 = rho * rho; r5 = r5 * rho; r5 = r5 * rho; r5 = r5 * rho; r53 = cbrt(r5); }
+        else { float r5 = rho * rho; r5 = r5 * rho; r5 = r5 * rho; r5 = r5 * rho; r53 = cbrt(r5); }
         es[0] += r53 * tf_e;
       }
     }
     if (ev.vw) {
-      const cpx<T> zz = res[sw<T, NP>(ev.slot_vw * RP + pr, j)];
-      const T w = odd ? zz.y : zz.x;
-      if constexpr (sizeof(T) == 8) if (coutp) coutp[ev.slot_vw * ev.cstride + gidx] = w;
+      const cpx<float> zz = res[sw<float, NP>(ev.slot_vw * RP + pr, j)];
+      const float w = odd ? zz.y : zz.x;
       // 1 / max(sqrt(rho_m), 1e-30), rho_m = rho if rho > 0 else 1e-30
-      const T inv_sq = pos ? z2 : (rho > (T)0 ? (T)1 / fmax(sqrt(rho), (T)kZero) : (T)1e15);
-      const T v = (T)0.5 * w * inv_sq;
+      const float inv_sq = pos ? z2 : (rho > 0.0f ? 1.0f / fmax(sqrt(rho), (float)kZero) : 1e15f);
+      const float v = 0.5f * w * inv_sq;
       pot += v * vw_y;
-      if (want_e && rho > (T)0) es[1] += rho * v * vw_y;
+      if (want_e && rho > 0.0f) es[1] += rho * v * vw_y;
     }
     if (ev.wt) {
-      const cpx<T> zz = res[sw<T, NP>(ev.slot_wt * RP + pr, j)];
-      const T kc = odd ? zz.y : zz.x;
-      if constexpr (sizeof(T) == 8) if (coutp) coutp[ev.slot_wt * ev.cstride + gidx] = kc;
-      T rb_over_rc;                                       // rc^(beta - 1), rc = max(rho, 1e-30)
+      const cpx<float> zz = res[sw<float, NP>(ev.slot_wt * RP + pr, j)];
+      const float kc = odd ? zz.y : zz.x;
+      float rb_over_rc;                                       // rc^(beta - 1), rc = max(rho, 1e-30)
       if (b56) {
         if (pos) rb_over_rc = rho * z3 * z3 * z2;          // rho^(1/3) rho^(-1/2)
-        else { const T rc = (T)kZero; rb_over_rc = sqrt(rc) * cbrt(rc) / rc; }
+        else { const float rc = (float)kZero; rb_over_rc = sqrt(rc) * cbrt(rc) / rc; }
       } else {
-        const T rc = rho < (T)kZero ? (T)kZero : rho;
+        const float rc = rho < (float)kZero ? (float)kZero : rho;
         rb_over_rc = pow(rc, wt_beta) / rc;
       }
-      const T v = two_alpha * rb_over_rc * kc;
+      const float v = two_alpha * rb_over_rc * kc;
       pot += v;
       if (want_e) es[2] += v * rho * inv_two_alpha;
     }
     if (ev.xc) {
-      T eps, vx;
-      pz_lda_ct<T>(rho, eps, vx, want_e);
+      float eps, vx;
+      pz_lda_ct<float>(rho, eps, vx, want_e);
       pot += vx;
       if (want_e) es[3] += eps * rho;
     }
     if (ev.hartree) {
-      const cpx<T> zz = res[sw<T, NP>(ev.slot_h * RP + pr, j)];
-      const T vh = odd ? zz.y : zz.x;
-      if constexpr (sizeof(T) == 8) if (coutp) coutp[ev.slot_h * ev.cstride + gidx] = vh;
+      const cpx<float> zz = res[sw<float, NP>(ev.slot_h * RP + pr, j)];
+      const float vh = odd ? zz.y : zz.x;
       pot += vh;
-      if (want_e) es[4] += (T)0.5 * vh * rho;
+      if (want_e) es[4] += 0.5f * vh * rho;
     }
     if (ev.pp) {
-      const T vl = vl_pre;
+      const float vl = vl_pre;
       pot += vl;
       if (want_e) es[5] += vl * rho;
     }
@@ -379,7 +364,7 @@ __global__ void __launch_bounds__(rows_threads_max<T, N>(), GB_CT_ROWS_MINB) k_c
   // prefetch registers
 #pragma unroll 1
   for (int m = 0, idx = tid; idx < 2 * RP * N; ++m, idx += blockDim.x) {
-    T rho, vl;
+    float rho, vl;
     if (m < PF) {
 #pragma unroll
       for (int q = 0; q < PF; ++q)
@@ -389,7 +374,7 @@ __global__ void __launch_bounds__(rows_threads_max<T, N>(), GB_CT_ROWS_MINB) k_c
       if (row >= a.nrows) continue;
       const int64_t gidx = row * N + idx % N;
       rho = __ldg(rhop + gidx);
-      vl = ev.pp ? __ldg(vlocp + gidx) : (T)0;
+      vl = ev.pp ? __ldg(vlocp + gidx) : 0.0f;
     }
     point(idx, rho, vl);
   }
@@ -413,30 +398,28 @@ __global__ void __launch_bounds__(rows_threads_max<T, N>(), GB_CT_ROWS_MINB) k_c
 
 // reciprocal-space kernel value, out of line
 template <typename T>
-__device__ __noinline__ T kernel_value_slow(const GInfo& g, int type, const void* arr, int i0, int i1, int k2) {
+__device__ __noinline__ float kernel_value_slow(const GInfo& g, int type, const void* arr, int i0, int i1, int k2) {
   return gbk::kernel_value<T>(g, type, arr, i0, i1, k2);
 }
 
 // ---- launchers -------------------------------------------------------------------
-template <typename T, bool PM = false>
-int ct_rows_fwd(gbofdft_plan* p, const void* in, void* spec, int64_t fstride, int ld2, int nf, const int* ops,
-                double beta, double scale, cudaStream_t st) {
+inline int ct_rows_fwd(gbofdft_plan* p, const void* in, void* spec, int64_t fstride, int nf, const int* ops, double beta,
+                       cudaStream_t st) {
   int rc = 1;
   ct_dispatch(p->n[2], [&](auto nc) {
     constexpr int N = decltype(nc)::value;
-    constexpr int RP = RowsCfg<T>::RP, NP = Pad<T, N>::NP;
+    constexpr int RP = kRowPairs, NP = Pad<float, N>::NP;
     CtRowsFwd a;
     a.in = in; a.out = spec; a.fstride = fstride;
-    a.nrows = p->n[0] * p->n[1]; a.ld2 = ld2; a.nf = nf;
+    a.nrows = p->n[0] * p->n[1]; a.nf = nf;
     for (int f = 0; f < GB_MAX_FIELDS; ++f) a.op[f] = f < nf ? ops[f] : OP_RHO;
     a.b56 = fabs(beta - 5.0 / 6.0) < 1e-15;
     a.beta.set(beta);
-    a.half.set(0.5 * scale);
     a.tw = p->tw[2];
-    const size_t sm = sizeof(cpx<T>) * (N + 2 * (size_t)nf * RP * NP) + sizeof(T) * 2 * RP * N;
-    if ((rc = ct_smem(k_ct_rows_fwd<T, N, PM>, sm))) return;
+    const size_t sm = sizeof(cpx<float>) * (N + 2 * (size_t)nf * RP * NP) + sizeof(float) * 2 * RP * N;
+    if ((rc = ct_smem(k_ct_rows_fwd<N>, sm))) return;
     const int nblk = (a.nrows + 2 * RP - 1) / (2 * RP);
-    k_ct_rows_fwd<T, N, PM><<<nblk, Tpl<N>::value * RP * nf, sm, st>>>(a);
+    k_ct_rows_fwd<N><<<nblk, Tpl<N>::value * RP * nf, sm, st>>>(a);
     gb_count_launch();
     cudaError_t e = cudaGetLastError();
     rc = e == cudaSuccess ? 0 : gb_set_error(GBOFDFT_ERR_CUDA, "ct_rows_fwd: %s", cudaGetErrorString(e));
@@ -444,18 +427,17 @@ int ct_rows_fwd(gbofdft_plan* p, const void* in, void* spec, int64_t fstride, in
   return rc;
 }
 
-template <typename T, bool PM = false>
-int ct_rows_inv(gbofdft_plan* p, const void* spec, int64_t fstride, int ld2, int nf, void* out, int64_t ostride,
-                double scale, const EvalDesc* ev, const void* rho, const void* vloc, void* pot, int calc_e,
-                double* partials, int64_t* nblk_out, cudaStream_t st) {
+inline int ct_rows_inv(gbofdft_plan* p, const void* spec, int64_t fstride, int nf, void* out, int64_t ostride,
+                       const EvalDesc* ev, const void* rho, const void* vloc, void* pot, int calc_e,
+                       double* partials, int64_t* nblk_out, cudaStream_t st) {
   int rc = 1;
   ct_dispatch(p->n[2], [&](auto nc) {
     constexpr int N = decltype(nc)::value;
-    constexpr int RP = RowsCfg<T>::RP, NP = Pad<T, N>::NP;
+    constexpr int RP = kRowPairs, NP = Pad<float, N>::NP;
     CtRowsInv a;
     memset(&a, 0, sizeof(a));
-    a.in = spec; a.fstride = fstride; a.nrows = p->n[0] * p->n[1]; a.ld2 = ld2; a.nf = nf; a.tw = p->tw[2];
-    a.out = out; a.ostride = ostride; a.scale.set(scale);
+    a.in = spec; a.fstride = fstride; a.nrows = p->n[0] * p->n[1]; a.nf = nf; a.tw = p->tw[2];
+    a.out = out; a.ostride = ostride;
     const int nblk = (a.nrows + 2 * RP - 1) / (2 * RP);
     if (nblk_out) *nblk_out = nblk;
     if (ev) {
@@ -469,22 +451,18 @@ int ct_rows_inv(gbofdft_plan* p, const void* spec, int64_t fstride, int ld2, int
       a.wt_beta.set(ev->wt_beta);
       a.b56 = fabs(ev->wt_beta - 5.0 / 6.0) < 1e-15;
       const int nfl = nf > 0 ? nf : 1;
-      const size_t sm = sizeof(cpx<T>) * (N + 2 * (size_t)nfl * RP * NP);
+      const size_t sm = sizeof(cpx<float>) * (N + 2 * (size_t)nfl * RP * NP);
       if (calc_e) {
-        if ((rc = ct_smem(k_ct_rows_inv_eval<T, N, true, PM>, sm))) return;
-        k_ct_rows_inv_eval<T, N, true, PM><<<nblk, Tpl<N>::value * RP * nfl, sm, st>>>(a);
+        if ((rc = ct_smem(k_ct_rows_inv_eval<N, true>, sm))) return;
+        k_ct_rows_inv_eval<N, true><<<nblk, Tpl<N>::value * RP * nfl, sm, st>>>(a);
       } else {
-        if ((rc = ct_smem(k_ct_rows_inv_eval<T, N, false, PM>, sm))) return;
-        k_ct_rows_inv_eval<T, N, false, PM><<<nblk, Tpl<N>::value * RP * nfl, sm, st>>>(a);
+        if ((rc = ct_smem(k_ct_rows_inv_eval<N, false>, sm))) return;
+        k_ct_rows_inv_eval<N, false><<<nblk, Tpl<N>::value * RP * nfl, sm, st>>>(a);
       }
-    } else if constexpr (PM) {
-      const size_t sm = sizeof(cpx<T>) * (N + 2 * (size_t)nf * RP * NP);
-      if ((rc = ct_smem(k_ct_rows_inv_store<T, N, true>, sm))) return;
-      k_ct_rows_inv_store<T, N, true><<<nblk, Tpl<N>::value * RP * nf, sm, st>>>(a);
     } else {
-      const size_t sm = sizeof(cpx<T>) * (N + 2 * (size_t)nf * RP * NP);
-      if ((rc = ct_smem(k_ct_rows_inv_store<T, N>, sm))) return;
-      k_ct_rows_inv_store<T, N><<<nblk, Tpl<N>::value * RP * nf, sm, st>>>(a);
+      const size_t sm = sizeof(cpx<float>) * (N + 2 * (size_t)nf * RP * NP);
+      if ((rc = ct_smem(k_ct_rows_inv_store<N>, sm))) return;
+      k_ct_rows_inv_store<N><<<nblk, Tpl<N>::value * RP * nf, sm, st>>>(a);
     }
     gb_count_launch();
     cudaError_t e = cudaGetLastError();
@@ -549,13 +527,12 @@ inline int plane_conv_f32(gbofdft_plan* p, void* spec, int64_t fstride, int nf, 
 #define GB_CT_DEFINE_PLANE()                                                                                   \
   int gb_ct_rows_fwd_pm_f32(gbofdft_plan* p, const void* in, void* spec, int64_t fstride, int nf,             \
                             const int* ops, double beta, cudaStream_t st) {                                   \
-    return gbct::ct_rows_fwd<float, true>(p, in, spec, fstride, 0, nf, ops, beta, 1.0, st);                   \
+    return gbct::ct_rows_fwd(p, in, spec, fstride, nf, ops, beta, st);                   \
   }                                                                                                            \
   int gb_ct_rows_inv_eval_pm_f32(gbofdft_plan* p, const void* spec, int64_t fstride, int nf,                  \
                                  const EvalDesc* ev, const void* rho, const void* vloc, void* pot, int calc_e,  \
                                  double* partials, int64_t* nblk, cudaStream_t st) {                           \
-    return gbct::ct_rows_inv<float, true>(p, spec, fstride, 0, nf, nullptr, 0, 1.0, ev, rho, vloc, pot,       \
-                                          calc_e, partials, nblk, st);                                         \
+    return gbct::ct_rows_inv(p, spec, fstride, nf, nullptr, 0, ev, rho, vloc, pot, calc_e, partials, nblk, st); \
   }                                                                                                            \
   int gb_plane_conv_f32(gbofdft_plan* p, void* spec, int64_t fstride, int nf, const KerDesc* kd,               \
                         const float* const* pm_arr, double scale, cudaStream_t st) {                          \
@@ -563,8 +540,8 @@ inline int plane_conv_f32(gbofdft_plan* p, void* spec, int64_t fstride, int nf, 
   }                                                                                                            \
   int gb_ct_rows_inv_store_pm_f32(gbofdft_plan* p, const void* spec, int64_t fstride, int nf, void* out,       \
                                   int64_t ostride, cudaStream_t st) {                                          \
-    return gbct::ct_rows_inv<float, true>(p, spec, fstride, 0, nf, out, ostride, 1.0, nullptr, nullptr,        \
-                                          nullptr, nullptr, 0, nullptr, nullptr, st);                          \
+    return gbct::ct_rows_inv(p, spec, fstride, nf, out, ostride, nullptr, nullptr, nullptr, nullptr, 0,        \
+                             nullptr, nullptr, st);                                                            \
   }                                                                                                            \
   int gb_plane_supported_f32(int n0, int n1, int n2) {                                                         \
     bool rows = gbct::ct_dispatch(n2, [](auto) {});                                                            \

@@ -45,10 +45,10 @@ struct DeltaRowsFwd {
 };
 
 // One CTA: RP row pairs, every field's change transformed along axis 2 (R2C)
-// and written plane-major (as k_ct_rows_fwd<float, N, true>).
+// and written plane-major (as k_ct_rows_fwd<N>).
 template <int N>
-__global__ void __launch_bounds__(rows_threads_max<float, N>(), GB_CT_ROWS_MINB) k_delta_rows_fwd(DeltaRowsFwd a) {
-  constexpr int RP = RowsCfg<float>::RP, TPL = Tpl<N>::value, NP = Pad<float, N>::NP, NH = N / 2 + 1;
+__global__ void __launch_bounds__(rows_threads_max<N>(), GB_CT_ROWS_MINB) k_delta_rows_fwd(DeltaRowsFwd a) {
+  constexpr int RP = kRowPairs, TPL = Tpl<N>::value, NP = Pad<float, N>::NP, NH = N / 2 + 1;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int nl = a.nf * RP;
   cpx<float>* tw = reinterpret_cast<cpx<float>*>(smem_raw);
@@ -178,8 +178,8 @@ __device__ __forceinline__ float pdelta(float bp, float L, float p) { return bp 
 // with rho or rho_ref at the 1e-30 clamp, or with rs on different sides of 1
 // (or within 1e-5 of it), take the FP64 epilogue at both densities.
 template <int N, bool WANT_E>
-__global__ void __launch_bounds__(rows_threads_max<float, N>(), GB_CT_ROWS_MINB) k_delta_rows_inv_eval(DeltaRowsInv a) {
-  constexpr int RP = RowsCfg<float>::RP, NP = Pad<float, N>::NP;
+__global__ void __launch_bounds__(rows_threads_max<N>(), GB_CT_ROWS_MINB) k_delta_rows_inv_eval(DeltaRowsInv a) {
+  constexpr int RP = kRowPairs, NP = Pad<float, N>::NP;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int nl = a.c.nf * RP;
   cpx<float>* tw = reinterpret_cast<cpx<float>*>(smem_raw);
@@ -189,7 +189,7 @@ __global__ void __launch_bounds__(rows_threads_max<float, N>(), GB_CT_ROWS_MINB)
   const int64_t base = (int64_t)blockIdx.x * 2 * RP;
   const cpx<float>* twg = reinterpret_cast<const cpx<float>*>(a.c.tw);
   for (int i = tid; i < N; i += blockDim.x) tw[i] = twg[i];
-  const cpx<float>* res = ct_rows_inv_lines<float, N, true>(a.c, base, tw, A, B);
+  const cpx<float>* res = ct_rows_inv_lines<N>(a.c, base, tw, A, B);
   const EvalDesc& ev = a.ev;
   constexpr float cx = 0.98474502184269654115f;           // (3/pi)^(1/3)
   constexpr float RSC = 0.62035049089940001667f;          // (3/(4 pi))^(1/3)
@@ -348,7 +348,7 @@ int gb_delta_rows_fwd(gbofdft_plan* p, const double* rho, const double* rho_ref,
   int rc = 1;
   ct_dispatch(p->n[2], [&](auto nc) {
     constexpr int N = decltype(nc)::value;
-    constexpr int RP = RowsCfg<float>::RP, NP = Pad<float, N>::NP;
+    constexpr int RP = kRowPairs, NP = Pad<float, N>::NP;
     DeltaRowsFwd a;
     memset(&a, 0, sizeof(a));
     a.rho = rho; a.ref = rho_ref; a.out = spec; a.fstride = fstride;
@@ -376,10 +376,10 @@ int gb_delta_rows_inv_eval(gbofdft_plan* p, const void* spec, int64_t fstride, i
   int rc = 1;
   ct_dispatch(p->n[2], [&](auto nc) {
     constexpr int N = decltype(nc)::value;
-    constexpr int RP = RowsCfg<float>::RP, NP = Pad<float, N>::NP;
+    constexpr int RP = kRowPairs, NP = Pad<float, N>::NP;
     DeltaRowsInv a;
     memset(&a, 0, sizeof(a));
-    a.c.in = spec; a.c.fstride = fstride; a.c.nrows = p->n[0] * p->n[1]; a.c.ld2 = 0; a.c.nf = nf;
+    a.c.in = spec; a.c.fstride = fstride; a.c.nrows = p->n[0] * p->n[1]; a.c.nf = nf;
     a.c.tw = p->tw[2];
     a.ev = *ev;
     a.rho = rho; a.rho_ref = rho_ref; a.pot_ref = pot_ref; a.vloc = vloc; a.cref = cref; a.cstride = cstride;

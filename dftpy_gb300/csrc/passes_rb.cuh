@@ -959,7 +959,7 @@ struct LwtRows {
   int first, m, below;
   int nrows, n2h, ld2, lp;
   RbAxis ax;
-  FastDiv dn, dnh;
+  FastDiv dnh;
   const void* tw;
   Sc half;
   Sc lo[GB_LWT_BATCH + 1], hi[GB_LWT_BATCH + 1], inv[GB_LWT_BATCH + 1];
@@ -1835,7 +1835,6 @@ static int lwt_rows(gbofdft_plan* p, const RbLwtRows& d, cudaStream_t st) {
   a.kf = d.kf; a.ra = d.ra; a.out1 = d.out1; a.out3 = d.out3; a.first = d.first;
   a.m = k.m; a.below = k.below;
   a.nrows = p->n[0] * p->n[1]; a.n2h = p->n2h; a.ld2 = d.ld2;
-  a.dn.set(p->n[2]);
   a.dnh.set(p->n2h);
   a.tw = p->tw[2];
   a.half.set(0.5 * d.scale);

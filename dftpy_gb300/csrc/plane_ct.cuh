@@ -7,7 +7,7 @@
 // Spectra are plane-major here: element (i0, i1, k2) of field f sits at
 //   spec[f * fstride + (k2 * n0 + i0) * n1 + i1]
 // so a plane is one contiguous block; the row passes read and write that
-// layout (PM instantiations of k_ct_rows_fwd / k_ct_rows_inv_eval).
+// layout (k_ct_rows_fwd / k_ct_rows_inv_eval).
 //
 // The FFT stages run in place in the plane buffer: every thread loads the
 // inputs of its butterflies (and twiddles them) into registers, the CTA

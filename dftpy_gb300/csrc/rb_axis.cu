@@ -33,12 +33,6 @@ RbAxis rb_axis(int n, bool f64, bool reverse) {
   if (f64) {
     int cur[8];
     search(n, 16, cur, 0, best, bestn);
-  } else if (n == 128) {
-    best[0] = 8; best[1] = 4; best[2] = 4;
-    bestn = 3;
-  } else if (n == 360) {
-    best[0] = 8; best[1] = 5; best[2] = 3; best[3] = 3;
-    bestn = 4;
   } else {
     static const int order[] = {8, 4, 2, 3, 5, 7};
     int m = n;

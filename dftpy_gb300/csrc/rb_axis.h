@@ -26,7 +26,8 @@ struct RbAxis {
 
 // The radices of a length in stage order (reverse: the other way round); nst = 0
 // when the length has a prime factor above 7.  FP64: composite radices up to 16,
-// as few stages as possible, largest first.  FP32: 8, 4, 2, 3, 5, 7.
+// as few stages as possible, largest first.  FP32: 8, 4, 2, 3, 5, 7 (the kernels of
+// one length have their own order, in the lists of passes_rb.cuh).
 RbAxis rb_axis(int n, bool f64, bool reverse);
 
 // Lengths whose FP32 row passes form sqrt(rho) as rho rsqrt(rho); the others take
