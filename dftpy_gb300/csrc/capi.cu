@@ -368,7 +368,7 @@ static int eval_extra(gbofdft_plan* p, const void* rho, const gbofdft_functional
   return rc;
 }
 
-// gbofdft_eval; cout != nullptr (FP64 compile-time-size passes) also stores
+// gbofdft_eval; cout != nullptr (FP64 register-blocked passes) also stores
 // the convolution results, field slot f at cout + f * N; extras = 0 leaves
 // out the LWT / WGC terms (the fused terms alone)
 static int eval_impl(gbofdft_plan* p, const void* rho, const gbofdft_functional* f, void* pot, double* energies,

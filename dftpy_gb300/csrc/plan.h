@@ -23,7 +23,7 @@ struct gbofdft_plan {
   int64_t NG;            // n0 n1 n2h (API spectrum size)
   int64_t NGld;          // n0 n1 ld2 (internal spectrum size)
   AxisPlan ax[3];
-  gbrb::RbAxis rb[3], rbi[3];   // register-blocked passes: radices largest first, smallest first
+  gbrb::RbAxis rb[3], rbi[3];   // register-blocked passes: radices in stage order, and the other way round
   void* tw[3];           // device twiddle tables, complex<prec>[n_axis]
   void* spec;            // GB_MAX_FIELDS internal spectra
   double* partials;      // per-CTA energy partial sums
@@ -65,7 +65,7 @@ struct EvalDesc {
   int slot_h, slot_vw, slot_wt;   // field slot of each convolution output
   double tf_x, vw_y, wt_alpha, wt_beta;
   double e_ion;
-  // optional (FP64 compile-time-size passes only): the convolution results
+  // optional (FP64 register-blocked passes only): the convolution results
   // before the pointwise epilogue, field slot f at cout + f * cstride
   void* cout;
   int64_t cstride;
