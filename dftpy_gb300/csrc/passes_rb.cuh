@@ -25,8 +25,9 @@
 #include "plan.h"
 
 // FP32 lengths with kernels of their own: the even 2, 3, 5, 7-smooth lengths
-// from 24 to 400 whose radices split into two stages of at most 25, and some
-// that need three
+// from 24 to 400 whose radices split into two stages of at most 25, and eight of
+// those that need three (196, 210, 224, 256, 280, 288, 320, 360).  294, 324, 350,
+// 384, 392, odd and longer lengths run the kernels of run-time lengths.
 #define GB_RB_LENGTHS_1(X) \
   X(24, GB_RB_G(8), GB_RB_G(3)) X(28, GB_RB_G(4), GB_RB_G(7)) X(30, GB_RB_G(2, 3), GB_RB_G(5)) \
   X(32, GB_RB_G(8), GB_RB_G(4)) X(36, GB_RB_G(4), GB_RB_G(3, 3)) X(40, GB_RB_G(8), GB_RB_G(5)) \
