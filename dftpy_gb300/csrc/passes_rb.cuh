@@ -91,24 +91,23 @@ __device__ __forceinline__ double rroot6(double x) {
 }
 
 // The roots of a positive density that the terms are made of: x^(1/3), x^(-1/3),
-// x^(-1/2) and (FP64) x^(-1/6), from single-precision seeds.  Each ends in one
-// correction by a residual that one or two roundings separate from the exact one,
-// so the first three are good to about one rounding themselves, and the terms to
-// no more than library calls of cbrt, sqrt and division gave them (rms error of
-// the potentials in 2^-53, 24 x 20 x 84: Thomas-Fermi 1.0, LDA 0.6; library 1.2,
-// 0.7; the powers of one x^(-1/6), 13 FP64 operations against 20, 1.6, 1.7).
+// x^(-1/2) and (FP64) x^(-1/6), from single-precision seeds.  x^(1/3), x^(-1/3) and
+// x^(-1/6) each end in a correction by r = 1 - x y0^6, a third of whose roundings
+// reaches them, so they are good to about one rounding themselves, and the terms to
+// no more than library calls of cbrt, sqrt and division gave them (rms error of the
+// potentials in 2^-53, 24 x 20 x 84: Thomas-Fermi 1.0, LDA 0.6; library 1.2, 0.7;
+// powers of one x^(-1/6), 14 FP64 operations against 17, 1.6 and 1.7).  x^(-1/2), a
+// product of two (0.8 rms), only ever meets a convolution's result, whose error is
+// thousands of roundings.
 template <typename T> struct Roots { T c, z3, z2, y; };
 __device__ __forceinline__ Roots<double> roots(double x) {
-  const float f = (float)x;
-  const double a = (double)rcbrtf(f), b = (double)rsqrtf(f);
-  // squares of FP32 numbers are exact; r = 1 - x a^3, e = 1 - x b^2
-  const double a2 = a * a, r = fma(-x, a2 * a, 1.0), e = fma(-x, b * b, 1.0);
+  const double y0 = (double)rsqrtf(cbrtf((float)x));     // (its square is exact)
+  const double y2 = y0 * y0, c0 = x * (y2 * y2), r = fma(-c0, y2, 1.0);
   Roots<double> q;
-  q.z3 = fma(a * r, fma(r, 2.0 / 9.0, 1.0 / 3.0), a);
-  q.z2 = fma(b * e, fma(e, 0.375, 0.5), b);
-  const double c = x * q.z3 * q.z3;
-  q.c = fma(fma(-(c * c), c, x), a2 * (1.0 / 3.0), c);
-  q.y = q.c * q.z2;
+  q.z3 = fma(y2 * r, fma(r, 2.0 / 9.0, 1.0 / 3.0), y2);
+  q.c = fma(c0 * r, fma(r, 5.0 / 9.0, 2.0 / 3.0), c0);
+  q.y = fma(y0 * r, fma(r, 7.0 / 72.0, 1.0 / 6.0), y0);
+  q.z2 = q.y * q.z3;
   return q;
 }
 __device__ __forceinline__ Roots<float> roots(float x) {
