@@ -25,7 +25,7 @@ from . import _lib
 
 # Part of every key: raised when the passes behind a schedule change speed.  A file
 # kept from before the register-blocked lines names the plane pipeline, the faster
-# one then; a 128^3 FP32 Wang-Teter potential takes 99 us with it, 81 without.
+# one then; a 128^3 FP32 Wang-Teter potential takes 95 us with it, 80 without.
 _PASSES = 2
 
 _CACHE = {}

@@ -214,7 +214,7 @@ int gbofdft_plan_create(const int nr[3], const double lattice[9], int precision,
   p->gi.full = p->full;
   // FP32 grids whose (n0, n1) plane fits in shared memory can evaluate through
   // the plane pipeline (GBOFDFT_PLANE=1, or chosen as a schedule); the
-  // register-blocked column passes are faster (128^3, WT: 81 against 99 us)
+  // register-blocked column passes are faster (128^3, WT: 80 against 95 us)
   const char* pe = getenv("GBOFDFT_PLANE");
   p->plane_ok = precision == GBOFDFT_F32 && gb_plane_supported_f32(nr[0], nr[1], nr[2]);
   p->plane = p->plane_ok && pe && pe[0] == '1';

@@ -1566,10 +1566,10 @@ template <typename K> inline int launch_check(const char* what) {
 }
 
 // f(axis type, reversed axis type) for a length.  The FP32 lengths listed
-// above have kernels with every index folded at compile time: the FP32 passes
-// are bound by instruction issue and fetch (128^3, three fields: a column pass
-// 12.5 -> 9.4 us, the convolution 34 -> 16 us), the FP64 ones by the FP64 pipe,
-// where the kernels with run-time lengths are as fast.  Each translation unit
+// above have kernels with every index folded at compile time: no radix switch, no
+// index arithmetic between a thread's loads (128^3, three fields: a column pass
+// 12.5 -> 9.4 us, the convolution 34 -> 16 us).  FP64 passes wait for the FP64
+// pipe, and the kernels with run-time lengths are as fast.  Each translation unit
 // holds one group of lengths (GB_RB_GROUP); group 0 holds every other length.
 // 1: the length belongs to another group.
 template <typename A, typename B> struct AxPair { using ax = A; using inv = B; };
